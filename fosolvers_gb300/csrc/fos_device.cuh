@@ -192,18 +192,35 @@ __device__ __forceinline__ df2 df_from_double(double x) {
 __device__ __forceinline__ double neg_bits(double x) {
   return __hiloint2double(__double2hiint(x) ^ (int)0x80000000u, __double2loint(x));
 }
+// x with its sign bit exclusive-or'ed with flip's (0 or 0x80000000)
+__device__ __forceinline__ double flip_sign(double x, int flip) {
+  return __hiloint2double(__double2hiint(x) ^ flip, __double2loint(x));
+}
 // finiteness from the exponent field of the high word (one 32-bit integer test, no FP64
 // compare)
 __device__ __forceinline__ bool finite_bits(double x) {
   return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
 }
 
-// 1/a in FP64 by Newton--Raphson iteration x <- x (2 - a x) from an FP32 seed (two steps
-// take the ~2^-23 seed error to the FP64 rounding level); four FP64 FMAs
+// 1/a and 1/sqrt(a) in FP64: the special-function unit's approximation (about 20 bits, full
+// binary64 range, not an FP64-pipe instruction) and one step of Householder's cubically
+// convergent iteration, which takes the seed's error to about 2^-60, so the result carries
+// the rounding of its last operation.  Three and five FP64 instructions, where the division
+// and square root operators issue about ten each.  No special cases: a zero, infinite or
+// (after flushing) subnormal argument gives a non-finite result.
 __device__ __forceinline__ double rcp64(double a) {
-  double x = f2d_bits(__frcp_rn(d2f_trunc(a)));
-  double e = fma(-a, x, 1.0);
-  x = fma(x, e, x);
-  e = fma(-a, x, 1.0);
-  return fma(x, e, x);
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  const double e = fma(-a, x, 1.0);  // 1/a = x (1 + e + e^2 + ...)
+  return fma(x, fma(e, e, e), x);
+}
+// also root = sqrt(a), from the same seed (one more instruction)
+__device__ __forceinline__ double rsqrt64(double a, double& root) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double t = a * y;
+  const double e = fma(-t, y, 1.0);  // a^(-1/2) = y (1 - e)^(-1/2) = y (1 + e/2 + 3 e^2/8 + ...)
+  const double q = e * fma(0.375, e, 0.5);
+  root = fma(t, q, t);
+  return fma(y, q, y);
 }

@@ -39,61 +39,59 @@ __device__ __forceinline__ void load_prim(const double* __restrict__ W, int c, P
 
 __device__ __forceinline__ void prim_from_cons(double rho, double mx, double my, double mz,
                                                double E, double gm1, P64& P) {
-  double inv = 1.0 / rho;
+  const double inv = rcp64(rho);
   P.rho = rho;
   P.u = mx * inv; P.v = my * inv; P.w = mz * inv;
-  P.p = gm1 * (E - 0.5 * (mx * mx + my * my + mz * mz) * inv);
+  P.p = gm1 * fma(-0.5, fma(mz, P.w, fma(my, P.v, mx * P.u)), E);
   P.H = (E + P.p) * inv;
-  P.s = sqrt(rho);
+  (void)rsqrt64(rho, P.s);
 }
 
 // Roe flux-difference splitting flow through one face (Euler.f90:90-126), FP64,
-// central part as the reference writes it: aP*(1/2 (F_L + F_R).n - 1/2 sum of waves)
+// central part as the reference writes it: aP*(1/2 (F_L + F_R).n - 1/2 sum of waves).
+// The FP64 pipe bounds the kernels that call it (2 lanes per clock and SM), so the five waves
+// are collected by direction before they meet the flux: with s-, s+ the acoustic strengths and
+// e the entropy strength times |un|, the sum of waves is
+//   A (1, ua, va, wa, .) + C (0, uJ, vJ, wJ, .) + G (0, n, .),
+//   A = e + s- + s+, C = |un| rhoA, G = c (s+ - s-) - C unJ,
+// and its energy row e q2/2 + (s- + s+) Ha + C (ua . uJ) + G un.  The averages come from the
+// jumps (ua = uL + sR/(sL + sR) uJ).  91 FP64 instructions where the waves added one by one
+// took about 150 (an FP64 Jv at 48^3 x 6 tetrahedra, primitives and gather included: 436 ->
+// 317 us; the FP64 pipe is what bounds it before and after).
 __device__ __forceinline__ void roe_flow64(const P64& L, const P64& R, double nx, double ny,
                                            double nz, double aP, double gm1, double flow[5]) {
-  const double inv = 1.0 / (L.s + R.s);
-  const double ua = (L.s * L.u + R.s * R.u) * inv;
-  const double va = (L.s * L.v + R.s * R.v) * inv;
-  const double wa = (L.s * L.w + R.s * R.w) * inv;
-  const double Ha = (L.s * L.H + R.s * R.H) * inv;
-  const double rhoA = L.s * R.s;
-  const double q2 = ua * ua + va * va + wa * wa;
-  const double c2 = gm1 * (Ha - 0.5 * q2);
-  const double ca = sqrt(c2);
-  const double ic2 = 1.0 / c2;
-  const double unA = ua * nx + va * ny + wa * nz;
-  const double rJ = R.rho - L.rho, pJ = R.p - L.p;
+  const double wR = R.s * rcp64(L.s + R.s);
+  const double rJ = R.rho - L.rho, pJ = R.p - L.p, HJ = R.H - L.H;
   const double uJ = R.u - L.u, vJ = R.v - L.v, wJ = R.w - L.w;
-  const double unJ = uJ * nx + vJ * ny + wJ * nz;
-  // entropy + shear waves
-  const double au = fabs(unA);
-  const double wE = rJ - pJ * ic2;
-  double d0 = au * wE;
-  double d1 = au * (wE * ua + rhoA * (uJ - nx * unJ));
-  double d2 = au * (wE * va + rhoA * (vJ - ny * unJ));
-  double d3 = au * (wE * wa + rhoA * (wJ - nz * unJ));
-  double d4 = au * (wE * (0.5 * q2) + rhoA * (ua * uJ + va * vJ + wa * wJ - unA * unJ));
-  // acoustic waves
-  const double s1 = fabs(unA - ca) * (0.5 * (pJ - rhoA * ca * unJ) * ic2);
-  d0 += s1;
-  d1 += s1 * (ua - nx * ca);
-  d2 += s1 * (va - ny * ca);
-  d3 += s1 * (wa - nz * ca);
-  d4 += s1 * (Ha - unA * ca);
-  const double s2 = fabs(unA + ca) * (0.5 * (pJ + rhoA * ca * unJ) * ic2);
-  d0 += s2;
-  d1 += s2 * (ua + nx * ca);
-  d2 += s2 * (va + ny * ca);
-  d3 += s2 * (wa + nz * ca);
-  d4 += s2 * (Ha + unA * ca);
-  const double unL = L.u * nx + L.v * ny + L.w * nz;
-  const double unR = R.u * nx + R.v * ny + R.w * nz;
+  const double ua = fma(wR, uJ, L.u), va = fma(wR, vJ, L.v), wa = fma(wR, wJ, L.w);
+  const double Ha = fma(wR, HJ, L.H);
+  const double rhoA = L.s * R.s;
+  const double hq = 0.5 * fma(wa, wa, fma(va, va, ua * ua));
+  const double c2 = gm1 * (Ha - hq);
+  double ca;
+  const double ic = rsqrt64(c2, ca);
+  const double ic2 = ic * ic;
+  const double unL = fma(L.w, nz, fma(L.v, ny, L.u * nx));
+  const double unJ = fma(wJ, nz, fma(vJ, ny, uJ * nx));
+  const double unR = unL + unJ, un = fma(wR, unJ, unL);
   const double mL = L.rho * unL, mR = R.rho * unR;
-  flow[0] = aP * (0.5 * (mL + mR) - 0.5 * d0);
-  flow[1] = aP * (0.5 * (mL * L.u + L.p * nx + mR * R.u + R.p * nx) - 0.5 * d1);
-  flow[2] = aP * (0.5 * (mL * L.v + L.p * ny + mR * R.v + R.p * ny) - 0.5 * d2);
-  flow[3] = aP * (0.5 * (mL * L.w + L.p * nz + mR * R.w + R.p * nz) - 0.5 * d3);
-  flow[4] = aP * (0.5 * (mL * L.H + mR * R.H) - 0.5 * d4);
+  // wave strengths
+  const double au = fabs(un);
+  const double e = au * fma(-pJ, ic2, rJ);
+  const double rc = rhoA * ca, k = 0.5 * ic2;
+  const double s1 = (fabs(un - ca) * k) * fma(-rc, unJ, pJ);
+  const double s2 = (fabs(un + ca) * k) * fma(rc, unJ, pJ);
+  const double s12 = s1 + s2;
+  const double A = e + s12, C = au * rhoA;
+  const double G = fma(-C, unJ, ca * (s2 - s1));
+  const double pn = (L.p + R.p) - G;
+  const double h = 0.5 * aP;
+  flow[0] = h * ((mL + mR) - A);
+  flow[1] = h * fma(pn, nx, fma(-C, uJ, fma(-A, ua, fma(mR, R.u, mL * L.u))));
+  flow[2] = h * fma(pn, ny, fma(-C, vJ, fma(-A, va, fma(mR, R.v, mL * L.v))));
+  flow[3] = h * fma(pn, nz, fma(-C, wJ, fma(-A, wa, fma(mR, R.w, mL * L.w))));
+  const double uu = fma(wa, wJ, fma(va, vJ, ua * uJ));
+  flow[4] = h * fma(-G, un, fma(-C, uu, fma(-s12, Ha, fma(-e, hq, fma(mR, R.H, mL * L.H)))));
 }
 
 // kV: the state is y + s v (a Jv), else y (compile-time, as in k_prim_hl)
@@ -224,15 +222,19 @@ __global__ void __launch_bounds__(kThreads) k_gather(
   if (c >= nC) return;
   int e[kW];
   load_ell<kW>(ell, c, e);
+  // every cell has at least one face: the first initialises the sums, and a flow's sign
+  // flips on the integer pipe, so a tetrahedron's sums are 15 FP64 additions
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int k = 0; k < kW; k++) {
     if (e[k] < 0) continue;
-    const double sg = (e[k] & 1) ? 1.0 : -1.0;
     const double2* F2 = reinterpret_cast<const double2*>(F + 6 * (size_t)(e[k] >> 1));
     const double2 a0 = __ldg(F2), a1 = __ldg(F2 + 1), a2 = __ldg(F2 + 2);
-    acc[0] += sg * a0.x; acc[1] += sg * a0.y; acc[2] += sg * a1.x; acc[3] += sg * a1.y;
-    acc[4] += sg * a2.x;
+    const int flip = (e[k] & 1) ? 0 : (int)0x80000000u;
+    const double t[5] = {flip_sign(a0.x, flip), flip_sign(a0.y, flip), flip_sign(a1.x, flip),
+                         flip_sign(a1.y, flip), flip_sign(a2.x, flip)};
+#pragma unroll
+    for (int q = 0; q < 5; q++) acc[q] = k == 0 ? t[q] : acc[q] + t[q];
   }
   gather_epilogue<kE>(nC, c, acc, __ldg(invV + c), vv, fy, d_s, a, out, flag);
 }
