@@ -99,6 +99,8 @@ struct fos_ctx {
   int* d_cdiag = nullptr;     // [nC] slot of the diagonal block, by internal cell
   int* d_ipos = nullptr;      // [nC] internal cell -> position
   int* d_ord = nullptr;       // [nC] position -> internal cell
+  unsigned char* d_cslot = nullptr;  // [4 or 8 per cell] block of the cell's row (0, 1, ...) of
+                                     // each face slot's neighbour (fused FP32 set-up)
   int* d_fslot = nullptr;     // [2*nFi] slots of blocks (L,R) and (R,L) per interior face
   void* d_Jraw = nullptr;     // [25*nnzb] unscaled Jacobian blocks (FP64, FP32 for FOS_ILU_FP32)
   void* d_Jb = nullptr;       // [25*nFb] boundary-face diagonal terms (same type)

@@ -239,36 +239,54 @@ __device__ __forceinline__ PrimT<float> load_prim_f32(const float* __restrict__ 
 // evaluated by both of its cells: FP32 arithmetic is cheap next to the scattered block
 // stores and the re-read of every off-diagonal block that a face-then-diagonal assembly
 // costs.
-// One block row of the FP32 Jacobian for cell c (the body of k_jac_cell32, shared with the
-// fused set-up k_pset32): the row's blocks go to st (row-major 25-float blocks at
-// st + 25 (slot - s0)); sdiag = the diagonal block's slot - s0.  The multiply-adds are
+// One block row of the FP32 Jacobian for cell c (shared by k_jac_cell32 and the fused set-up
+// k_pset32): emit(k, f, isR, a, b, value) takes entry (a, b) of the off-diagonal block of the
+// cell's k-th face f, D returns the diagonal block.  The loads of every face are issued before
+// the first face's arithmetic: the warps that run this are few (their staging fills the
+// shared memory), so a face must not wait for the one before it.  The multiply-adds are
 // written out (fmaf), so both kernels produce the same bits.
-template <int kW>
-__device__ __forceinline__ void jac_row32(int c, int nC, int nFi, int s0, int sdiag,
-                                          const int* __restrict__ ell,
+template <int kW, typename Emit>
+__device__ __forceinline__ void jac_row32(int c, int nC, int nFi, const int* __restrict__ ell,
                                           const int* __restrict__ cnb,
                                           const float4* __restrict__ cna,
-                                          const int* __restrict__ fslot,
                                           const float* __restrict__ Whl,
                                           const double* __restrict__ Gb,
-                                          const float4* __restrict__ Sc, float gg,
-                                          float* __restrict__ st) {
+                                          const float4* __restrict__ Sc, float gg, float D[25],
+                                          Emit&& emit) {
+  int ent[kW], nbr[kW];
+  if constexpr (kW == 4) {
+    const int4 e4 = __ldg(reinterpret_cast<const int4*>(ell) + c);
+    const int4 q4 = __ldg(reinterpret_cast<const int4*>(cnb) + c);
+    ent[0] = e4.x; ent[1] = e4.y; ent[2] = e4.z; ent[3] = e4.w;
+    nbr[0] = q4.x; nbr[1] = q4.y; nbr[2] = q4.z; nbr[3] = q4.w;
+  } else {
+#pragma unroll
+    for (int k = 0; k < kW; k++) {
+      ent[k] = __ldg(ell + (size_t)kW * c + k);
+      nbr[k] = __ldg(cnb + (size_t)kW * c + k);
+    }
+  }
   const PrimT<float> P = load_prim_f32(Whl, c);
-  float D[25];
+  // the cell across each face (the cell itself where there is none) and the face's geometry
+  float4 nas[kW];
+  PrimT<float> Qs[kW];
+#pragma unroll
+  for (int k = 0; k < kW; k++) {
+    nas[k] = __ldg(cna + (size_t)k * nC + c);
+    Qs[k] = load_prim_f32(Whl, nbr[k]);
+  }
 #pragma unroll
   for (int k = 0; k < 25; k++) D[k] = 0.0f;
-#pragma unroll 1
+#pragma unroll
   for (int k = 0; k < kW; k++) {
-    const int ek = __ldg(ell + (size_t)kW * c + k);
+    const int ek = ent[k];
     if (ek < 0) continue;
     const int f = ek >> 1;
     const bool isR = ek & 1;
-    const float4 na = __ldg(cna + (size_t)k * nC + c);  // the face's FP32 geometry, per cell
+    const float4 na = nas[k];
     const float n[3] = {na.x, na.y, na.z};
-    PrimT<float> Q;
-    if (f < nFi) {
-      Q = load_prim_f32(Whl, __ldg(cnb + (size_t)kW * c + k));  // the cell across the face
-    } else {  // ghost primitives of k_jac_ghost64
+    PrimT<float> Q = Qs[k];
+    if (f >= nFi) {  // ghost primitives of k_jac_ghost64
       const double2* G2 = reinterpret_cast<const double2*>(Gb + 6 * (size_t)f);
       const double2 a0 = __ldg(G2), a1 = __ldg(G2 + 1), a2 = __ldg(G2 + 2);
       Q = {{d2f_trunc(a0.x), d2f_trunc(a0.y), d2f_trunc(a1.x)}, d2f_trunc(a1.y),
@@ -285,24 +303,19 @@ __device__ __forceinline__ void jac_row32(int c, int nC, int nFi, int s0, int sd
     float Ab[25];
     anfj<float>(n, ua, Ha, ca, gg, Ab);
     const float h = 0.5f * na.w;
-    if (f >= nFi) {  // boundary pair: diagonal term only (its A(u_c) part is in S_c)
 #pragma unroll
-      for (int q = 0; q < 25; q++) D[q] = fmaf(-h, Ab[q], D[q]);
-      continue;
-    }
+    for (int q = 0; q < 25; q++) D[q] = fmaf(-h, Ab[q], D[q]);
+    if (f >= nFi) continue;  // boundary pair: diagonal term only (its A(u_c) part is in S_c)
     // the neighbour's normal flux Jacobian with the face normal: +aP/2 for cell R, -aP/2 for L
     const float v2Q = Q.u[0] * Q.u[0] + Q.u[1] * Q.u[1] + Q.u[2] * Q.u[2];
     const float vnQ = Q.u[0] * n[0] + Q.u[1] * n[1] + Q.u[2] * n[2];
     const float sh = isR ? h : -h;
-    float* off = st + 25 * (fslot[2 * f + (isR ? 1 : 0)] - s0);
 #pragma unroll
     for (int a = 0; a < 5; a++)
 #pragma unroll
-      for (int b = 0; b < 5; b++) {
-        off[5 * a + b] =
-            fmaf(h, Ab[5 * a + b], __fmul_rn(sh, nfj<float>(a, b, n, Q.u, Q.H, gg, v2Q, vnQ)));
-        D[5 * a + b] = fmaf(-h, Ab[5 * a + b], D[5 * a + b]);
-      }
+      for (int b = 0; b < 5; b++)
+        emit(k, f, isR, a, b,
+             fmaf(h, Ab[5 * a + b], __fmul_rn(sh, nfj<float>(a, b, n, Q.u, Q.H, gg, v2Q, vnQ))));
   }
   if (Sc) {  // -A(S_c/2; u_c): the own-state terms of a cell whose faces do not close
     const float4 S4 = __ldg(Sc + c);
@@ -315,9 +328,6 @@ __device__ __forceinline__ void jac_row32(int c, int nC, int nFi, int s0, int sd
       for (int b = 0; b < 5; b++)
         D[5 * a + b] = __fsub_rn(D[5 * a + b], nfj<float>(a, b, Sh, P.u, P.H, gg, v2P, vnP));
   }
-  float* dg = st + 25 * sdiag;
-#pragma unroll
-  for (int k = 0; k < 25; k++) dg[k] = D[k];
 }
 
 template <int kW>
@@ -337,8 +347,14 @@ __global__ void __launch_bounds__(64) k_jac_cell32(
     const int p = ipos[c];
     s0 = prow[p];
     nbk = prow[p + 1] - s0;
-    jac_row32<kW>(c, nC, nFi, s0, cdiag[c] - s0, ell, cnb, cna, fslot, Whl, Gb, Sc,
-                  d2f_trunc(g), st);
+    float D[25];
+    jac_row32<kW>(c, nC, nFi, ell, cnb, cna, Whl, Gb, Sc, d2f_trunc(g), D,
+                  [&](int, int f, bool isR, int a, int b, float v) {
+                    st[25 * (fslot[2 * f + (isR ? 1 : 0)] - s0) + 5 * a + b] = v;
+                  });
+    float* dg = st + 25 * (cdiag[c] - s0);
+#pragma unroll
+    for (int k = 0; k < 25; k++) dg[k] = D[k];
   }
   __syncwarp();
   // the warp's rows, one after another: row r = [25 s0_r, 25 (s0_r + nbk_r)) of J
@@ -568,74 +584,126 @@ __global__ void __launch_bounds__(kT) k_ilu_factor(
 
 // Fused FP32 set-up: one level (colour) of the block ILU(0) factorisation of
 // P = I - gamma diag(1/v) J with the rows of J assembled in the same kernel, so J is never
-// written to or read back from HBM.  Thread per row, a warp takes 32 rows of the level:
-//   A. the row's Jacobian blocks (jac_row32, the arithmetic of k_jac_cell32) staged in shared
-//      memory, then P = delta - (gamma/v) J in place;
-//   B. the update operations with the finished rows of earlier levels (L_pq = P_pq inv(D_q),
-//      P_pj -= L_pq U_qj, operands from LU), then the Gauss--Jordan inverse of the diagonal
-//      block in registers -- every lane its own row, so the 32 rows' operand loads are in
-//      flight together;
+// written to or read back from HBM.  One warp per block, thread per row, 32 rows of the level:
+//   0. the operands of the row's first two update operations (blocks of finished rows of
+//      earlier levels) start on their way into shared memory (cp.async);
+//   A. the row's Jacobian blocks (jac_row32, the arithmetic of k_jac_cell32), scaled to
+//      P = delta - (gamma/v) J as they are formed: the off-diagonal blocks go to the row's
+//      staging area in the factor's column-major order, the diagonal block stays in registers;
+//   B. the update operations L_pq = P_pq inv(D_q), P_pj -= L_pq U_qj, the operand of the
+//      operation after next always in flight, L_pq kept in registers between its operations,
+//      then the Gauss--Jordan inverse of the diagonal block;
 //   C. the warp stores its 32 rows one after another, each as its two contiguous ranges (L
-//      blocks, then inverted diagonal and U blocks), transposed to the column-major factor
-//      layout on the way, so the stores are coalesced.
-// The arithmetic is k_ilu_factor's operation for operation (ilu_mul_sub, ilu_gj_step), so the
+//      blocks, then inverted diagonal and U blocks).
+// What bounds it is the load/store unit and the issue slots, not HBM.  An operand block is 100
+// bytes at a 4-byte alignment; read by each lane with 25 loads it cost 25 x 32 cache lookups
+// per operation, so the lane now copies the 7 aligned 16-byte pieces that hold it.  Staging in
+// the stored order takes the transposition and its divisions (half the kernel's instructions)
+// out of C.  Staging and buffers (23 KB a warp) leave nine warps on an SM, which is why the
+// loads run ahead.  1.57 M tetrahedra, all four colours: 1190 us before, @@ us.
+// The arithmetic is k_ilu_factor's operation for operation (ilu_dot5, ilu_gj_step), so the
 // factors equal the two-kernel path's bit for bit.
+constexpr int kOpW = 28;  // floats of an operand's aligned 16-byte pieces
+
+__device__ __forceinline__ void op_copy(const float* LU, int blk, float* buf) {
+  const float* src = LU + ((25 * (size_t)blk) & ~(size_t)3);
+  const unsigned dst = (unsigned)__cvta_generic_to_shared(buf);
+#pragma unroll
+  for (int i = 0; i < kOpW / 4; i++)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * i),
+                 "l"(src + 4 * i)
+                 : "memory");
+}
+__device__ __forceinline__ void op_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
 template <int kW>
-__global__ void __launch_bounds__(64) k_pset32(
+__global__ void __launch_bounds__(32) k_pset32(
     int n, const int* __restrict__ rows, int p0, const int* __restrict__ prow,
     const int* __restrict__ pdiag, const int* __restrict__ ord, const double* __restrict__ invV,
     double gamma, int nC, int nFi, const int* __restrict__ ell, const int* __restrict__ cnb,
-    const float4* __restrict__ cna, const int* __restrict__ fslot,
+    const float4* __restrict__ cna, const unsigned char* __restrict__ cslot,
     const float* __restrict__ Whl, const double* __restrict__ Gb, const float4* __restrict__ Sc,
     double g, const int* __restrict__ upd_ptr, const int3* __restrict__ upd,
-    const int* __restrict__ plst, const int* __restrict__ pdu, float* __restrict__ LU,
+    const int* __restrict__ plst, const int* __restrict__ pdu, float* LU,
     int* __restrict__ ierr) {
-  constexpr int kRow = (kW + 1) * 25;
-  __shared__ float stg[2][32][kRow];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t = (blockIdx.x * 2 + warp) * 32 + lane;
-  float* st = stg[warp][lane];
-  int p = 0, s0 = 0, nb = 0, sd = 0;
+  constexpr int kRow = (kW + 1) * 25;  // odd: the lanes' rows fall in distinct banks
+  constexpr int kSlots = kW == 4 ? 4 : 8;
+  __shared__ __align__(16) float stg[32][kRow];
+  __shared__ __align__(16) float ops[2][32][kOpW];
+  const int lane = threadIdx.x;
+  const int t = blockIdx.x * 32 + lane;
+  float* st = stg[lane];
+  int p = 0, nb = 0, sd = 0;
   if (t < n) {
-    // A
+    // 0
     p = rows ? rows[t] : p0 + t;
-    s0 = prow[p];
+    const int o0 = upd_ptr[p], no = upd_ptr[p + 1] - o0;
+    const int3 none = make_int3(0, 0, 0);
+    int3 op = no > 0 ? upd[o0] : none, op1 = no > 1 ? upd[o0 + 1] : none,
+         op2 = no > 2 ? upd[o0 + 2] : none;
+    if (no > 0) op_copy(LU, op.y, ops[0][lane]);
+    op_commit();
+    if (no > 1) op_copy(LU, op1.y, ops[1][lane]);
+    op_commit();
+    const int s0 = prow[p];
     nb = prow[p + 1] - s0;
     sd = pdiag[p] - s0;
+    // A
     const int c = ord[p];
-    jac_row32<kW>(c, nC, nFi, s0, sd, ell, cnb, cna, fslot, Whl, Gb, Sc, d2f_trunc(g), st);
-    const float sc = d2f_trunc(gamma * invV[c]);
-    for (int b = 0; b < nb; b++) {
-      float* blk = st + 25 * b;
+    int slot[kW];  // block of the row that each face's off-diagonal block is
+    {
+      const unsigned* cs = reinterpret_cast<const unsigned*>(cslot + (size_t)kSlots * c);
 #pragma unroll
-      for (int k = 0; k < 25; k++)
-        blk[k] = fmaf(-sc, blk[k], (b == sd && k % 6 == 0) ? 1.0f : 0.0f);
+      for (int k = 0; k < kW; k++) slot[k] = (int)((__ldg(cs + k / 4) >> (8 * (k & 3))) & 0xffu);
     }
+    const float sc = d2f_trunc(gamma * invV[c]);
+    float D[25];
+    jac_row32<kW>(c, nC, nFi, ell, cnb, cna, Whl, Gb, Sc, d2f_trunc(g), D,
+                  [&](int k, int, bool, int a, int b, float v) {
+                    st[25 * slot[k] + 5 * b + a] = fmaf(-sc, v, 0.0f);
+                  });
+#pragma unroll
+    for (int k = 0; k < 25; k++) D[k] = fmaf(-sc, D[k], k % 6 == 0 ? 1.0f : 0.0f);
     // B
-    const int o1 = upd_ptr[p + 1];
-    for (int o = upd_ptr[p]; o < o1; o++) {
-      const int3 op = upd[o];
-      const float* Ab = st + 25 * (op.x - s0);
-      const float* B = LU + 25 * (size_t)op.y;  // column-major, finished in earlier levels
-      float* dst = st + 25 * ((op.z < 0 ? op.x : op.z) - s0);
+    float A[25];  // the L block of the last scaling operation, row-major
+#pragma unroll
+    for (int k = 0; k < 25; k++) A[k] = 0.0f;
+#pragma unroll 1
+    for (int o = 0; o < no; o++) {
+      asm volatile("cp.async.wait_group 1;" ::: "memory");  // this operation's operand is here
+      float* buf = ops[o & 1][lane];
       float Bv[25];
 #pragma unroll
-      for (int k = 0; k < 25; k++) Bv[k] = __ldg(B + k);
+      for (int k = 0; k < 25; k++) Bv[k] = buf[((25 * op.y) & 3) + k];
+      if (o + 2 < no) op_copy(LU, op2.y, buf);
+      op_commit();
+      const int3 op3 = o + 3 < no ? upd[o0 + o + 3] : none;
+      if (op.z < 0) {
+        float* Lb = st + 25 * (op.x - s0);
 #pragma unroll
-      for (int i = 0; i < 5; i++) {
-        float A[5];
+        for (int i = 0; i < 5; i++) {
+          float Ai[5];
 #pragma unroll
-        for (int k = 0; k < 5; k++) A[k] = Ab[5 * i + k];
+          for (int k = 0; k < 5; k++) Ai[k] = Lb[5 * k + i];
 #pragma unroll
-        for (int b = 0; b < 5; b++) {
-          const float acc = ilu_dot5(A, Bv + 5 * b);
-          dst[5 * i + b] = op.z < 0 ? acc : dst[5 * i + b] - acc;
+          for (int b = 0; b < 5; b++) A[5 * i + b] = ilu_dot5(Ai, Bv + 5 * b);
+#pragma unroll
+          for (int b = 0; b < 5; b++) Lb[5 * b + i] = A[5 * i + b];
         }
-      }
-    }
-    float D[25];
+      } else if (op.z - s0 == sd) {
 #pragma unroll
-    for (int k = 0; k < 25; k++) D[k] = st[25 * sd + k];
+        for (int i = 0; i < 5; i++)
+#pragma unroll
+          for (int b = 0; b < 5; b++) D[5 * i + b] -= ilu_dot5(A + 5 * i, Bv + 5 * b);
+      } else {
+        float* dst = st + 25 * (op.z - s0);
+#pragma unroll
+        for (int i = 0; i < 5; i++)
+#pragma unroll
+          for (int b = 0; b < 5; b++) dst[5 * b + i] -= ilu_dot5(A + 5 * i, Bv + 5 * b);
+      }
+      op = op1; op1 = op2; op2 = op3;
+    }
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 5; k++) {
@@ -648,22 +716,23 @@ __global__ void __launch_bounds__(64) k_pset32(
     }
     if (!ok) atomicMin(ierr, p + 1);
 #pragma unroll
-    for (int k = 0; k < 25; k++) st[25 * sd + k] = D[k];
+    for (int i = 0; i < 5; i++)
+#pragma unroll
+      for (int j = 0; j < 5; j++) st[25 * sd + 5 * j + i] = D[5 * i + j];
   }
   __syncwarp();
-  // C: row r's blocks [0, sd_r) go to the L region at plst, [sd_r, nb_r) to the D/U region at
-  // pdu; factor entry (i, j) of a block sits at 5 j + i (column-major), staging at 5 i + j
+  // C: row r's blocks [0, sd_r) go to the L region at plst, [sd_r, nb_r) to the D/U region at pdu
+  const int lo = nb ? plst[p] : 0, hi = nb ? pdu[p] - sd : 0;
   for (int rr = 0; rr < 32; rr++) {
-    const int nbr = __shfl_sync(0xffffffffu, nb, rr);
-    if (nbr == 0) continue;  // row past the end of the level
-    const int sdr = __shfl_sync(0xffffffffu, sd, rr);
-    const int pr = __shfl_sync(0xffffffffu, p, rr);
-    const float* src = stg[warp][rr];
-    float* dl = LU + 25 * (size_t)plst[pr];
-    float* du = LU + 25 * (size_t)pdu[pr] - 25 * (size_t)sdr;
-    for (int e = lane; e < 25 * nbr; e += 32) {
-      const int b = e / 25, r = e - 25 * b, i = r % 5, j = r / 5;
-      (b < sdr ? dl : du)[e] = src[25 * b + 5 * i + j];
+    const int nv = 25 * __shfl_sync(0xffffffffu, nb, rr);
+    if (nv == 0) continue;  // row past the end of the level
+    const int nl = 25 * __shfl_sync(0xffffffffu, sd, rr);
+    float* dl = LU + 25 * (size_t)__shfl_sync(0xffffffffu, lo, rr);
+    float* du = LU + 25 * (ptrdiff_t)__shfl_sync(0xffffffffu, hi, rr);
+#pragma unroll
+    for (int i = 0; i < (kRow + 31) / 32; i++) {
+      const int e = lane + 32 * i;
+      if (e < nv) (e < nl ? dl : du)[e] = stg[rr][e];
     }
   }
 }
@@ -934,6 +1003,17 @@ int fos_jac_setup(fos_ctx* c) {
     fslot[2 * f] = slot_of(pL, pR);
     fslot[2 * f + 1] = slot_of(pR, pL);
   }
+  if (fos_pset_is_fused(c)) {  // the same, by cell and face slot (k_pset32)
+    const int w = c->ell_w == 4 ? 4 : 8;
+    std::vector<unsigned char> cslot((size_t)w * nC, 0);
+    std::vector<unsigned char> cnt(nC, 0);
+    for (int f = 0; f < nFi; f++) {  // a cell's slots: its interior faces in this order
+      const int L = c->h_faceL[f], R = c->h_faceR[f];
+      cslot[(size_t)w * L + cnt[L]++] = (unsigned char)(fslot[2 * f] - prow[ipos[L]]);
+      cslot[(size_t)w * R + cnt[R]++] = (unsigned char)(fslot[2 * f + 1] - prow[ipos[R]]);
+    }
+    if (up(&c->d_cslot, cslot)) return -100;
+  }
   // schedule: colours (contiguous position ranges) or level sets (lists of positions)
   std::vector<int> rows_f, rows_b;
   if (c->ilu_colors) {
@@ -1047,8 +1127,8 @@ int fos_jac_setup(fos_ctx* c) {
   FOS_CUDA(cudaMalloc((void**)&c->d_Jb, 25 * jb * (size_t)std::max(c->nFb, 1)));
   FOS_CUDA(cudaMalloc((void**)&c->d_ilu_tmp, 16 * sizeof(double) * (size_t)nC));  // 2 AoS vectors
   FOS_CUDA(cudaMalloc((void**)&c->d_ierr, sizeof(int)));
-  if (f32)
-    FOS_CUDA(cudaMalloc((void**)&c->d_LU32, 25 * sizeof(float) * (size_t)c->nnzb));
+  if (f32)  // (+ 4: the aligned pieces that hold the last block)
+    FOS_CUDA(cudaMalloc((void**)&c->d_LU32, sizeof(float) * (25 * (size_t)c->nnzb + 4)));
   else
     FOS_CUDA(cudaMalloc((void**)&c->d_LU, 25 * sizeof(double) * (size_t)c->nnzb));
   return 0;
@@ -1131,10 +1211,11 @@ int fos_pset_fused(fos_ctx* c, const double* y, double gamma) {
     const int n = c->lev_f[l + 1] - c->lev_f[l];
     const int* rows = c->d_lrows_f ? c->d_lrows_f + c->lev_f[l] : nullptr;
     auto k = c->ell_w == 4 ? k_pset32<4> : k_pset32<6>;
-    fos_launch(c, k, (n + 63) / 64, 64, n, rows, c->lev_f[l], (const int*)c->d_prow,
+    fos_launch(c, k, (n + 31) / 32, 32, n, rows, c->lev_f[l], (const int*)c->d_prow,
                (const int*)c->d_pdiag, (const int*)c->d_ord, (const double*)c->d_invV, gamma,
                c->nC, c->nFi, (const int*)c->d_ell, (const int*)c->d_cnb,
-               (const float4*)c->d_cna32, (const int*)c->d_fslot, (const float*)c->d_Whl,
+               (const float4*)c->d_cna32, (const unsigned char*)c->d_cslot,
+               (const float*)c->d_Whl,
                (const double*)c->d_F, (const float4*)c->d_closure32, c->gamm,
                (const int*)c->d_upd_ptr, (const int3*)c->d_upd, (const int*)c->d_plst,
                (const int*)c->d_pdu, c->d_LU32, c->d_ierr);
