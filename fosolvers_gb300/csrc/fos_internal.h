@@ -182,7 +182,7 @@ int fos_d2h_reference(fos_ctx* c, const double* d_internal, double* h);
 int fos_jv_sigma(fos_ctx* c, double* d_scal, double ynorm, double eps, double b);
 int fos_jv_sigma_known(fos_ctx* c, double* d_scal, double ynorm, double vnorm, double eps,
                        double b);
-int fos_prim_hl_launch(fos_ctx* c, const double* y);  // FP32 (hi, lo) primitives
+int fos_prim_jac_launch(fos_ctx* c, const double* y, float* W);  // the FP32 Jacobian's primitives
 int fos_prim_launch(fos_ctx* c, const double* y);
 int fos_gnn_precond(fos_ctx* c, const double* y, const double* r, double gamma, double* z);
 // fos_jacobian.cu

@@ -261,8 +261,9 @@ gather_fn gather_kernel(int ell_w, int ek) {
 // Layout: 16 floats (64 B) per cell = (rho, u, v, w, H, p) hi, (rho, u, v, w, H, p) lo,
 // sqrt(rho), 0, 0, 0.
 // kV: the state is y + s v (a Jv), else y; a compile-time switch, so a residual issues no
-// predicated-off FP64 FMAs
-template <bool kV>
+// predicated-off FP64 FMAs.  kJac: for the Jacobian, which reads the pairs' FP32 sums only:
+// 8 floats (32 B, one sector) per cell = (u, v, w, H, sqrt(rho), 0, 0, 0)
+template <bool kV, bool kJac = false>
 __global__ void __launch_bounds__(kThreads) k_prim_hl(int nC, const double* __restrict__ y,
                                                       const double* __restrict__ v,
                                                       const double* __restrict__ d_s, double gm1,
@@ -284,6 +285,12 @@ __global__ void __launch_bounds__(kThreads) k_prim_hl(int nC, const double* __re
   const df2 ke = df_add(df_add(df_mul(mx, u), df_mul(my, vv)), df_mul(mz, w));  // rho |u|^2
   const df2 p = df_mul(g, df_add(E, df_scale(ke, -0.5f)));
   const df2 H = df_mul(df_add(E, p), inv);
+  if constexpr (kJac) {
+    float4* w4 = reinterpret_cast<float4*>(W + 8 * (size_t)c);
+    w4[0] = make_float4(u.h + u.l, vv.h + vv.l, w.h + w.l, H.h + H.l);
+    w4[1] = make_float4(sqrtf(r.h + r.l), 0.0f, 0.0f, 0.0f);
+    return;
+  }
   float4* w4 = reinterpret_cast<float4*>(W + 16 * (size_t)c);
   w4[0] = make_float4(r.h, u.h, vv.h, w.h);
   w4[1] = make_float4(H.h, p.h, r.l, u.l);
@@ -642,9 +649,9 @@ int fos_residual_launch(fos_ctx* c, const double* y, const double* v, const doub
   return 0;
 }
 
-int fos_prim_hl_launch(fos_ctx* c, const double* y) {
-  fos_launch(c, k_prim_hl<false>, nblk(c->nC), kThreads, c->nC, y, nullptr, nullptr, c->gamm - 1.0,
-             c->d_Whl);
+int fos_prim_jac_launch(fos_ctx* c, const double* y, float* W) {
+  fos_launch(c, k_prim_hl<false, true>, nblk(c->nC), kThreads, c->nC, y, nullptr, nullptr,
+             c->gamm - 1.0, W);
   FOS_LAUNCH_CHECK();
   return 0;
 }
