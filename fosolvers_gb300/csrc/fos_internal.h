@@ -121,8 +121,11 @@ struct fos_ctx {
   int* d_pnbL = nullptr;
   int* d_pnbU = nullptr;
   int ilu_nbw = 4;
-  int* d_plst = nullptr;      // [nC] storage block of the first L block of every position
-  int* d_pdu = nullptr;       // [nC] storage block of the diagonal block of every position
+  std::vector<int> sw_blocks_f, sw_blocks_b;  // colours: most blocks of a 32-row tile, per level
+  int sw_top0 = 0;            // colours: storage block of the top colour's first diagonal block
+  int sm_count = 0;
+  int* d_plst = nullptr;      // [nC+1] storage block of the first L block of every position
+  int* d_pdu = nullptr;       // [nC+1] storage block of the diagonal block of every position
   int ilu_nlev_f = 0, ilu_nlev_b = 0;
   std::vector<int> lev_f, lev_b;    // level pointers (colour starts when colouring)
   std::vector<char> lev_f_hasL;     // forward level l has L blocks (else y = r there: no launch)

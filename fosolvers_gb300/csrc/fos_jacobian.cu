@@ -926,6 +926,223 @@ __global__ void __launch_bounds__(kT) k_ilu_bwd(int n, const int* __restrict__ r
   ilu_diag_store(lane, a, active, p, acc, Dp, zv);
 }
 
+// ---- the FP32 sweeps of colour-ordered factors (the rows of a level are a range of positions)
+// One warp per block, thread per row, tiles of 32 rows by grid stride.  The blocks a sweep reads
+// for a tile are one contiguous range of the factor, so one bulk copy brings them to shared
+// memory, two tiles in flight, and a lane reads its row's blocks from there: the factor is
+// streamed once, at full width, and marked evict-first so that the vectors the rows gather
+// from stay in the L2.  The gathers of a tile (the neighbours' finished rows, one 32-byte sector
+// each) are issued while the tile before it is computed.  DRAM bounds it (80-85% busy in the
+// large levels).  The five-lanes-per-row kernels above ask the L1 for 20 bytes at a time (88%
+// busy, DRAM at 68%); they remain for level sets, whose rows are scattered, and for FP64 factors,
+// where seven 200-byte blocks a row leave two such warps on an SM and half of its FP64 units
+// idle (hexahedra 47x45x43: 88 us in the sweeps against 51).  A lane forms the row's five sums
+// in the same order: the same bits.  FP32 apply: 80^3 x 6 tetrahedra 510 -> 447 us, 90^3
+// hexahedra 151 -> 120 us, 30^3 x 6 60 -> 50 us, no change below (launches).
+enum { kSwFwd = 0, kSwTop = 1, kSwBwd = 2 };  // y = r - L y; also z = inv(D) y; z = inv(D)(y - U z)
+constexpr int kSwTile = 32;
+constexpr int kSwHead = 16;                // two mbarriers
+constexpr unsigned kSwSpin = 1u << 22;     // tries of one wait before giving up
+constexpr int kSmemMax = 227 * 1024;       // shared memory a block may have
+constexpr int kSmemSm = 228 * 1024;        // and an SM (1 KB of it taken per block)
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) {
+  return (unsigned)__cvta_generic_to_shared(p);
+}
+// the copy's phase has completed; false when the limit ran out (a copy that never lands)
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned phase) {
+  for (unsigned i = 0; i < kSwSpin; i++) {
+    unsigned done;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(bar), "r"(phase)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void bulk_copy(unsigned dst, const void* src, unsigned bytes, unsigned bar,
+                                          unsigned long long policy) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1], %2, [%3], %4;" ::"r"(dst),
+      "l"(src), "r"(bytes), "r"(bar), "l"(policy)
+      : "memory");
+}
+// a row's five values (stored as eight)
+__device__ __forceinline__ void load_row5(const float* v, float x[5]) {
+  const float4 a = *reinterpret_cast<const float4*>(v);
+  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+  x[4] = v[4];
+}
+__device__ __forceinline__ void store_row5(float* v, const float x[5]) {
+  float4* d = reinterpret_cast<float4*>(v);
+  d[0] = make_float4(x[0], x[1], x[2], x[3]);
+  d[1] = make_float4(x[4], 0.0f, 0.0f, 0.0f);
+}
+
+template <int kNW, int kMode>
+__global__ void __launch_bounds__(32) k_sweep(int n, int p0, const int* __restrict__ nbr,
+                                              const int* __restrict__ start, int diag0,
+                                              const float* __restrict__ LU, float* yv, float* zv,
+                                              int stage_blocks) {
+  constexpr int kNB = kNW == 4 ? 4 : 6;        // neighbours of a row (lists are kNW wide)
+  constexpr int kAl = 4;                // floats of 16 bytes
+  extern __shared__ __align__(16) unsigned char sw_smem[];
+  const int lane = threadIdx.x;
+  // stage: the tile's range (aligned down, so up to kAl - 1 elements more), then for kSwTop the
+  // tile's inverted diagonal blocks (likewise)
+  const int n_main = (25 * stage_blocks + 2 * kAl - 1) / kAl * kAl;
+  const int n_diag = kMode == kSwTop ? (25 * kSwTile + 2 * kAl - 1) / kAl * kAl : 0;
+  float* stage0 = reinterpret_cast<float*>(sw_smem + kSwHead);
+  const int n_stage = n_main + n_diag;
+  const unsigned bar0 = smem_addr(sw_smem);
+  unsigned long long policy = 0;
+  if (lane == 0) {
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncwarp();
+  const int ntiles = (n + kSwTile - 1) / kSwTile;
+  const float* gv = kMode == kSwBwd ? zv : yv;  // what the neighbours' rows are read from
+
+  struct Meta {  // a lane's row of a tile: neighbours, first block and the block after its last
+    int q[kNB], off, end;
+  };
+  auto load_meta = [&](int tile, Meta& m) {
+    const int t = tile * kSwTile + lane;
+#pragma unroll
+    for (int k = 0; k < kNB; k++) m.q[k] = -1;
+    m.off = m.end = 0;
+    if (tile < ntiles && t < n) {
+      const int p = p0 + t;
+      const int4 a = __ldg(reinterpret_cast<const int4*>(nbr + (size_t)kNW * p));
+      m.q[0] = a.x; m.q[1] = a.y; m.q[2] = a.z; m.q[3] = a.w;
+      if constexpr (kNB > 4) {
+        const int2 b = __ldg(reinterpret_cast<const int2*>(nbr + (size_t)kNW * p + 4));
+        m.q[4] = b.x; m.q[5] = b.y;
+      }
+      m.off = __ldg(start + p);
+      m.end = __ldg(start + p + 1);
+    }
+  };
+  auto issue = [&](int tile, const Meta& m, int s) {  // copies of the tile into stage s
+    if (tile >= ntiles) return;
+    const int rows = min(kSwTile, n - tile * kSwTile);
+    const int b0 = __shfl_sync(0xffffffffu, m.off, 0), b1 = __shfl_sync(0xffffffffu, m.end, rows - 1);
+    if (lane == 0) {
+      float* dst = stage0 + (size_t)s * n_stage;
+      const unsigned bar = bar0 + 8 * s;
+      const size_t e0 = (25 * (size_t)b0) / kAl * kAl;
+      const unsigned by = b1 > b0 ? (unsigned)((25 * (size_t)b1 - e0 + kAl - 1) / kAl * 16) : 0;
+      size_t d0 = 0;
+      unsigned dby = 0;
+      if constexpr (kMode == kSwTop) {  // the rows' diagonal blocks: one each, from diag0 on
+        const size_t first = 25 * ((size_t)diag0 + (size_t)tile * kSwTile);
+        d0 = first / kAl * kAl;
+        dby = (unsigned)((first + 25 * (size_t)rows - d0 + kAl - 1) / kAl * 16);
+      }
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(by + dby)
+                   : "memory");
+      if (by) bulk_copy(smem_addr(dst), LU + e0, by, bar, policy);
+      if (dby) bulk_copy(smem_addr(dst + n_main), LU + d0, dby, bar, policy);
+    }
+  };
+  auto gather = [&](int tile, const Meta& m, float own[5], float G[kNB][5]) {
+    const int t = tile * kSwTile + lane;
+    if (tile < ntiles && t < n) load_row5(yv + 8 * (size_t)(p0 + t), own);
+#pragma unroll
+    for (int k = 0; k < kNB; k++)
+      if (m.q[k] >= 0) load_row5(gv + 8 * (size_t)m.q[k], G[k]);
+  };
+
+  int tile = blockIdx.x;
+  const int step = gridDim.x;
+  Meta m0, m1, m2;
+  load_meta(tile, m0);
+  load_meta(tile + step, m1);
+  load_meta(tile + 2 * step, m2);
+  issue(tile, m0, 0);
+  issue(tile + step, m1, 1);
+  float own[5], G[kNB][5], own1[5], G1[kNB][5];
+  gather(tile, m0, own, G);
+  unsigned phase = 0;  // bit s: parity of stage s's next completion
+  for (int s = 0; tile < ntiles; tile += step, s ^= 1) {
+    Meta m3;
+    load_meta(tile + 3 * step, m3);
+    gather(tile + step, m1, own1, G1);
+    const bool ok = mbar_wait(bar0 + 8 * s, (phase >> s) & 1u);
+    phase ^= 1u << s;
+    const int t = tile * kSwTile + lane;
+    const int b0 = __shfl_sync(0xffffffffu, m0.off, 0);
+    if (t < n) {
+      const int p = p0 + t;
+      const float* st = stage0 + (size_t)s * n_stage;
+      const float* B = st + (int)((25 * (size_t)b0) % kAl) + 25 * (m0.off - b0);
+      float acc[5];
+#pragma unroll
+      for (int a = 0; a < 5; a++) acc[a] = own[a];
+#pragma unroll
+      for (int k = 0; k < kNB; k++) {
+        if (m0.q[k] >= 0) {
+          const float* Bk = B + 25 * (kMode == kSwBwd ? k + 1 : k);
+#pragma unroll
+          for (int b = 0; b < 5; b++)
+#pragma unroll
+            for (int a = 0; a < 5; a++) acc[a] -= Bk[5 * b + a] * G[k][b];
+        }
+      }
+      if (!ok) {
+#pragma unroll
+        for (int a = 0; a < 5; a++) acc[a] = NAN;
+      }
+      if constexpr (kMode == kSwFwd) {
+        store_row5(yv + 8 * (size_t)p, acc);
+      } else {
+        const float* Dp = B;
+        if constexpr (kMode == kSwTop) {
+          const size_t first = 25 * ((size_t)diag0 + (size_t)tile * kSwTile);
+          Dp = st + n_main + (int)(first % kAl) + 25 * lane;
+        }
+        float z[5];
+#pragma unroll
+        for (int a = 0; a < 5; a++) z[a] = 0.0f;
+#pragma unroll
+        for (int b = 0; b < 5; b++)
+#pragma unroll
+          for (int a = 0; a < 5; a++) z[a] += Dp[5 * b + a] * acc[b];
+        store_row5(zv + 8 * (size_t)p, z);
+      }
+    }
+    __syncwarp();  // every lane is done with stage s
+    issue(tile + 2 * step, m2, s);
+    m0 = m1; m1 = m2; m2 = m3;
+#pragma unroll
+    for (int a = 0; a < 5; a++) own[a] = own1[a];
+#pragma unroll
+    for (int k = 0; k < kNB; k++)
+#pragma unroll
+      for (int a = 0; a < 5; a++) G[k][a] = G1[k][a];
+  }
+}
+// dynamic shared memory of k_sweep
+size_t sweep_smem(int mode, int stage_blocks) {
+  const int n_main = (25 * stage_blocks + 7) / 4 * 4;
+  const int n_diag = mode == kSwTop ? (25 * kSwTile + 7) / 4 * 4 : 0;
+  return kSwHead + 2 * sizeof(float) * (size_t)(n_main + n_diag);
+}
+decltype(&k_sweep<4, kSwFwd>) sweep_kernel(int nbw, int mode) {
+  if (nbw == 4)
+    return mode == kSwFwd ? k_sweep<4, kSwFwd> : mode == kSwTop ? k_sweep<4, kSwTop> : k_sweep<4, kSwBwd>;
+  return mode == kSwFwd ? k_sweep<8, kSwFwd> : mode == kSwTop ? k_sweep<8, kSwTop> : k_sweep<8, kSwBwd>;
+}
+
 }  // namespace
 
 namespace {
@@ -1084,15 +1301,30 @@ int fos_jac_setup(fos_ctx* c) {
     for (int p = c->lev_f[top]; p < c->lev_f[top + 1] && noU; p++) noU = prow[p + 1] == pdiag[p] + 1;
     c->ilu_fuse_top = noU;
   }
-  // factor storage: the L region (every row's L blocks by position), then the D/U region
-  std::vector<int> plst(nC), pdu(nC);
+  // factor storage: the L region (every row's L blocks by position), then the D/U region; one
+  // entry more than rows, so that a row's blocks end where the next row's begin
+  std::vector<int> plst(nC + 1), pdu(nC + 1);
   {
     int nl = 0;
     for (int p = 0; p < nC; p++) {
       plst[p] = nl;
       nl += pdiag[p] - prow[p];
     }
-    for (int p = 0; p < nC; p++) pdu[p] = nl + (prow[p] - plst[p]);
+    plst[nC] = nl;
+    for (int p = 0; p <= nC; p++) pdu[p] = nl + (prow[p] - plst[p]);
+  }
+  // colours: the most blocks that a tile of k_sweep brings to shared memory, per level
+  if (c->ilu_colors) {
+    auto most = [&](const std::vector<int>& lev, const std::vector<int>& at) {
+      std::vector<int> m(lev.size() - 1, 0);
+      for (size_t l = 0; l + 1 < lev.size(); l++)
+        for (int p = lev[l]; p < lev[l + 1]; p += kSwTile)
+          m[l] = std::max(m[l], at[std::min(p + kSwTile, lev[l + 1])] - at[p]);
+      return m;
+    };
+    c->sw_blocks_f = most(c->lev_f, plst);
+    c->sw_blocks_b = most(c->lev_b, pdu);
+    c->sw_top0 = pdu[c->lev_f[c->ilu_colors - 1]];
   }
   // factor update lists (IKJ): for q in lower(p) by position: scale L_pq, then
   // P_pj -= L_pq U_qj for every j in upper(q) that is also in row p
@@ -1129,6 +1361,14 @@ int fos_jac_setup(fos_ctx* c) {
         nbU[(size_t)w * p + (s - pdiag[p] - 1)] = pcol[s];
     }
     if (up(&c->d_pnbL, nbL) || up(&c->d_pnbU, nbU)) return -100;
+  }
+  if (c->ilu_colors) {
+    int sms = 0;
+    FOS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+    c->sm_count = sms;
+    for (int mode : {kSwFwd, kSwTop, kSwBwd})
+      FOS_CUDA(cudaFuncSetAttribute(sweep_kernel(c->ilu_nbw, mode),
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
   }
   c->h_prow = prow;
   c->h_pcol = pcol;
@@ -1282,6 +1522,20 @@ int fos_ilu_factor(fos_ctx* c, double gamma) {
   return 0;
 }
 
+// one level of a colour-ordered FP32 sweep
+static void sweep_level(fos_ctx* c, int mode, int l, const float* LU, float* yv, float* zv) {
+  const std::vector<int>& lev = mode == kSwBwd ? c->lev_b : c->lev_f;
+  const int n = lev[l + 1] - lev[l];
+  const int blocks = (mode == kSwBwd ? c->sw_blocks_b : c->sw_blocks_f)[l];
+  const size_t smem = sweep_smem(mode, blocks);
+  const int per_sm = std::max(1, std::min(24, (int)(kSmemSm / (smem + 1024))));
+  const int grid = std::min((n + kSwTile - 1) / kSwTile, c->sm_count * per_sm);
+  c->n_launch++;
+  sweep_kernel(c->ilu_nbw, mode)<<<grid, 32, smem, c->stream>>>(
+      n, lev[l], mode == kSwBwd ? c->d_pnbU : c->d_pnbL, mode == kSwBwd ? c->d_pdu : c->d_plst,
+      c->sw_top0, LU, yv, zv, blocks);
+}
+
 template <typename TF>
 static int ilu_apply_t(fos_ctx* c, const TF* LU, const double* r, double* z,
                        double* d_zsq = nullptr) {
@@ -1290,18 +1544,27 @@ static int ilu_apply_t(fos_ctx* c, const TF* LU, const double* r, double* z,
   fos_launch(c, k_ilu_in<TF>, nb(c->nC, 256), 256, c->nC, (const int*)c->d_ipos, r, yv);
   const int nf = c->ilu_nlev_f;
   for (int l = 0; l < nf; l++) {
-    const int n = c->lev_f[l + 1] - c->lev_f[l];
-    const int* rows = c->d_lrows_f ? c->d_lrows_f + c->lev_f[l] : nullptr;
     const bool top = c->ilu_fuse_top && l == nf - 1;
     if (!top && !c->lev_f_hasL[l]) continue;  // a level without L blocks keeps y = r
+    if constexpr (sizeof(TF) == 4)
+      if (c->ilu_colors) {
+        sweep_level(c, top ? kSwTop : kSwFwd, l, LU, yv, zv);
+        continue;
+      }
+    const int n = c->lev_f[l + 1] - c->lev_f[l];
+    const int* rows = c->d_lrows_f ? c->d_lrows_f + c->lev_f[l] : nullptr;
     auto k = top ? (c->ilu_nbw == 4 ? k_ilu_fwd<TF, true, 4> : k_ilu_fwd<TF, true, 8>)
                  : (c->ilu_nbw == 4 ? k_ilu_fwd<TF, false, 4> : k_ilu_fwd<TF, false, 8>);
     fos_launch(c, k, nb_rows5(n), kT, n, rows, c->lev_f[l], (const int*)c->d_pnbL,
                (const int*)c->d_plst, (const int*)c->d_pdu, LU, yv, zv);
   }
   for (int l = c->ilu_fuse_top ? 1 : 0; l < c->ilu_nlev_b; l++) {
-    // colours run backwards for the upper sweep
-    const int lc = c->ilu_colors ? c->ilu_nlev_b - 1 - l : l;
+    const int lc = c->ilu_colors ? c->ilu_nlev_b - 1 - l : l;  // colours run backwards here
+    if constexpr (sizeof(TF) == 4)
+      if (c->ilu_colors) {
+        sweep_level(c, kSwBwd, lc, LU, yv, zv);
+        continue;
+      }
     const int n = c->lev_b[lc + 1] - c->lev_b[lc];
     const int* rows = c->d_lrows_b ? c->d_lrows_b + c->lev_b[lc] : nullptr;
     fos_launch(c, c->ilu_nbw == 4 ? k_ilu_bwd<TF, 4> : k_ilu_bwd<TF, 8>, nb_rows5(n), kT, n,
