@@ -107,42 +107,105 @@ struct PrimT {
   T u[3], H, s;
 };
 
-// Blocks of face f from its two sides' primitives (Roe averages, Euler.f90:207-209): both
-// off-diagonal blocks of an interior face, or the boundary pair's diagonal term
-template <typename T, typename TJ>
-__device__ __forceinline__ void jac_face_blocks(int f, int nFi, const T n[3], T aP,
-                                                const PrimT<T>& L, const PrimT<T>& R, T gg,
-                                                const int* __restrict__ fslot,
-                                                TJ* __restrict__ J, TJ* __restrict__ Jb) {
-  const T inv = T(1) / (L.s + R.s);
-  const T ua[3] = {(L.s * L.u[0] + R.s * R.u[0]) * inv, (L.s * L.u[1] + R.s * R.u[1]) * inv,
-                   (L.s * L.u[2] + R.s * R.u[2]) * inv};
-  const T Ha = (L.s * L.H + R.s * R.H) * inv;
-  const T ca = sqrt((gg - T(1)) * (Ha - T(0.5) * (ua[0] * ua[0] + ua[1] * ua[1] + ua[2] * ua[2])));
-  T Ab[25];
-  anfj<T>(n, ua, Ha, ca, gg, Ab);
-  const T v2L = L.u[0] * L.u[0] + L.u[1] * L.u[1] + L.u[2] * L.u[2];
-  const T vnL = L.u[0] * n[0] + L.u[1] * n[1] + L.u[2] * n[2];
-  const T v2R = R.u[0] * R.u[0] + R.u[1] * R.u[1] + R.u[2] * R.u[2];
-  const T vnR = R.u[0] * n[0] + R.u[1] * n[1] + R.u[2] * n[2];
-  const T h = T(0.5) * aP;
+// h A~ - h F'(U) (S < 0) or h A~ + h F'(U) (S > 0), A~ = |A~| of the face, F' = eulerNFJ with
+// hn = h n: the entries of one off-diagonal block, two FMAs each at most (u and H of the side,
+// hvn = u . hn, g1n = (g - 1) hn)
+template <int S>
+__device__ __forceinline__ void jac_block64(const double A[25], const double hn[3], const double g1n[3],
+                                            const double u[3], double H, double g, double out[25]) {
+  constexpr double s = S;
+  const double g1 = g - 1.0;
+  const double hvn = fma(u[2], hn[2], fma(u[1], hn[1], u[0] * hn[0]));
+  const double k = 0.5 * g1 * fma(u[2], u[2], fma(u[1], u[1], u[0] * u[0]));
+  const double shv = s * hvn, g1v = g1 * shv;
+  out[0] = A[0];
+  out[4] = A[4];
+#pragma unroll
+  for (int j = 0; j < 3; j++) out[1 + j] = A[1 + j] + s * hn[j];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const int r = 5 * (1 + i);
+    out[r] = fma(s * hn[i], k, fma(-u[i], shv, A[r]));
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      const double t = fma(s * u[i], hn[j], fma(-s * g1n[i], u[j], A[r + 1 + j]));
+      out[r + 1 + j] = i == j ? t + shv : t;
+    }
+    out[r + 4] = A[r + 4] + s * g1n[i];
+  }
+  out[20] = fma(k - H, shv, A[20]);
+#pragma unroll
+  for (int j = 0; j < 3; j++) out[21 + j] = fma(s * H, hn[j], fma(-g1v, u[j], A[21 + j]));
+  out[24] = fma(g, shv, A[24]);
+}
+
+// Blocks of face f from its two sides' primitives (Roe averages, Euler.f90:207-209), FP64: both
+// off-diagonal blocks of an interior face, or the boundary pair's diagonal term.  The FP64 pipe
+// bounds it, so the half area h is folded into the normal and the wave weights, |A~| (anfj's
+// decomposition) is built with one FMA per rank-1 term, and each block adds its side's eulerNFJ
+// to it with two: about 240 FP64 instructions a face instead of 370.  Set-up and one apply on
+// 47x45x43 hexahedra, with the diagonal kernel and the Gauss--Jordan step below: 625 -> 524 us.
+__device__ __forceinline__ void jac_face_blocks(int f, int nFi, const double n[3], double aP,
+                                                const PrimT<double>& L, const PrimT<double>& R,
+                                                double g, const int* __restrict__ fslot,
+                                                double* __restrict__ J, double* __restrict__ Jb) {
+  const double g1 = g - 1.0, h = 0.5 * aP;
+  const double wR = R.s * rcp64(L.s + R.s);
+  double u[3], hn[3], g1n[3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    u[i] = fma(wR, R.u[i] - L.u[i], L.u[i]);
+    hn[i] = h * n[i];
+    g1n[i] = g1 * hn[i];
+  }
+  const double H = fma(wR, R.H - L.H, L.H);
+  const double hq = 0.5 * fma(u[2], u[2], fma(u[1], u[1], u[0] * u[0]));
+  const double vn = fma(u[2], n[2], fma(u[1], n[1], u[0] * n[0]));
+  double c;
+  const double ic = rsqrt64(g1 * (H - hq), c);
+  const double av = fabs(vn), hav = h * av, k = 0.5 * h * ic * ic;
+  const double wm = k * (fabs(vn - c) - av), wp = k * (fabs(vn + c) - av);
+  const double g1q = g1 * hq, cv = c * vn;
+  double lm[5], lp[5], cn[3], A[25];
+  lm[0] = wm * (g1q + cv);
+  lp[0] = wp * (g1q - cv);
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    cn[j] = c * n[j];
+    lm[1 + j] = -wm * fma(g1, u[j], cn[j]);
+    lp[1 + j] = -wp * fma(g1, u[j], -cn[j]);
+  }
+  lm[4] = wm * g1;
+  lp[4] = wp * g1;
+#pragma unroll
+  for (int b = 0; b < 5; b++) {
+    const double sum = lm[b] + lp[b];
+    A[b] = b == 0 ? sum + hav : sum;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const double base = b == 0 ? -hav * u[i] : b == 1 + i ? hav : 0.0;
+      A[5 * (1 + i) + b] = fma(u[i] - cn[i], lm[b], b == 0 || b == 1 + i
+                                                        ? fma(u[i] + cn[i], lp[b], base)
+                                                        : (u[i] + cn[i]) * lp[b]);
+    }
+    const double p4 = b == 4 ? fma(H + cv, lp[b], hav) : (H + cv) * lp[b];
+    A[20 + b] = fma(H - cv, lm[b], p4);
+  }
+  double o[25];
   if (f < nFi) {
-    TJ* oLR = J + 25 * (size_t)fslot[2 * f];      // block (L, R) = JacP(1:5,6:10)
-    TJ* oRL = J + 25 * (size_t)fslot[2 * f + 1];  // block (R, L) = JacP(6:10,1:5)
+    double* oLR = J + 25 * (size_t)fslot[2 * f];      // block (L, R) = JacP(1:5,6:10)
+    double* oRL = J + 25 * (size_t)fslot[2 * f + 1];  // block (R, L) = JacP(6:10,1:5)
+    jac_block64<-1>(A, hn, g1n, R.u, R.H, g, o);
 #pragma unroll
-    for (int a = 0; a < 5; a++)
+    for (int q = 0; q < 25; q++) oLR[q] = o[q];
+    jac_block64<1>(A, hn, g1n, L.u, L.H, g, o);
 #pragma unroll
-      for (int b = 0; b < 5; b++) {
-        oLR[5 * a + b] = (TJ)(-h * (nfj<T>(a, b, n, R.u, R.H, gg, v2R, vnR) - Ab[5 * a + b]));
-        oRL[5 * a + b] = (TJ)(h * (nfj<T>(a, b, n, L.u, L.H, gg, v2L, vnL) + Ab[5 * a + b]));
-      }
+    for (int q = 0; q < 25; q++) oRL[q] = o[q];
   } else {
-    TJ* d = Jb + 25 * (size_t)(f - nFi);  // boundary pair's diagonal term
+    double* d = Jb + 25 * (size_t)(f - nFi);  // boundary pair's diagonal term
+    jac_block64<1>(A, hn, g1n, L.u, L.H, g, o);
 #pragma unroll
-    for (int a = 0; a < 5; a++)
-#pragma unroll
-      for (int b = 0; b < 5; b++)
-        d[5 * a + b] = (TJ)(-h * (nfj<T>(a, b, n, L.u, L.H, gg, v2L, vnL) + Ab[5 * a + b]));
+    for (int q = 0; q < 25; q++) d[q] = neg_bits(o[q]);
   }
 }
 
@@ -187,7 +250,6 @@ __global__ void __launch_bounds__(kT) k_jac_ghost64(int nFi, int nF, int nC,
 }
 
 // FP64 form: FP64 primitives and geometry
-template <typename TJ>
 __global__ void __launch_bounds__(kT) k_jac_face(int nFi, int nF, int nC,
                                                  const int2* __restrict__ faceLR,
                                                  const double2* __restrict__ faceNA,
@@ -196,8 +258,8 @@ __global__ void __launch_bounds__(kT) k_jac_face(int nFi, int nF, int nC,
                                                  const int* __restrict__ fslot,
                                                  const int* __restrict__ bcT,
                                                  const double* __restrict__ bcP, int maxP,
-                                                 double g, double r, TJ* __restrict__ J,
-                                                 TJ* __restrict__ Jb) {
+                                                 double g, double r, double* __restrict__ J,
+                                                 double* __restrict__ Jb) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nF) return;
   const int2 lr = faceLR[f];
@@ -208,7 +270,7 @@ __global__ void __launch_bounds__(kT) k_jac_face(int nFi, int nF, int nC,
   if (f < nFi) load_prim(W, lr.y, R);
   else ghost_prim(f, nC, lr, y, bcT, bcP, maxP, n01.x, n01.y, n2a.x, g, r, R);
   const PrimT<double> PL = {{L.u, L.v, L.w}, L.H, L.s}, PR = {{R.u, R.v, R.w}, R.H, R.s};
-  jac_face_blocks<double, TJ>(f, nFi, n, n2a.y, PL, PR, g, fslot, J, Jb);
+  jac_face_blocks(f, nFi, n, n2a.y, PL, PR, g, fslot, J, Jb);
 }
 
 // FP32 form: FP32 arithmetic from the per-cell primitives (double-float, rounded to FP32) and
@@ -371,58 +433,33 @@ __global__ void __launch_bounds__(64) k_jac_cell32(
   }
 }
 
-template <typename TJ>
+// Diagonal blocks of the FP64 form, five lanes per cell (lane a sums row a, so that a block is
+// read and written as 200 consecutive bytes), the cell's faces in ascending order.
 __global__ void __launch_bounds__(kT) k_jac_diag(int nC, int nFi, const int* __restrict__ crow,
                                                  const int* __restrict__ cent,
                                                  const int* __restrict__ fslot,
                                                  const int* __restrict__ cdiag,
-                                                 const TJ* __restrict__ Jb,
-                                                 TJ* __restrict__ J) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nC) return;
-  TJ D[25];
-#pragma unroll
-  for (int k = 0; k < 25; k++) D[k] = TJ(0);
-  for (int e = crow[c]; e < crow[c + 1]; e++) {
+                                                 const double* __restrict__ Jb,
+                                                 double* __restrict__ J) {
+  const int lane = threadIdx.x & 31;
+  const int sub = lane / 5, a = lane - 5 * sub;
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) / 32 * 6 + sub;
+  if (sub >= 6 || c >= nC) return;
+  double D[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  const int e0 = crow[c], e1 = crow[c + 1];
+#pragma unroll 6
+  for (int e = e0; e < e1; e++) {
     const int ent = cent[e], f = ent >> 1;
-    if (f < nFi) {
-      // cell is L: diag += JacP(1:5,1:5) = -block(R,L); cell is R: diag += -block(L,R)
-      const TJ* o = J + 25 * (size_t)fslot[2 * f + ((ent & 1) ? 0 : 1)];
+    // cell is L: diag += JacP(1:5,1:5) = -block(R,L); cell is R: diag += -block(L,R)
+    const double* o = f < nFi ? J + 25 * (size_t)fslot[2 * f + ((ent & 1) ? 0 : 1)]
+                              : Jb + 25 * (size_t)(f - nFi);
+    const int flip = f < nFi ? (int)0x80000000u : 0;
 #pragma unroll
-      for (int k = 0; k < 25; k++) D[k] -= o[k];
-    } else {
-      const TJ* o = Jb + 25 * (size_t)(f - nFi);
-#pragma unroll
-      for (int k = 0; k < 25; k++) D[k] += o[k];
-    }
+    for (int k = 0; k < 5; k++) D[k] += flip_sign(o[5 * a + k], flip);
   }
-  TJ* dst = J + 25 * (size_t)cdiag[c];
+  double* dst = J + 25 * (size_t)cdiag[c] + 5 * a;
 #pragma unroll
-  for (int k = 0; k < 25; k++) dst[k] = D[k];
-}
-
-// invert a 5x5 block in place by Gauss--Jordan without pivoting (scalar ilu0 eliminates
-// inside the diagonal block without pivoting too, ilut.f:1893-1898); false on a zero pivot
-template <typename T>
-__device__ __forceinline__ bool inv5(T a[25]) {
-  bool ok = true;
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    const T piv = a[5 * k + k];
-    ok &= (piv != T(0));
-    const T ip = T(1) / piv;
-    // row k scaled; column k becomes the inverse's column
-#pragma unroll
-    for (int j = 0; j < 5; j++) a[5 * k + j] = (j == k) ? ip : a[5 * k + j] * ip;
-#pragma unroll
-    for (int i = 0; i < 5; i++) {
-      if (i == k) continue;
-      const T f = a[5 * i + k];
-#pragma unroll
-      for (int j = 0; j < 5; j++) a[5 * i + j] = (j == k) ? -f * ip : a[5 * i + j] - f * a[5 * k + j];
-    }
-  }
-  return ok;
+  for (int k = 0; k < 5; k++) dst[k] = D[k];
 }
 
 // One level of the block ILU(0) factorisation.  Five lanes per block row p (lane a owns
@@ -441,14 +478,9 @@ __device__ __forceinline__ bool inv5(T a[25]) {
 // factors (k_ilu_factor, k_pset32) rounds the same way:
 //   (A B)(i, b) = sum_k A(i, k) B(k, b), k ascending, one fused multiply-add per term;
 //   Gauss--Jordan step k on row a of D with rk = row k before the step.
-__device__ __forceinline__ float ilu_dot5(const float A[5], const float* Bcol) {
-  float acc = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 5; k++) acc = fmaf(A[k], Bcol[k], acc);
-  return acc;
-}
-__device__ __forceinline__ double ilu_dot5(const double A[5], const double* Bcol) {
-  double acc = 0.0;
+template <typename TF>
+__device__ __forceinline__ TF ilu_dot5(const TF A[5], const TF* Bcol) {
+  TF acc = TF(0);
 #pragma unroll
   for (int k = 0; k < 5; k++) acc = fma(A[k], Bcol[k], acc);
   return acc;
@@ -459,15 +491,19 @@ __device__ __forceinline__ TF ilu_mul(TF a, TF b) {
 }
 template <typename TF>
 __device__ __forceinline__ void ilu_gj_step(int a, int k, const TF rk[5], TF Da[5]) {
-  const TF ip = TF(1) / rk[k];
-  if (a == k) {
+  TF ip;
+  if constexpr (sizeof(TF) == 4) ip = 1.0f / rk[k]; else ip = rcp64(rk[k]);
+  const bool own = a == k;  // row k itself becomes the scaled row
+  const TF f = Da[k];
 #pragma unroll
-    for (int b = 0; b < 5; b++) Da[b] = (b == k) ? ip : ilu_mul(rk[b], ip);
-  } else {
-    const TF f = Da[k];
-#pragma unroll
-    for (int b = 0; b < 5; b++) Da[b] = (b == k) ? -ilu_mul(f, ip) : fma(-f, ilu_mul(rk[b], ip), Da[b]);
+  for (int b = 0; b < 5; b++) {
+    if (b == k) continue;
+    const TF t = ilu_mul(rk[b], ip);
+    const TF v = fma(-f, t, Da[b]);
+    Da[b] = own ? t : v;
   }
+  const TF v = -ilu_mul(f, ip);
+  Da[k] = own ? ip : v;
 }
 
 template <typename TF>
@@ -1411,7 +1447,6 @@ template <typename TJ>
 static int jac_assemble_t(fos_ctx* c, const double* y) {
   if (int rc = ensure_jraw(c)) return rc;
   TJ* J = reinterpret_cast<TJ*>(c->d_Jraw);
-  TJ* Jb = reinterpret_cast<TJ*>(c->d_Jb);
   if constexpr (sizeof(TJ) == sizeof(float)) {
     float* wj = reinterpret_cast<float*>(c->d_W);  // (every user of d_W writes it first)
     if (int rc = fos_prim_jac_launch(c, y, wj)) return rc;
@@ -1435,17 +1470,18 @@ static int jac_assemble_t(fos_ctx* c, const double* y) {
     FOS_LAUNCH_CHECK();
     return 0;
   } else {
+    double* Jb = reinterpret_cast<double*>(c->d_Jb);
     if (int rc = fos_prim_launch(c, y)) return rc;
-    fos_launch(c, k_jac_face<TJ>, nb(c->nF), kT, c->nFi, c->nF, c->nC,
+    fos_launch(c, k_jac_face, nb(c->nF), kT, c->nFi, c->nF, c->nC,
                (const int2*)c->d_faceLR, (const double2*)c->d_faceNA, (const double*)c->d_W, y,
                (const int*)c->d_fslot, (const int*)c->d_bcT, (const double*)c->d_bcP, c->maxP,
                c->gamm, c->r, J, Jb);
+    fos_launch(c, k_jac_diag, nb_rows5(c->nC), kT, c->nC, c->nFi, (const int*)c->d_crow,
+               (const int*)c->d_cent, (const int*)c->d_fslot, (const int*)c->d_cdiag,
+               (const double*)Jb, J);
+    FOS_LAUNCH_CHECK();
+    return 0;
   }
-  fos_launch(c, k_jac_diag<TJ>, nb(c->nC), kT, c->nC, c->nFi, (const int*)c->d_crow,
-             (const int*)c->d_cent, (const int*)c->d_fslot, (const int*)c->d_cdiag,
-             (const TJ*)Jb, J);
-  FOS_LAUNCH_CHECK();
-  return 0;
 }
 
 int fos_jac_assemble(fos_ctx* c, const double* y) {
