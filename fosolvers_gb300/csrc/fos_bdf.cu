@@ -77,6 +77,7 @@ template <int NV, bool NRM>
 __global__ void __launch_bounds__(kT) k_mdot(long n, const double* __restrict__ V, long ldv,
                                              const double* __restrict__ w,
                                              double* __restrict__ part) {
+  pdl_entry();
   constexpr int NA = NV + (NRM ? 1 : 0);
   double acc[NA];
 #pragma unroll
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(kT) k_update(long n, const double* __restrict_
                                                const double* __restrict__ s2,
                                                double* __restrict__ w,
                                                double* __restrict__ part) {
+  pdl_entry();
   __shared__ double hs[NV];
   if (threadIdx.x < NV) hs[threadIdx.x] = s2 ? h[threadIdx.x] * s2[threadIdx.x] : h[threadIdx.x];
   __syncthreads();
@@ -128,6 +130,7 @@ __global__ void __launch_bounds__(kT) k_update(long n, const double* __restrict_
 
 // out[l] = sum of part[l * np ...]
 __global__ void k_final(int nv, int np, const double* __restrict__ part, double* __restrict__ out) {
+  pdl_entry();
   const int l = blockIdx.x;
   if (l >= nv) return;
   double s = 0.0;
@@ -144,10 +147,12 @@ __global__ void k_final(int nv, int np, const double* __restrict__ part, double*
 }
 
 __global__ void k_scale(long n, const double* __restrict__ x, double a, double* __restrict__ y) {
+  pdl_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = a * x[i];
 }
 __global__ void k_axpy(long n, double a, const double* __restrict__ x, double* __restrict__ y) {
+  pdl_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] += a * x[i];
 }
@@ -159,6 +164,7 @@ template <bool kAcc, bool kAdd>
 __global__ void k_comb(long n, int nv, const double* __restrict__ Z, long ldz,
                        const double* __restrict__ cc, double* __restrict__ x,
                        double* __restrict__ yadd) {
+  pdl_entry();
   __shared__ double cs[kMaxVec];
   if (threadIdx.x < kMaxVec) cs[threadIdx.x] = threadIdx.x < nv ? cc[threadIdx.x] : 0.0;
   __syncthreads();
@@ -180,6 +186,7 @@ __global__ void k_comb(long n, int nv, const double* __restrict__ Z, long ldz,
 // hist = y_n (q=1) or 4/3 y_n - 1/3 y_{n-1} (q=2)
 __global__ void k_hist(long n, int q, const double* __restrict__ yn, const double* __restrict__ ym,
                        double* __restrict__ h) {
+  pdl_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   h[i] = q == 1 ? yn[i] : (4.0 / 3.0) * yn[i] - (1.0 / 3.0) * ym[i];
@@ -190,6 +197,7 @@ __global__ void k_hist(long n, int q, const double* __restrict__ yn, const doubl
 template <int P>
 __global__ void k_predict(long n, const double* __restrict__ yn, const double* __restrict__ ym,
                           const double* __restrict__ ym2, double* __restrict__ y) {
+  pdl_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double dlt = __dsub_rn(yn[i], ym[i]);
@@ -203,6 +211,7 @@ __global__ void __launch_bounds__(kT) k_newton_res(long n, const double* __restr
                                                    double gamma, double* __restrict__ b,
                                                    double* __restrict__ b2,
                                                    double* __restrict__ part) {
+  pdl_entry();
   double acc[2] = {0.0, 0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const double yi = y[i];
@@ -224,6 +233,7 @@ struct Comb8 {
   int nv;
 };
 __global__ void k_lincomb(long n, Comb8 cb, double* __restrict__ out) {
+  pdl_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double s = 0.0;
@@ -234,6 +244,7 @@ __global__ void k_lincomb(long n, Comb8 cb, double* __restrict__ out) {
 __global__ void __launch_bounds__(kT) k_wrms_part(long n, const double* __restrict__ a,
                                                   const double* __restrict__ w, double rtol,
                                                   double atol, double* __restrict__ part) {
+  pdl_entry();
   double acc[1] = {0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const double e = a[i] / (rtol * fabs(w[i]) + atol);

@@ -120,6 +120,7 @@ __global__ void __launch_bounds__(256) k_gnn_in(int nC, const double* __restrict
                                                 const GnnScales* __restrict__ sc,
                                                 float* __restrict__ X0,
                                                 unsigned short* __restrict__ h0) {
+  pdl_entry();
   __shared__ __align__(16) float xs[256][NIN];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int f0 = 2 * lane;
@@ -232,6 +233,7 @@ __global__ void __launch_bounds__(kT) k_gnn_layer(
     const unsigned short* __restrict__ hin, unsigned short* __restrict__ hout,
     unsigned short* __restrict__ mkeep, const float* __restrict__ Wb,
     const double* __restrict__ v, double* __restrict__ z, float* __restrict__ zhat) {
+  pdl_entry();
   constexpr int RS = 2 * H + 8;  // row stride (bf16) of the tiles: 272 B, 16-byte aligned
   __shared__ __align__(16) unsigned short Xs[kTile][RS];   // [h ; m], then the layer output
   __shared__ __align__(16) unsigned short As[H][RS];
@@ -402,6 +404,7 @@ __global__ void __launch_bounds__(256) k_gnn_scale_part(int nC, int nF, const do
                                                         const double* __restrict__ invV,
                                                         const float4* __restrict__ faceNA,
                                                         float* __restrict__ part) {
+  pdl_entry();
   float acc[10] = {0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nC; i += gridDim.x * blockDim.x) {
     const float r = d2f_trunc(y[i]);
@@ -436,6 +439,7 @@ __global__ void __launch_bounds__(256) k_gnn_scale_part(int nC, int nF, const do
 }
 __global__ void k_gnn_scale_final(int nC, int nF, int np, const float* __restrict__ part,
                                   GnnScales* __restrict__ sc) {
+  pdl_entry();
   // one warp: lane l sums partials l, l+32, ... (fixed order), then a shuffle tree
   const int lane = threadIdx.x & 31;
   float s[10] = {0};
@@ -467,6 +471,7 @@ __global__ void __launch_bounds__(256) k_gnn_out_bwd(int nC, const float* __rest
                                                      const float* __restrict__ Wb, float invN,
                                                      float* __restrict__ dh3,
                                                      float* __restrict__ part) {
+  pdl_entry();
   // part layout per block: [0] loss, [1..5] dd, [6 .. 6+5*64) dD
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const GnnScales s = *sc;
@@ -539,6 +544,7 @@ __global__ void __launch_bounds__(kT) k_gnn_layer_bwd(
     const unsigned short* __restrict__ hout, const float* __restrict__ dhout,
     const unsigned short* __restrict__ Ab, float* __restrict__ dhin, float* __restrict__ dm,
     float* __restrict__ part) {
+  pdl_entry();
   __shared__ __align__(16) unsigned short Xs[kTile][2 * H + 8];   // [h_in ; m] rows
   __shared__ __align__(16) unsigned short Ds[kTile][H + 8];       // bf16(delta) rows
   __shared__ __align__(16) unsigned short As[H][2 * H + 8];
@@ -653,6 +659,7 @@ __global__ void __launch_bounds__(kT) k_gnn_edge_bwd(
     const float4* __restrict__ faceNA, const GnnScales* __restrict__ sc,
     const float* __restrict__ Wl, const unsigned short* __restrict__ hin,
     const float* __restrict__ dm, float* __restrict__ dhin, float* __restrict__ part) {
+  pdl_entry();
   __shared__ float Gs[H * 5];
   __shared__ float acc_s[kT / 32][H * 5];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -709,6 +716,7 @@ __global__ void __launch_bounds__(256) k_gnn_in_bwd(int nC, const float* __restr
                                                     const unsigned short* __restrict__ h0,
                                                     const float* __restrict__ dh0,
                                                     float* __restrict__ part) {
+  pdl_entry();
   __shared__ float red[8][H * NIN + H];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   // warp per cell: lane owns features 2 lane, 2 lane + 1
@@ -751,6 +759,7 @@ __global__ void __launch_bounds__(256) k_gnn_in_bwd(int nC, const float* __restr
 
 // [loss, dd(5), dD(5 x 64)] -> gradient of d and of the first five rows of D
 __global__ void k_gnn_head_grad(const float* __restrict__ hs, float* __restrict__ grad) {
+  pdl_entry();
   for (int k = threadIdx.x; k < 5 + 5 * H; k += blockDim.x) {
     if (k < 5) grad[OFF_DB + k] += hs[1 + k];
     else grad[OFF_D + (k - 5)] += hs[1 + k];
@@ -760,6 +769,7 @@ __global__ void k_gnn_head_grad(const float* __restrict__ hs, float* __restrict_
 // sum np partial vectors of length len (fixed order) into dst (+= when accumulate)
 __global__ void k_sum_parts(int np, int len, const float* __restrict__ part,
                             float* __restrict__ dst, float scale) {
+  pdl_entry();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= len) return;
   float s = 0.0f;
@@ -771,6 +781,7 @@ __global__ void k_sum_parts(int np, int len, const float* __restrict__ part,
 __global__ void k_adam(int n, float* __restrict__ w, const float* __restrict__ gr,
                        float* __restrict__ m1, float* __restrict__ m2, float lr, float b1,
                        float b2, float eps, float c1, float c2, float* __restrict__ wb) {
+  pdl_entry();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const float g = gr[k];
@@ -783,10 +794,12 @@ __global__ void k_adam(int n, float* __restrict__ w, const float* __restrict__ g
   wb[k] = __bfloat162float(__float2bfloat16_rn(nw));
 }
 __global__ void k_round_bf16(int n, const float* __restrict__ w, float* __restrict__ wb) {
+  pdl_entry();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) wb[k] = __bfloat162float(__float2bfloat16_rn(w[k]));
 }
 __global__ void k_layer_bits(const float* __restrict__ wb, unsigned short* __restrict__ Ab) {
+  pdl_entry();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= NL * H * 2 * H) return;
   const int l = k / (H * 2 * H), r = k % (H * 2 * H);

@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(32 * kWarps) k_ilut_factor(
     double* __restrict__ Uval, int* __restrict__ Ucnt, double* __restrict__ dinv,
     int* __restrict__ levL, int* __restrict__ done, int* __restrict__ ctr, long spin,
     int withhold) {
+  pdl_entry();
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned hmask = 4u * cap - 1u;
@@ -391,6 +392,7 @@ __device__ __forceinline__ double wait_value(const double* x, int j, double v, i
 }
 
 __global__ void k_fill_pending(long n, double* __restrict__ x) {
+  pdl_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) x[i] = __longlong_as_double((long long)kPending);
 }
@@ -433,6 +435,7 @@ __global__ void __launch_bounds__(256) k_ilut_fwd(int n, int lfil, const int* __
                                                   const double* y, double* z, double* x,
                                                   int* __restrict__ ctr, long spin,
                                                   int withhold) {
+  pdl_entry();
   const int lane = threadIdx.x & 31;
   const size_t slot = (size_t)(lfil > 0 ? lfil : 1);
   for (;;) {
@@ -460,6 +463,7 @@ __global__ void __launch_bounds__(256) k_ilut_bwd(int n, int lfil, const int* __
                                                   const int* __restrict__ perm,
                                                   const double* __restrict__ z, double* x,
                                                   int* __restrict__ ctr, long spin) {
+  pdl_entry();
   const int lane = threadIdx.x & 31;
   const size_t slot = (size_t)(lfil > 0 ? lfil : 1);
   for (;;) {
@@ -479,6 +483,7 @@ __global__ void __launch_bounds__(256) k_ilut_bwd(int n, int lfil, const int* __
 // column in [0, n); bad[0] = 1 + first failing row
 __global__ void k_ilut_check(int n, const int* __restrict__ ia, const int* __restrict__ ja,
                              int* __restrict__ bad) {
+  pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int b = ia[i], e = ia[i + 1];
@@ -806,6 +811,7 @@ extern "C" int fos_ilut_info(const fos_ilut* f, long* out) {
 namespace {
 
 __global__ void k_pcsr_rows(int nC, const int* __restrict__ prow, int* __restrict__ ia) {
+  pdl_entry();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r > 5 * nC) return;
   if (r == 5 * nC) { ia[r] = 25 * prow[nC]; return; }
@@ -815,6 +821,7 @@ __global__ void k_pcsr_rows(int nC, const int* __restrict__ prow, int* __restric
 
 __global__ void k_pcsr_cols(int nC, const int* __restrict__ prow, const int* __restrict__ pcol,
                             int* __restrict__ ja) {
+  pdl_entry();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= 5 * nC) return;
   const int p = r / 5, a = r - 5 * p, s0 = prow[p], nb = prow[p + 1] - s0;
@@ -828,6 +835,7 @@ template <typename TJ>
 __global__ void k_pcsr_vals(int nC, const int* __restrict__ prow, const int* __restrict__ pdiag,
                             const int* __restrict__ ord, const double* __restrict__ vol,
                             double gamma, const TJ* __restrict__ J, double* __restrict__ A) {
+  pdl_entry();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= 5 * nC) return;
   const int p = r / 5, a = r - 5 * p, s0 = prow[p], nb = prow[p + 1] - s0;
@@ -842,6 +850,7 @@ __global__ void k_pcsr_vals(int nC, const int* __restrict__ prow, const int* __r
 
 __global__ void k_ilut_in(int nC, const int* __restrict__ ipos, const double* __restrict__ r,
                           double* __restrict__ x) {
+  pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nC) return;
   const size_t q = 5 * (size_t)ipos[i];
@@ -851,6 +860,7 @@ __global__ void k_ilut_in(int nC, const int* __restrict__ ipos, const double* __
 
 __global__ void k_ilut_out(int nC, const int* __restrict__ ipos, const double* __restrict__ x,
                            double* __restrict__ z) {
+  pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nC) return;
   const size_t q = 5 * (size_t)ipos[i];

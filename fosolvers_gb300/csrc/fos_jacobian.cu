@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(kT) k_jac_ghost64(int nFi, int nF, int nC,
                                                     const int* __restrict__ bcT,
                                                     const double* __restrict__ bcP, int maxP,
                                                     double g, double r, double* __restrict__ Gb) {
+  pdl_entry();
   const int f = nFi + blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nF) return;
   const int2 lr = __ldg(faceLR + f);
@@ -260,6 +261,7 @@ __global__ void __launch_bounds__(kT) k_jac_face(int nFi, int nF, int nC,
                                                  const double* __restrict__ bcP, int maxP,
                                                  double g, double r, double* __restrict__ J,
                                                  double* __restrict__ Jb) {
+  pdl_entry();
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nF) return;
   const int2 lr = faceLR[f];
@@ -403,6 +405,7 @@ __global__ void __launch_bounds__(64) k_jac_cell32(
     const float4* __restrict__ cna, const int* __restrict__ fslot,
     const float* __restrict__ Wj, const double* __restrict__ Gb, const float4* __restrict__ Sc,
     double g, float* __restrict__ J) {
+  pdl_entry();
   constexpr int kRow = (kW + 1) * 25;  // floats of a full block row
   __shared__ float stg[2][32][kRow];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -441,6 +444,7 @@ __global__ void __launch_bounds__(kT) k_jac_diag(int nC, int nFi, const int* __r
                                                  const int* __restrict__ cdiag,
                                                  const double* __restrict__ Jb,
                                                  double* __restrict__ J) {
+  pdl_entry();
   const int lane = threadIdx.x & 31;
   const int sub = lane / 5, a = lane - 5 * sub;
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) / 32 * 6 + sub;
@@ -525,6 +529,7 @@ __global__ void __launch_bounds__(kT) k_ilu_factor(
     double gamma, const TJ* __restrict__ J, const int* __restrict__ upd_ptr,
     const int3* __restrict__ upd, const int* __restrict__ plst, const int* __restrict__ pdu,
     TF* __restrict__ LU, int* __restrict__ ierr) {
+  pdl_entry();
   // update operands (inv(D_q), U_qj of earlier levels) of the first kPre operations of a row
   // are fetched into shared memory before the elimination, all loads in flight at once
   constexpr int kPre = sizeof(TF) == 4 ? 8 : 0;
@@ -674,6 +679,7 @@ __global__ void __launch_bounds__(32) k_pset32(
     double g, const int* __restrict__ upd_ptr, const int3* __restrict__ upd,
     const int* __restrict__ plst, const int* __restrict__ pdu, float* LU,
     int* __restrict__ ierr) {
+  pdl_entry();
   constexpr int kRow = kW * 25 + 1;  // odd: the lanes' rows fall in distinct banks
   constexpr int kSlots = kW == 4 ? 4 : 8;
   __shared__ __align__(16) float stg[32][kRow];  // the off-diagonal blocks, in slot order
@@ -795,6 +801,7 @@ __global__ void __launch_bounds__(32) k_pset32(
 template <typename TF>
 __global__ void k_ilu_in(int nC, const int* __restrict__ ipos, const double* __restrict__ r,
                          TF* __restrict__ rv) {
+  pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nC) return;
   TF v[8];
@@ -816,6 +823,7 @@ __global__ void k_ilu_in(int nC, const int* __restrict__ ipos, const double* __r
 template <typename TF>
 __global__ void k_ilu_out(int nC, const int* __restrict__ ipos, const TF* __restrict__ zv,
                           double* __restrict__ z) {
+  pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nC) return;
   const TF* src = zv + 8 * (size_t)ipos[i];
@@ -834,6 +842,7 @@ __global__ void __launch_bounds__(kRedThreads) k_ilu_out_sq(int nC, const int* _
                                                             const TF* __restrict__ zv,
                                                             double* __restrict__ z,
                                                             double* __restrict__ part) {
+  pdl_entry();
   TF acc_t = TF(0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nC; i += gridDim.x * blockDim.x) {
     const TF* src = zv + 8 * (size_t)ipos[i];
@@ -903,6 +912,7 @@ __global__ void __launch_bounds__(kT) k_ilu_fwd(int n, const int* __restrict__ r
                                                 const int* __restrict__ pdu,
                                                 const TF* __restrict__ LU, TF* __restrict__ yv,
                                                 TF* __restrict__ zv) {
+  pdl_entry();
   const int lane = threadIdx.x & 31;
   const int sub = lane / 5, a = lane - 5 * sub;
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) / 32 * 6 + sub;
@@ -937,6 +947,7 @@ __global__ void __launch_bounds__(kT) k_ilu_bwd(int n, const int* __restrict__ r
                                                 const int* __restrict__ pdu,
                                                 const TF* __restrict__ LU,
                                                 const TF* __restrict__ yv, TF* __restrict__ zv) {
+  pdl_entry();
   const int lane = threadIdx.x & 31;
   const int sub = lane / 5, a = lane - 5 * sub;
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) / 32 * 6 + sub;
@@ -1025,6 +1036,7 @@ __global__ void __launch_bounds__(32) k_sweep(int n, int p0, const int* __restri
                                               const int* __restrict__ start, int diag0,
                                               const float* __restrict__ LU, float* yv, float* zv,
                                               int stage_blocks) {
+  pdl_entry();
   constexpr int kNB = kNW == 4 ? 4 : 6;        // neighbours of a row (lists are kNW wide)
   constexpr int kAl = 4;                // floats of 16 bytes
   extern __shared__ __align__(16) unsigned char sw_smem[];
@@ -1566,10 +1578,9 @@ static void sweep_level(fos_ctx* c, int mode, int l, const float* LU, float* yv,
   const size_t smem = sweep_smem(mode, blocks);
   const int per_sm = std::max(1, std::min(24, (int)(kSmemSm / (smem + 1024))));
   const int grid = std::min((n + kSwTile - 1) / kSwTile, c->sm_count * per_sm);
-  c->n_launch++;
-  sweep_kernel(c->ilu_nbw, mode)<<<grid, 32, smem, c->stream>>>(
-      n, lev[l], mode == kSwBwd ? c->d_pnbU : c->d_pnbL, mode == kSwBwd ? c->d_pdu : c->d_plst,
-      c->sw_top0, LU, yv, zv, blocks);
+  fos_launch_smem(c, sweep_kernel(c->ilu_nbw, mode), grid, 32, smem, n, lev[l],
+                  mode == kSwBwd ? c->d_pnbU : c->d_pnbL, mode == kSwBwd ? c->d_pdu : c->d_plst,
+                  c->sw_top0, LU, yv, zv, blocks);
 }
 
 template <typename TF>

@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(kThreads) k_prim64(int nC, const double* __res
                                                      const double* __restrict__ v,
                                                      const double* __restrict__ d_s, double gm1,
                                                      double* __restrict__ W) {
+  pdl_entry();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nC) return;
   double U[5];
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(kThreads) k_face64(
     const double* __restrict__ W, const double* __restrict__ y, const double* __restrict__ v,
     const double* __restrict__ d_s, const int* __restrict__ bcT, const double* __restrict__ bcP,
     int maxP, double g, double r, double* __restrict__ F) {
+  pdl_entry();
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nF) return;
   const int2 lr = __ldg(faceLR + f);
@@ -218,6 +220,7 @@ __global__ void __launch_bounds__(kThreads) k_gather(
     const double* __restrict__ invV, const double* __restrict__ vv,
     const double* __restrict__ fy, const double* __restrict__ d_s, double a,
     double* __restrict__ out, int* __restrict__ flag) {
+  pdl_entry();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nC) return;
   int e[kW];
@@ -268,6 +271,7 @@ __global__ void __launch_bounds__(kThreads) k_prim_hl(int nC, const double* __re
                                                       const double* __restrict__ v,
                                                       const double* __restrict__ d_s, double gm1,
                                                       float* __restrict__ W) {
+  pdl_entry();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nC) return;
   double U[5];
@@ -367,6 +371,7 @@ __global__ void __launch_bounds__(kThreads) k_bface32(
     const double* __restrict__ y, const double* __restrict__ v, const double* __restrict__ d_s,
     const int* __restrict__ bcT, const double* __restrict__ bcP, int maxP, double g, double r,
     double* __restrict__ F, int all64) {
+  pdl_entry();
   const int f = nFi + blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nF) return;
   const int2 lr = __ldg(faceLR + f);
@@ -433,6 +438,7 @@ __global__ void __launch_bounds__(kThreads) k_cell32(
     double a, double* __restrict__ out, int* __restrict__ flag,
     const double2* __restrict__ faceNA64, unsigned char* __restrict__ fsel, float theta,
     double gm1d) {
+  pdl_entry();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nC) return;
   int e[kW], nbr[kW];
@@ -548,6 +554,7 @@ cell32_fn cell32_kernel(int ell_w, bool hyb, int ek, bool sc) {
 
 __global__ void k_permute(int nC, int nplanes, const int* __restrict__ idx,
                           const double* __restrict__ in, double* __restrict__ out) {
+  pdl_entry();
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= (long)nplanes * nC) return;
   const int q = (int)(k / nC), i = (int)(k - (long)q * nC);
@@ -562,6 +569,7 @@ __device__ __forceinline__ double warp_sum(double x) {
 
 __global__ void __launch_bounds__(kRedThreads) k_sumsq_part(const double* __restrict__ x, long n,
                                                             double* __restrict__ part) {
+  pdl_entry();
   double s = 0.0;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const double t = x[i];
@@ -579,6 +587,7 @@ __global__ void __launch_bounds__(kRedThreads) k_sumsq_part(const double* __rest
 }
 
 __global__ void k_sum_final(const double* __restrict__ part, int np, double* __restrict__ out) {
+  pdl_entry();
   double s = 0.0;
   for (int i = threadIdx.x; i < np; i += blockDim.x) s += part[i];
   __shared__ double sh[32];
@@ -594,6 +603,7 @@ __global__ void k_sum_final(const double* __restrict__ part, int np, double* __r
 
 // s, 1/s and b/s of the Jv (scal[1..3]; the epilogue reads them as d_s[0..2])
 __global__ void k_sigma(double* scal, double ynorm, double eps, double b) {
+  pdl_entry();
   const double vn2 = scal[0];
   const double s = vn2 > 0.0 ? eps * (1.0 + ynorm) / sqrt(vn2) : 0.0;
   scal[1] = s;
@@ -603,6 +613,7 @@ __global__ void k_sigma(double* scal, double ynorm, double eps, double b) {
 
 // the same with ||v||_2 supplied by the caller (no reduction pass over v)
 __global__ void k_sigma_known(double* scal, double ynorm, double vnorm, double eps, double b) {
+  pdl_entry();
   const double s = vnorm > 0.0 ? eps * (1.0 + ynorm) / vnorm : 0.0;
   scal[0] = vnorm * vnorm;
   scal[1] = s;
