@@ -51,25 +51,61 @@ __device__ __forceinline__ double warp_sum(double x) {
   return x;
 }
 
-// block-reduce nv accumulators into part[l * gridDim.x + blockIdx.x]
-template <int NV>
-__device__ __forceinline__ void block_reduce_store(double (&acc)[NV], int nv, double* part) {
-  __shared__ double sh[kT / 32][kMaxVec];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// Sums of eight accumulators over a warp by halving what each lane holds: 9 FP64 additions per
+// lane where eight butterflies take 40 (an FP64 instruction holds its quarter of an SM for 64
+// clocks, so on small grids the trees were most of a dot product).  Lane l then has sum l / 4.
+__device__ __forceinline__ double warp_sum8(const double (&v)[8], int lane) {
+  double a[4], b[2], c;
 #pragma unroll
-  for (int l = 0; l < NV; l++) {
-    if (l < nv) {
-      double s = warp_sum(acc[l]);
-      if (lane == 0) sh[wid][l] = s;
+  for (int j = 0; j < 4; j++) {
+    const double keep = (lane & 16) ? v[j + 4] : v[j], send = (lane & 16) ? v[j] : v[j + 4];
+    a[j] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const double keep = (lane & 8) ? a[j + 2] : a[j], send = (lane & 8) ? a[j] : a[j + 2];
+    b[j] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  {
+    const double keep = (lane & 4) ? b[1] : b[0], send = (lane & 4) ? b[0] : b[1];
+    c = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  }
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  return c + __shfl_xor_sync(0xffffffffu, c, 1);
+}
+
+// block-reduce NV accumulators into part[l * gridDim.x + blockIdx.x] (any block size up to kT)
+template <int NV>
+__device__ __forceinline__ void block_reduce_store(double (&acc)[NV], double* part) {
+  __shared__ double sh[kT / 32][kMaxVec + 8];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int l0 = 0; l0 < NV; l0 += 8) {
+    if constexpr (NV >= 3) {
+      double v[8];
+#pragma unroll
+      for (int l = 0; l < 8; l++) v[l] = l0 + l < NV ? acc[l0 + l < NV ? l0 + l : 0] : 0.0;
+      const double s = warp_sum8(v, lane);
+      if ((lane & 3) == 0) sh[wid][l0 + (lane >> 2)] = s;
+    } else {
+#pragma unroll
+      for (int l = 0; l < NV; l++) {
+        const double s = warp_sum(acc[l]);
+        if (lane == 0) sh[wid][l] = s;
+      }
     }
   }
   __syncthreads();
-  for (int l = threadIdx.x; l < nv; l += blockDim.x) {
+  for (int l = threadIdx.x; l < NV; l += blockDim.x) {
     double s = 0.0;
-    for (int w = 0; w < kT / 32; w++) s += sh[w][l];
+    for (int w = 0; w < nw; w++) s += sh[w][l];
     part[(size_t)l * gridDim.x + blockIdx.x] = s;
   }
 }
+
+struct Coef {  // coefficients passed with the launch
+  double c[kMaxVec];
+};
 
 // h[l] = V_l . w for l < NV (NV fixed at compile time: accumulators stay in registers),
 // plus h[NV] = ||w||^2 when NRM
@@ -88,23 +124,22 @@ __global__ void __launch_bounds__(kT) k_mdot(long n, const double* __restrict__ 
     for (int l = 0; l < NV; l++) acc[l] += V[(size_t)l * ldv + i] * wi;
     if (NRM) acc[NA - 1] += wi * wi;
   }
-  block_reduce_store<NA>(acc, NA, part);
+  block_reduce_store<NA>(acc, part);
 }
 
 // w -= sum_l h[l] s2[l] V_l ; then part <- V_l . w (MODE 0, CGS2 second pass), ||w||^2
 // (MODE 1), or both (MODE 2: the DGKS test and, when it fails, the second pass's
-// coefficients come out of the same sweep over V).  s2 (null: all 1) are the squared
-// scales of unnormalised basis vectors (v_l = s_l V_l), so h = V^T w gives the coefficients
+// coefficients come out of the same sweep over V).  s2 are the squared scales of
+// unnormalised basis vectors (v_l = s_l V_l), so h = V^T w gives the coefficients
 // of the projection onto the v_l.
 template <int NV, int MODE>
 __global__ void __launch_bounds__(kT) k_update(long n, const double* __restrict__ V, long ldv,
-                                               const double* __restrict__ h,
-                                               const double* __restrict__ s2,
+                                               const double* __restrict__ h, const Coef s2,
                                                double* __restrict__ w,
                                                double* __restrict__ part) {
   pdl_entry();
   __shared__ double hs[NV];
-  if (threadIdx.x < NV) hs[threadIdx.x] = s2 ? h[threadIdx.x] * s2[threadIdx.x] : h[threadIdx.x];
+  if (threadIdx.x < NV) hs[threadIdx.x] = h[threadIdx.x] * s2.c[threadIdx.x];
   __syncthreads();
   constexpr int NA = MODE == 0 ? NV : MODE == 1 ? 1 : NV + 1;
   double acc[NA];
@@ -125,24 +160,28 @@ __global__ void __launch_bounds__(kT) k_update(long n, const double* __restrict_
     }
     if (MODE != 0) acc[NA - 1] += wi * wi;
   }
-  block_reduce_store<NA>(acc, NA, part);
+  block_reduce_store<NA>(acc, part);
 }
 
-// out[l] = sum of part[l * np ...]
-__global__ void k_final(int nv, int np, const double* __restrict__ part, double* __restrict__ out) {
+// out[l] = sum of part[l * np ...], also into host[l] (page-locked, when given: the copy that
+// would follow is saved); with flag, host[nv] = 1 where *flag is set
+__global__ void k_final(int nv, int np, const double* __restrict__ part, double* __restrict__ out,
+                        double* host, const int* flag) {
   pdl_entry();
   const int l = blockIdx.x;
   if (l >= nv) return;
   double s = 0.0;
   for (int i = threadIdx.x; i < np; i += blockDim.x) s += part[(size_t)l * np + i];
-  __shared__ double sh[32];
+  __shared__ double sh[8];
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    double t = threadIdx.x < (int)(blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
-    t = warp_sum(t);
-    if (threadIdx.x == 0) out[l] = t;
+  if (threadIdx.x == 0) {
+    double t = sh[0];
+    for (int w = 1; w < (int)(blockDim.x >> 5); w++) t += sh[w];
+    out[l] = t;
+    if (host) host[l] = t;
+    if (flag && l == 0) host[nv] = *flag ? 1.0 : 0.0;
   }
 }
 
@@ -162,12 +201,8 @@ __global__ void k_axpy(long n, double a, const double* __restrict__ x, double* _
 // the vector loop is not unrolled, so no FP64 instruction is issued predicated off.
 template <bool kAcc, bool kAdd>
 __global__ void k_comb(long n, int nv, const double* __restrict__ Z, long ldz,
-                       const double* __restrict__ cc, double* __restrict__ x,
-                       double* __restrict__ yadd) {
+                       const Coef cs, double* __restrict__ x, double* __restrict__ yadd) {
   pdl_entry();
-  __shared__ double cs[kMaxVec];
-  if (threadIdx.x < kMaxVec) cs[threadIdx.x] = threadIdx.x < nv ? cc[threadIdx.x] : 0.0;
-  __syncthreads();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double s = 0.0;
@@ -175,11 +210,11 @@ __global__ void k_comb(long n, int nv, const double* __restrict__ Z, long ldz,
   if constexpr (kAcc) {
     s = x[i];
   } else if (nv > 0) {
-    s = cs[0] * Z[i];
+    s = cs.c[0] * Z[i];
     l0 = 1;
   }
 #pragma unroll 1
-  for (int l = l0; l < nv; l++) s = fma(cs[l], Z[(size_t)l * ldz + i], s);
+  for (int l = l0; l < nv; l++) s = fma(cs.c[l], Z[(size_t)l * ldz + i], s);
   if constexpr (kAdd) yadd[i] += s;
   else x[i] = s;
 }
@@ -223,7 +258,7 @@ __global__ void __launch_bounds__(kT) k_newton_res(long n, const double* __restr
     acc[0] = fma(B, B, acc[0]);
     acc[1] = fma(yi, yi, acc[1]);
   }
-  block_reduce_store<2>(acc, 2, part);
+  block_reduce_store<2>(acc, part);
 }
 
 // out = sum_l c[l] p[l] (up to 8 vectors, summed in order l = 0, 1, ...)
@@ -250,7 +285,7 @@ __global__ void __launch_bounds__(kT) k_wrms_part(long n, const double* __restri
     const double e = a[i] / (rtol * fabs(w[i]) + atol);
     acc[0] += e * e;
   }
-  block_reduce_store<1>(acc, 1, part);
+  block_reduce_store<1>(acc, part);
 }
 
 inline int nb(long n) { return (int)((n + kT - 1) / kT); }
@@ -367,8 +402,20 @@ struct Driver {
     ilu_ref_rate = (its > 0 && bnorm > 0.0 && res > 0.0) ? std::pow(res / bnorm, 1.0 / its) : 0.0;
   }
 
-  int reduce(int nv, double* out) {  // k_final over wk.part into device out
-    fos_launch(c, k_final, nv, 256, nv, kRedBlocks, wk.part, out);
+  // Blocks and threads of the kernels that sum over all unknowns: 128 threads a block, one block
+  // an SM, up to 16 unknowns a thread; beyond that kRedBlocks blocks of kT.  With the large
+  // shape everywhere a thread of a small grid summed one element and the block's trees were the
+  // rest (184,320 unknowns, 15 vectors: 34 us a multi-dot, 13 us this way).
+  int rblocks = kRedBlocks, rthreads = kT;
+  void set_shape() {
+    const long few = 152L * 128 * 16;
+    if (wk.N > few) return;
+    rthreads = 128;
+    rblocks = (int)std::max<long>(1, std::min<long>(152, (wk.N + 127) / 128));
+  }
+  // k_final over wk.part into device out, and into host (page-locked) when given
+  int reduce(int nv, double* out, double* host = nullptr, const int* flag = nullptr) {
+    fos_launch(c, k_final, nv, 128, nv, rblocks, wk.part, out, host, flag);
     FOS_LAUNCH_CHECK();
     return 0;
   }
@@ -376,7 +423,7 @@ struct Driver {
   int mdot(int nv, const double* V, long ldv, const double* w) {
     switch (nv) {
 #define FOS_MDOT(K) \
-  case K: fos_launch(c, k_mdot<K, NRM>, kRedBlocks, kT, wk.N, V, ldv, w, wk.part); break;
+  case K: fos_launch(c, k_mdot<K, NRM>, rblocks, rthreads, wk.N, V, ldv, w, wk.part); break;
       FOS_MDOT(1) FOS_MDOT(2) FOS_MDOT(3) FOS_MDOT(4) FOS_MDOT(5) FOS_MDOT(6) FOS_MDOT(7)
       FOS_MDOT(8) FOS_MDOT(9) FOS_MDOT(10) FOS_MDOT(11) FOS_MDOT(12) FOS_MDOT(13) FOS_MDOT(14)
       FOS_MDOT(15) FOS_MDOT(16) FOS_MDOT(17) FOS_MDOT(18) FOS_MDOT(19) FOS_MDOT(20) FOS_MDOT(21)
@@ -389,11 +436,10 @@ struct Driver {
     return 0;
   }
   template <int MODE>
-  int update(int nv, const double* V, long ldv, const double* h, double* w,
-             const double* s2 = nullptr) {
+  int update(int nv, const double* V, long ldv, const double* h, double* w, const Coef& s2) {
     switch (nv) {
 #define FOS_UPD(K) \
-  case K: fos_launch(c, k_update<K, MODE>, kRedBlocks, kT, wk.N, V, ldv, h, s2, w, wk.part); break;
+  case K: fos_launch(c, k_update<K, MODE>, rblocks, rthreads, wk.N, V, ldv, h, s2, w, wk.part); break;
       FOS_UPD(1) FOS_UPD(2) FOS_UPD(3) FOS_UPD(4) FOS_UPD(5) FOS_UPD(6) FOS_UPD(7) FOS_UPD(8)
       FOS_UPD(9) FOS_UPD(10) FOS_UPD(11) FOS_UPD(12) FOS_UPD(13) FOS_UPD(14) FOS_UPD(15)
       FOS_UPD(16) FOS_UPD(17) FOS_UPD(18) FOS_UPD(19) FOS_UPD(20) FOS_UPD(21) FOS_UPD(22)
@@ -410,6 +456,7 @@ struct Driver {
     FOS_CUDA(cudaStreamSynchronize(c->stream));
     return 0;
   }
+  int sq_np = 0;  // partial sums of ||z||^2 that the last psolve left (0: the sum is formed)
   double gamma_cur = 0.0;  // gamma of the current linear solve (input of the learned preconditioner)
   // z = M^-1 r; with d_zsq (plain ILU(0) only, else ignored) also ||z||^2 into d_zsq from
   // the apply's own pass over z -- the norm the next Jv of z needs.  Returns in *have_sq
@@ -429,7 +476,7 @@ struct Driver {
       return fos_gnn_precond(c, y, wk.u, gamma_cur, z);
     }
     if (have_sq) *have_sq = d_zsq != nullptr;
-    return fos_ilu_apply(c, r, z, d_zsq);
+    return fos_ilu_apply(c, r, z, d_zsq, &sq_np);
   }
   // Expected cost of a fixed residual reduction: iteration time / -log(rate per iteration).
   // The network is not applied while its last solve's rate at its iteration time buys that
@@ -468,15 +515,13 @@ struct Driver {
     setup_made = true;
     return c->ilu_ierr ? 3 : 0;
   }
-  // w = J_G v at state y with f(y) = fy
-  // w = J_G v by the finite difference; have_sq: ||v||^2 is already in c->d_scal[0]
+  // w = J_G v at state y, f(y) = fy, by the finite difference; have_sq: the last psolve left ||v||^2
   int jv(const double* y, const double* fy, const double* v, double* w, double gamma,
          double ynorm, bool have_sq = false) {
     st.n_jv++;
     st.n_rhs++;
-    int rc = have_sq ? 0 : fos_norm2_dev(c, v, wk.N, c->d_scal);
-    if (rc) return rc;
-    rc = fos_jv_sigma(c, c->d_scal, ynorm, eps, -gamma);
+    int rc = have_sq ? fos_jv_sigma(c, c->d_scal, sq_np, ynorm, eps, -gamma)
+                     : fos_norm2_sigma(c, v, wk.N, c->d_scal, ynorm, eps, -gamma);
     if (rc) return rc;
     return fos_residual_launch(c, y, v, c->d_scal + 1, fy, w, 1.0, -gamma, 1);
   }
@@ -496,13 +541,13 @@ struct Driver {
       int rc = fos_residual_launch(c, y, nullptr, nullptr, nullptr, wk.f, 0.0, 0.0, 0);
       if (rc) return rc;
       st.n_rhs++;
-      fos_launch(c, k_newton_res, kRedBlocks, kT, N, (const double*)y, (const double*)wk.f,
+      fos_launch(c, k_newton_res, rblocks, rthreads, N, (const double*)y, (const double*)wk.f,
                  hist, gamma, wk.b, wk.V, wk.part);
-      if ((rc = reduce(2, wk.sc))) return rc;
-      FOS_CUDA(cudaMemcpyAsync(hb, wk.sc, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-      FOS_CUDA(cudaMemcpyAsync(c->h_scal, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+      if ((rc = reduce(2, wk.sc, c->h_scal, c->d_flag))) return rc;
       FOS_CUDA(cudaStreamSynchronize(c->stream));
-      if (*(int*)c->h_scal) return 2;  // non-finite residual
+      hb[0] = c->h_scal[0];
+      hb[1] = c->h_scal[1];
+      if (c->h_scal[2] != 0.0) return 2;  // non-finite residual
       // the first pass also gives ||y_0||
       if (k == 0) gtol = o.newton_rtol * std::sqrt(hb[1]) + o.newton_atol * std::sqrt((double)N);
       const double gn = std::sqrt(hb[0]);
@@ -581,7 +626,12 @@ struct Driver {
     // only on the steps that cancel more (the plain 1/sqrt(2) threshold reran it on almost
     // every step of a well-preconditioned solve, where J M^-1 v is close to v).
     const double reorth_frac = std::min(0.5, o.lin_rtol * o.lin_rtol);
-    double* d_sig2 = wk.sc + 5 * kMaxVec;
+    double* hh = c->h_scal;  // the sums of a step: V^T w and ||w||^2, at kMaxVec the second pass's
+    auto scales = [&](int nv) {
+      Coef s2{};
+      std::copy(sig2.begin(), sig2.begin() + nv, s2.c);
+      return s2;
+    };
     if (added) *added = false;
     bool d_written = false;  // wk.d holds the correction of the cycles so far
     *its = 0;
@@ -600,8 +650,6 @@ struct Driver {
         fos_launch(c, k_scale, nb(N), kT, N, rvec, 1.0 / beta, wk.V);
         sig[0] = sig2[0] = 1.0;
       }
-      FOS_CUDA(cudaMemcpyAsync(d_sig2, sig2.data(), sizeof(double), cudaMemcpyHostToDevice,
-                               c->stream));
       bool fallback = false;
       std::fill(g.begin(), g.end(), 0.0);
       g[0] = beta;
@@ -625,17 +673,18 @@ struct Driver {
         // V^T w' (MODE 2) so the second pass needs no separate sweep over V for its
         // coefficients; otherwise it returns ||w'||^2 only (MODE 1).
         const bool fused = last_reorth;
+        const Coef s2 = scales(nv);
         if ((rc = mdot<true>(nv, wk.V, N, wj))) return rc;              // V^T w, ||w||^2
-        if ((rc = reduce(nv + 1, wk.sc))) return rc;
+        if ((rc = reduce(nv + 1, wk.sc, hh))) return rc;
         if (fused) {
-          if ((rc = update<2>(nv, wk.V, N, wk.sc, wj, d_sig2))) return rc;  // w -= V s2 h; V^T w, ||w||^2
-          if ((rc = reduce(nv + 1, wk.sc + kMaxVec))) return rc;
-          if ((rc = fetch(wk.sc, hbuf.data(), 2 * kMaxVec))) return rc;
+          if ((rc = update<2>(nv, wk.V, N, wk.sc, wj, s2))) return rc;  // w -= V s2 h; V^T w, ||w||^2
+          if ((rc = reduce(nv + 1, wk.sc + kMaxVec, hh + kMaxVec))) return rc;
         } else {
-          if ((rc = update<1>(nv, wk.V, N, wk.sc, wj, d_sig2))) return rc;  // w -= V s2 h, ||w||^2
-          if ((rc = reduce(1, wk.sc + kMaxVec + nv))) return rc;
-          if ((rc = fetch(wk.sc, hbuf.data(), kMaxVec + nv + 1))) return rc;
+          if ((rc = update<1>(nv, wk.V, N, wk.sc, wj, s2))) return rc;  // w -= V s2 h, ||w||^2
+          if ((rc = reduce(1, wk.sc + kMaxVec + nv, hh + kMaxVec + nv))) return rc;
         }
+        FOS_CUDA(cudaStreamSynchronize(c->stream));
+        std::copy(hh, hh + kMaxVec + nv + 1, hbuf.begin());
         double* col = &H[(size_t)(m + 1) * j];
         for (int l = 0; l < nv; l++) col[l] = sig[j] * sig[l] * hbuf[l];
         double hn2 = hbuf[kMaxVec + nv];
@@ -644,17 +693,18 @@ struct Driver {
           const double* h2 = wk.sc + kMaxVec;  // V^T w' (device), from MODE 2 or a sweep
           if (!fused) {
             if ((rc = mdot<false>(nv, wk.V, N, wj))) return rc;
-            if ((rc = reduce(nv, wk.sc + kMaxVec))) return rc;
+            if ((rc = reduce(nv, wk.sc + kMaxVec, hh + kMaxVec))) return rc;
           }
-          if ((rc = update<1>(nv, wk.V, N, h2, wj, d_sig2))) return rc;
-          if ((rc = reduce(1, wk.sc + 3 * kMaxVec))) return rc;
-          if ((rc = fetch(wk.sc + kMaxVec, hbuf.data() + kMaxVec, 2 * kMaxVec + 1))) return rc;
+          if ((rc = update<1>(nv, wk.V, N, h2, wj, s2))) return rc;
+          if ((rc = reduce(1, wk.sc + 3 * kMaxVec, hh + 3 * kMaxVec))) return rc;
+          FOS_CUDA(cudaStreamSynchronize(c->stream));
+          std::copy(hh + kMaxVec, hh + 3 * kMaxVec + 1, hbuf.begin() + kMaxVec);
           for (int l = 0; l < nv; l++) col[l] += sig[j] * sig[l] * hbuf[kMaxVec + l];
           hn2 = hbuf[3 * kMaxVec];
           reorth++;
           st.n_reorth++;
         }
-        // the fetch synchronised the stream: the host clock has the iteration's whole cost
+        // the stream is synchronised: the host clock has the iteration's whole cost
         note_iteration_time(std::chrono::duration<double, std::milli>(
                                 std::chrono::steady_clock::now() - t_it).count());
         const double wn = std::sqrt(hn2);  // ||W_{j+1}||
@@ -663,8 +713,6 @@ struct Driver {
         if (wn > 0.0) {
           sig[j + 1] = 1.0 / wn;
           sig2[j + 1] = sig[j + 1] * sig[j + 1];
-          FOS_CUDA(cudaMemcpyAsync(d_sig2 + j + 1, sig2.data() + j + 1, sizeof(double),
-                                   cudaMemcpyHostToDevice, c->stream));
         }
         for (int l = 0; l < j; l++) {
           const double t0 = cs[l] * col[l] + sn[l] * col[l + 1];
@@ -706,11 +754,10 @@ struct Driver {
         yv[l] = s / H[l + (size_t)(m + 1) * l];
       }
       for (int l = 0; l < kend; l++) yv[l] *= sig[l];  // z_l = sig[l] z'_l
-      FOS_CUDA(cudaMemcpyAsync(wk.sc + 4 * kMaxVec, yv.data(), sizeof(double) * kend,
-                               cudaMemcpyHostToDevice, c->stream));
+      Coef cz{};
+      std::copy(yv.begin(), yv.begin() + kend, cz.c);
       double* yadd = (conv && !d_written && y_add) ? y_add : nullptr;
       {
-        const double* cz = wk.sc + 4 * kMaxVec;
         const double* Zc = wk.Z;
         if (yadd)  // (only while d holds nothing yet)
           fos_launch(c, k_comb<false, true>, nb(N), kT, N, kend, Zc, N, cz, wk.d, yadd);
@@ -777,6 +824,7 @@ extern "C" int fos_bdf_run(fos_ctx* c, double t0, double* y, const fos_bdf_opts*
   const bool resume = opts->resume && wk.has_hist;
   const double eps = opts->jv_eps > 0.0 ? opts->jv_eps : jv_eps_default(c);
   Driver dr{c, wk, *opts, st, eps};
+  dr.set_shape();
   dr.ilu_ref_its = wk.ilu_ref_its;
   dr.ilu_ref_rate = wk.ilu_ref_rate;
   double t = t0;
@@ -939,11 +987,10 @@ struct Adapt {
   }
   // ||a||_WRMS with weights from w
   int wrms(const double* a, const double* w, double rtol, double atol, double* out) {
-    fos_launch(c, k_wrms_part, kRedBlocks, kT, N, a, w, rtol, atol, wk.part);
-    if (int rc = dr.reduce(1, wk.sc + 5 * kMaxVec)) return rc;
-    double h = 0.0;
-    if (int rc = dr.fetch(wk.sc + 5 * kMaxVec, &h, 1)) return rc;
-    *out = std::sqrt(h / (double)N);
+    fos_launch(c, k_wrms_part, dr.rblocks, dr.rthreads, N, a, w, rtol, atol, wk.part);
+    if (int rc = dr.reduce(1, wk.sc + 5 * kMaxVec, c->h_scal)) return rc;
+    FOS_CUDA(cudaStreamSynchronize(c->stream));
+    *out = std::sqrt(c->h_scal[0] / (double)N);
     return 0;
   }
 };
@@ -993,6 +1040,7 @@ extern "C" int fos_bdf_adaptive(fos_ctx* c, double t0, double tout, double* y,
   const long max_steps = ad->max_steps > 0 ? ad->max_steps : 100000;
   const double eps = nk->jv_eps > 0.0 ? nk->jv_eps : jv_eps_default(c);
   Driver dr{c, wk, *nk, st, eps};
+  dr.set_shape();
   dr.ilu_ref_its = wk.ilu_ref_its;
   dr.ilu_ref_rate = wk.ilu_ref_rate;
   Adapt A{c, wk, dr, N};
@@ -1173,6 +1221,7 @@ extern "C" int fos_linear_solve_dev(fos_ctx* c, double t, const double* y, const
   const long N = wk.N;
   const double eps = opts->jv_eps > 0.0 ? opts->jv_eps : jv_eps_default(c);
   Driver dr{c, wk, *opts, st, eps};
+  dr.set_shape();
   dr.ilu_ref_its = wk.ilu_ref_its;
   dr.ilu_ref_rate = wk.ilu_ref_rate;
   dr.t_step = t;

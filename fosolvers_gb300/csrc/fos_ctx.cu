@@ -491,9 +491,7 @@ extern "C" int fos_euler_jv_dev(fos_ctx* c, double t, const double* y, const dou
     return -1;
   }
   // s = eps (1 + ||y||) / ||v|| evaluated on the device (scal[0] = ||v||^2, scal[1] = s)
-  int rc = fos_norm2_dev(c, v, 5L * c->nC, c->d_scal);
-  if (rc) return rc;
-  rc = fos_jv_sigma(c, c->d_scal, ynorm, eps, b);
+  const int rc = fos_norm2_sigma(c, v, 5L * c->nC, c->d_scal, ynorm, eps, b);
   if (rc) return rc;
   return fos_residual_launch(c, y, v, c->d_scal + 1, fy, out, a, b, 1);
 }

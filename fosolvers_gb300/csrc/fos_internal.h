@@ -208,8 +208,12 @@ int fos_permute_plane(fos_ctx* c, const double* in, double* out, int dir, int q)
 // waiting for the last copy (synchronise c->stream before reading h)
 int fos_h2d_internal(fos_ctx* c, const double* h, double* d_internal);
 int fos_d2h_reference(fos_ctx* c, const double* d_internal, double* h);
-// s = eps (1 + ynorm)/||v||, 1/s and b/s into d_scal[1..3] (||v||^2 in d_scal[0])
-int fos_jv_sigma(fos_ctx* c, double* d_scal, double ynorm, double eps, double b);
+// s = eps (1 + ynorm)/||v||, 1/s and b/s into d_scal[1..3]; ||v||^2 is the sum of d_red[0..np)
+// (and goes to d_scal[0]), or is in d_scal[0] (np = 0)
+int fos_jv_sigma(fos_ctx* c, double* d_scal, int np, double ynorm, double eps, double b);
+// the same with ||v||^2 formed from v
+int fos_norm2_sigma(fos_ctx* c, const double* v, long n, double* d_scal, double ynorm, double eps,
+                    double b);
 int fos_jv_sigma_known(fos_ctx* c, double* d_scal, double ynorm, double vnorm, double eps,
                        double b);
 int fos_prim_jac_launch(fos_ctx* c, const double* y, float* W);  // the FP32 Jacobian's primitives
@@ -222,8 +226,10 @@ int fos_jac_assemble(fos_ctx* c, const double* y);
 bool fos_pset_is_fused(const fos_ctx* c);
 int fos_pset_fused(fos_ctx* c, const double* y, double gamma);
 int fos_ilu_factor(fos_ctx* c, double gamma);
-// z = P^-1 r; with d_zsq also ||z||^2 into d_zsq (device), from the same pass over z
-int fos_ilu_apply(fos_ctx* c, const double* r, double* z, double* d_zsq = nullptr);
+// z = P^-1 r; with d_zsq also ||z||^2 from the same pass over z: into d_zsq (device; *np = 0), or
+// left as *np partial sums in d_red
+int fos_ilu_apply(fos_ctx* c, const double* r, double* z, double* d_zsq = nullptr,
+                  int* np = nullptr);
 // fos_ilut.cu: the Euler preconditioner with ILUT (FOS_PREC_ILUT)
 int fos_ilut_ctx_factor(fos_ctx* c, double gamma);
 int fos_ilut_ctx_apply(fos_ctx* c, const double* r, double* z);

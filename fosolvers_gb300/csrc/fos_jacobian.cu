@@ -1584,8 +1584,8 @@ static void sweep_level(fos_ctx* c, int mode, int l, const float* LU, float* yv,
 }
 
 template <typename TF>
-static int ilu_apply_t(fos_ctx* c, const TF* LU, const double* r, double* z,
-                       double* d_zsq = nullptr) {
+static int ilu_apply_t(fos_ctx* c, const TF* LU, const double* r, double* z, double* d_zsq,
+                       int* np) {
   TF* yv = reinterpret_cast<TF*>(c->d_ilu_tmp);
   TF* zv = yv + 8 * (size_t)c->nC;
   fos_launch(c, k_ilu_in<TF>, nb(c->nC, 256), 256, c->nC, (const int*)c->d_ipos, r, yv);
@@ -1619,10 +1619,15 @@ static int ilu_apply_t(fos_ctx* c, const TF* LU, const double* r, double* z,
                (const TF*)yv, zv);
   }
   if (d_zsq) {
-    fos_launch(c, k_ilu_out_sq<TF>, kRedBlocks, kRedThreads, c->nC, (const int*)c->d_ipos,
+    const int blocks = std::min(kRedBlocks, nb(c->nC, kRedThreads));
+    fos_launch(c, k_ilu_out_sq<TF>, blocks, kRedThreads, c->nC, (const int*)c->d_ipos,
                (const TF*)zv, z, c->d_red);
     FOS_LAUNCH_CHECK();
-    return fos_sum_partials(c, kRedBlocks, d_zsq);
+    if (np) {
+      *np = blocks;
+      return 0;
+    }
+    return fos_sum_partials(c, blocks, d_zsq);
   }
   fos_launch(c, k_ilu_out<TF>, nb(c->nC, 256), 256, c->nC, (const int*)c->d_ipos,
              (const TF*)zv, z);
@@ -1630,13 +1635,14 @@ static int ilu_apply_t(fos_ctx* c, const TF* LU, const double* r, double* z,
   return 0;
 }
 
-int fos_ilu_apply(fos_ctx* c, const double* r, double* z, double* d_zsq) {
+int fos_ilu_apply(fos_ctx* c, const double* r, double* z, double* d_zsq, int* np) {
+  if (np) *np = 0;
   if (c->flags & FOS_PREC_ILUT) {
     if (int rc = fos_ilut_ctx_apply(c, r, z)) return rc;
     return d_zsq ? fos_norm2_dev(c, z, 5L * c->nC, d_zsq) : 0;
   }
-  if (c->flags & FOS_ILU_FP32) return ilu_apply_t<float>(c, c->d_LU32, r, z, d_zsq);
-  return ilu_apply_t<double>(c, c->d_LU, r, z, d_zsq);
+  if (c->flags & FOS_ILU_FP32) return ilu_apply_t<float>(c, c->d_LU32, r, z, d_zsq, np);
+  return ilu_apply_t<double>(c, c->d_LU, r, z, d_zsq, np);
 }
 
 // Block Jacobian in position space: rowptr (nC+1) / col (positions) / 25-value blocks.

@@ -16,6 +16,7 @@
 // faces into the cell gather (k_cell32: each interior face evaluated by both of its cells,
 // bit-identically); boundary faces go through k_bface32 (ghost state and flow in FP64,
 // stored as the difference from the cell's own flux).  Sums are in FP64 in both variants.
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <string>
@@ -601,10 +602,26 @@ __global__ void k_sum_final(const double* __restrict__ part, int np, double* __r
   }
 }
 
-// s, 1/s and b/s of the Jv (scal[1..3]; the epilogue reads them as d_s[0..2])
-__global__ void k_sigma(double* scal, double ynorm, double eps, double b) {
+// s, 1/s and b/s of the Jv (scal[1..3]; the epilogue reads them as d_s[0..2]) from ||v||^2, the
+// sum of part[0..np), which goes to scal[0] (np = 0: it is there already); one block, its scalar
+// arithmetic by one thread
+__global__ void __launch_bounds__(256) k_sigma(double* scal, const double* __restrict__ part,
+                                               int np, double ynorm, double eps, double b) {
   pdl_entry();
-  const double vn2 = scal[0];
+  __shared__ double sh[8];
+  double vn2 = 0.0;
+  if (np > 0) {
+    double q = 0.0;
+    for (int i = threadIdx.x; i < np; i += blockDim.x) q += part[i];
+    q = warp_sum(q);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = q;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int w = 0; w < (int)(blockDim.x >> 5); w++) vn2 += sh[w];
+  }
+  if (threadIdx.x != 0) return;
+  if (np > 0) scal[0] = vn2;
+  else vn2 = scal[0];
   const double s = vn2 > 0.0 ? eps * (1.0 + ynorm) / sqrt(vn2) : 0.0;
   scal[1] = s;
   scal[2] = s > 0.0 ? 1.0 / s : 0.0;
@@ -674,9 +691,16 @@ int fos_prim_launch(fos_ctx* c, const double* y) {
   return 0;
 }
 
+// blocks of the sum of squares: about eight elements a thread (more, and smaller, sums on a small
+// vector would be trees), kRedBlocks at most
+static int sumsq_blocks(long n) {
+  return (int)std::max<long>(1, std::min<long>(kRedBlocks, n / (8L * kRedThreads)));
+}
+
 int fos_norm2_dev(fos_ctx* c, const double* x, long n, double* d_out_sq) {
-  fos_launch(c, k_sumsq_part, kRedBlocks, kRedThreads, x, n, c->d_red);
-  fos_launch(c, k_sum_final, 1, 1024, c->d_red, kRedBlocks, d_out_sq);
+  const int np = sumsq_blocks(n);
+  fos_launch(c, k_sumsq_part, np, kRedThreads, x, n, c->d_red);
+  fos_launch(c, k_sum_final, 1, 1024, c->d_red, np, d_out_sq);
   FOS_LAUNCH_CHECK();
   return 0;
 }
@@ -687,10 +711,17 @@ int fos_sum_partials(fos_ctx* c, int np, double* d_out) {
   return 0;
 }
 
-int fos_jv_sigma(fos_ctx* c, double* d_scal, double ynorm, double eps, double b) {
-  fos_launch(c, k_sigma, 1, 1, d_scal, ynorm, eps, b);
+int fos_jv_sigma(fos_ctx* c, double* d_scal, int np, double ynorm, double eps, double b) {
+  fos_launch(c, k_sigma, 1, np > 0 ? 256 : 32, d_scal, (const double*)c->d_red, np, ynorm, eps, b);
   FOS_LAUNCH_CHECK();
   return 0;
+}
+
+int fos_norm2_sigma(fos_ctx* c, const double* x, long n, double* d_scal, double ynorm, double eps,
+                    double b) {
+  const int np = sumsq_blocks(n);
+  fos_launch(c, k_sumsq_part, np, kRedThreads, x, n, c->d_red);
+  return fos_jv_sigma(c, d_scal, np, ynorm, eps, b);
 }
 
 int fos_jv_sigma_known(fos_ctx* c, double* d_scal, double ynorm, double vnorm, double eps,
