@@ -447,11 +447,27 @@ __global__ void __launch_bounds__(kThreads) k_cell32(
   load_ell<kW>(cnb, c, nbr);  // the cells across the faces: no wait on the face arrays
   PHL P;
   load_hl(W, c, P);
-  // FP64 accumulation in ELL order; the first face initialises the sums (every cell has
-  // at least one face, and ELL rows are padded at the end).  The terms come negated from
-  // the face arithmetic (FP32 or FP64, where negation is exact), so the sums are plain
-  // additions: acc = n_0 + n_1 + ..., no FP64 negation for the first term
+  // Accumulation in ELL order; the first face initialises the sums (every cell has at least
+  // one face, and ELL rows are padded at the end).  The terms come negated from the face
+  // arithmetic (where negation is exact), so the sums are plain additions.
+  // The FP64 flux terms of kHyb are summed in FP64.  Without it every interior term is an FP32
+  // number, and the sum is carried as an FP32 pair (error-free TwoSum, its errors summed: about
+  // 48 bits, what the primitives carry) and widened once: 5 FP64 additions a cell instead of 15
+  // (30 for a hexahedron with its closure term), and half the widenings, on a kernel whose FP64
+  // pipe was the bound (a Jv's 25 FP64 instructions took 79 of 109 us at 64^3 x 6: now 15).
+  // The error against 64-bit values is that of the FP32 terms, the same as with FP64 sums.
   double acc[5];
+  float as[5], ae[5];
+  auto add = [&](int q, bool first, float t) {
+    if (first) {
+      as[q] = t;
+      ae[q] = 0.0f;
+    } else {
+      const df2 r = df_two_sum(as[q], t);
+      as[q] = r.h;
+      ae[q] += r.l;
+    }
+  };
 #pragma unroll
   for (int k = 0; k < kW; k++) {
     if (k > 0 && e[k] < 0) continue;
@@ -507,16 +523,30 @@ __global__ void __launch_bounds__(kThreads) k_cell32(
                             -sw * (Q.s - P.s), P.s + Q.s, P.s * Q.s, na.x, na.y, na.z, na.w,
                             gm1, dF, dw);
 #pragma unroll
-        for (int q = 0; q < 5; q++) t[q] = f2d_bits(fmaf(-sw, dw[q], -dF[q]));
+        for (int q = 0; q < 5; q++) {
+          const float tq = fmaf(-sw, dw[q], -dF[q]);
+          if constexpr (kHyb) t[q] = f2d_bits(tq);
+          else add(q, k == 0, tq);
+        }
       }
     } else {  // boundary face (cell is L): the FP64 difference of k_bface32, negated
       const double2* F2 = reinterpret_cast<const double2*>(Fb + 6 * (size_t)f);
       const double2 a0 = __ldg(F2), a1 = __ldg(F2 + 1), a2 = __ldg(F2 + 2);
       t[0] = neg_bits(a0.x); t[1] = neg_bits(a0.y); t[2] = neg_bits(a1.x);
       t[3] = neg_bits(a1.y); t[4] = neg_bits(a2.x);
-    }
+      if constexpr (!kHyb) {
 #pragma unroll
-    for (int q = 0; q < 5; q++) acc[q] = k == 0 ? t[q] : acc[q] + t[q];
+        for (int q = 0; q < 5; q++) {
+          const df2 d = df_from_double(t[q]);
+          add(q, k == 0, d.h);
+          ae[q] += d.l;
+        }
+      }
+    }
+    if constexpr (kHyb) {
+#pragma unroll
+      for (int q = 0; q < 5; q++) acc[q] = k == 0 ? t[q] : acc[q] + t[q];
+    }
   }
   // own flux through the closure vector (kSc: the grid has cells whose faces do not close):
   // rho u.S, rho u u.S + p S, rho H u.S.  A compile-time switch: as a run-time branch the
@@ -524,11 +554,17 @@ __global__ void __launch_bounds__(kThreads) k_cell32(
   if constexpr (kSc) {
     const float4 S = __ldg(Sc + c);
     const float t = P.h[0] * (P.h[1] * S.x + P.h[2] * S.y + P.h[3] * S.z);
-    acc[0] -= f2d_bits(t);
-    acc[1] -= f2d_bits(fmaf(t, P.h[1], P.h[5] * S.x));
-    acc[2] -= f2d_bits(fmaf(t, P.h[2], P.h[5] * S.y));
-    acc[3] -= f2d_bits(fmaf(t, P.h[3], P.h[5] * S.z));
-    acc[4] -= f2d_bits(t * P.h[4]);
+    const float own[5] = {t, fmaf(t, P.h[1], P.h[5] * S.x), fmaf(t, P.h[2], P.h[5] * S.y),
+                          fmaf(t, P.h[3], P.h[5] * S.z), t * P.h[4]};
+#pragma unroll
+    for (int q = 0; q < 5; q++) {
+      if constexpr (kHyb) acc[q] -= f2d_bits(own[q]);
+      else add(q, false, -own[q]);
+    }
+  }
+  if constexpr (!kHyb) {
+#pragma unroll
+    for (int q = 0; q < 5; q++) acc[q] = f2d_bits(as[q]) + f2d_bits(ae[q]);
   }
   gather_epilogue<kE>(nC, c, acc, __ldg(invV + c), vv, fy, d_s, a, out, flag);
 }
