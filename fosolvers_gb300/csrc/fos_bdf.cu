@@ -107,24 +107,21 @@ struct Coef {  // coefficients passed with the launch
   double c[kMaxVec];
 };
 
-// h[l] = V_l . w for l < NV (NV fixed at compile time: accumulators stay in registers),
-// plus h[NV] = ||w||^2 when NRM
-template <int NV, bool NRM>
+// h[l] = V_l . w for l < NV (NV fixed at compile time: accumulators stay in registers)
+template <int NV>
 __global__ void __launch_bounds__(kT) k_mdot(long n, const double* __restrict__ V, long ldv,
                                              const double* __restrict__ w,
                                              double* __restrict__ part) {
   pdl_entry();
-  constexpr int NA = NV + (NRM ? 1 : 0);
-  double acc[NA];
+  double acc[NV];
 #pragma unroll
-  for (int l = 0; l < NA; l++) acc[l] = 0.0;
+  for (int l = 0; l < NV; l++) acc[l] = 0.0;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const double wi = w[i];
 #pragma unroll
     for (int l = 0; l < NV; l++) acc[l] += V[(size_t)l * ldv + i] * wi;
-    if (NRM) acc[NA - 1] += wi * wi;
   }
-  block_reduce_store<NA>(acc, part);
+  block_reduce_store<NV>(acc, part);
 }
 
 // w -= sum_l h[l] s2[l] V_l ; then part <- V_l . w (MODE 0, CGS2 second pass), ||w||^2
@@ -419,11 +416,10 @@ struct Driver {
     FOS_LAUNCH_CHECK();
     return 0;
   }
-  template <bool NRM>
   int mdot(int nv, const double* V, long ldv, const double* w) {
     switch (nv) {
 #define FOS_MDOT(K) \
-  case K: fos_launch(c, k_mdot<K, NRM>, rblocks, rthreads, wk.N, V, ldv, w, wk.part); break;
+  case K: fos_launch(c, k_mdot<K>, rblocks, rthreads, wk.N, V, ldv, w, wk.part); break;
       FOS_MDOT(1) FOS_MDOT(2) FOS_MDOT(3) FOS_MDOT(4) FOS_MDOT(5) FOS_MDOT(6) FOS_MDOT(7)
       FOS_MDOT(8) FOS_MDOT(9) FOS_MDOT(10) FOS_MDOT(11) FOS_MDOT(12) FOS_MDOT(13) FOS_MDOT(14)
       FOS_MDOT(15) FOS_MDOT(16) FOS_MDOT(17) FOS_MDOT(18) FOS_MDOT(19) FOS_MDOT(20) FOS_MDOT(21)
@@ -674,8 +670,8 @@ struct Driver {
         // coefficients; otherwise it returns ||w'||^2 only (MODE 1).
         const bool fused = last_reorth;
         const Coef s2 = scales(nv);
-        if ((rc = mdot<true>(nv, wk.V, N, wj))) return rc;              // V^T w, ||w||^2
-        if ((rc = reduce(nv + 1, wk.sc, hh))) return rc;
+        if ((rc = mdot(nv, wk.V, N, wj))) return rc;  // V^T w
+        if ((rc = reduce(nv, wk.sc, hh))) return rc;
         if (fused) {
           if ((rc = update<2>(nv, wk.V, N, wk.sc, wj, s2))) return rc;  // w -= V s2 h; V^T w, ||w||^2
           if ((rc = reduce(nv + 1, wk.sc + kMaxVec, hh + kMaxVec))) return rc;
@@ -688,11 +684,15 @@ struct Driver {
         double* col = &H[(size_t)(m + 1) * j];
         for (int l = 0; l < nv; l++) col[l] = sig[j] * sig[l] * hbuf[l];
         double hn2 = hbuf[kMaxVec + nv];
-        last_reorth = hn2 < reorth_frac * hbuf[nv];
+        // ||w||^2 of the test as ||w'||^2 plus the squares of what was taken out (the v_l are
+        // orthonormal to ~eps / lin_rtol): one FP64 instruction per unknown fewer in the multi-dot
+        double w2 = hn2;
+        for (int l = 0; l < nv; l++) w2 += sig2[l] * hbuf[l] * hbuf[l];
+        last_reorth = hn2 < reorth_frac * w2;
         if (last_reorth) {
           const double* h2 = wk.sc + kMaxVec;  // V^T w' (device), from MODE 2 or a sweep
           if (!fused) {
-            if ((rc = mdot<false>(nv, wk.V, N, wj))) return rc;
+            if ((rc = mdot(nv, wk.V, N, wj))) return rc;
             if ((rc = reduce(nv, wk.sc + kMaxVec, hh + kMaxVec))) return rc;
           }
           if ((rc = update<1>(nv, wk.V, N, h2, wj, s2))) return rc;
