@@ -12,7 +12,7 @@
 //                      ascending face id (fixed, deterministic summation order)
 //   ell    int[4*nC]      the same entries at fixed width (one int4 load per tetrahedron)
 //   W      double[8*nC]   per-cell primitives AoS (rho,u,v,w,H,p,sqrt(rho),0)
-//   Whl    float[16*nC]   FP32 (hi, lo) primitives for the FP32 flux
+//   Whl    float[12*nC]   FP32 (hi, lo) primitives for the FP32 flux
 //   F      double[6*nF]   per-face flows, AoS (5 + pad) so a gather reads 48 B per face
 #include <algorithm>
 #include <cmath>
@@ -345,7 +345,7 @@ extern "C" int fos_ctx_create(fos_ctx** out, int nC, int nE, int nPi, int nPb, c
     FOS_TRY(upload(&c->d_cnb, cnb.data(), cnb.size()));
     FOS_TRY(upload(&c->d_cna32, cna.data(), cna.size()));
   }
-  FOS_TRY(dalloc(&c->d_Whl, 16 * (size_t)nC));
+  FOS_TRY(dalloc(&c->d_Whl, 12 * (size_t)nC));
   if (flags & FOS_FLUX_HYBRID) {
     FOS_TRY(dalloc(&c->d_fsel, (size_t)nP));
     FOS_TRY(cudaMemset(c->d_fsel, 0, (size_t)nP) == cudaSuccess ? 0 : -100);

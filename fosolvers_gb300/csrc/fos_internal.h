@@ -79,7 +79,7 @@ struct fos_ctx {
 
   // ---- device work
   double* d_W = nullptr;      // [8*nC] primitive AoS (rho,u,v,w,H,p,sqrt(rho),0)
-  float* d_Whl = nullptr;     // [16*nC] FP32 (hi, lo) primitives
+  float* d_Whl = nullptr;     // [12*nC] FP32 (hi, lo) primitives
   double* d_F = nullptr;      // [6*nF] face flows, AoS
   double* d_stage = nullptr;  // [5*nC] reference-order staging
   double* d_y = nullptr;      // [5*nC] internal-order callback buffers

@@ -262,8 +262,9 @@ gather_fn gather_kernel(int ell_w, int ek) {
 // a face jump (hR - hL) + (lR - lL) keeps FP32 relative accuracy of the jump itself while
 // the face arithmetic issues FP32 instructions only.  The primitives are formed in
 // double-float arithmetic (df_*: FP32 pipe); only the Jv perturbation y + s v is FP64.
-// Layout: 16 floats (64 B) per cell = (rho, u, v, w, H, p) hi, (rho, u, v, w, H, p) lo,
-// sqrt(rho), 0, 0, 0.
+// Layout: 12 floats (48 B) per cell = (rho, u, v, w, H, p) hi, (rho, u, v, w, H, p) lo.  sqrt(rho)
+// is formed by whoever loads the cell: a fourth 16-byte load per neighbour cost more on a kernel
+// whose L1 is 76% busy than ten FP32 instructions (FP32 Jv at 80^3 x 6 tetrahedra: 293 -> 268 us).
 // kV: the state is y + s v (a Jv), else y; a compile-time switch, so a residual issues no
 // predicated-off FP64 FMAs.  kJac: for the Jacobian, which reads the pairs' FP32 sums only:
 // 8 floats (32 B, one sector) per cell = (u, v, w, H, sqrt(rho), 0, 0, 0)
@@ -296,22 +297,21 @@ __global__ void __launch_bounds__(kThreads) k_prim_hl(int nC, const double* __re
     w4[1] = make_float4(sqrtf(r.h + r.l), 0.0f, 0.0f, 0.0f);
     return;
   }
-  float4* w4 = reinterpret_cast<float4*>(W + 16 * (size_t)c);
+  float4* w4 = reinterpret_cast<float4*>(W + 12 * (size_t)c);
   w4[0] = make_float4(r.h, u.h, vv.h, w.h);
   w4[1] = make_float4(H.h, p.h, r.l, u.l);
   w4[2] = make_float4(vv.l, w.l, H.l, p.l);
-  w4[3] = make_float4(sqrtf(r.h + r.l), 0.0f, 0.0f, 0.0f);
 }
 
 struct PHL {
   float h[6], l[6], s;
 };
 __device__ __forceinline__ void load_hl(const float* __restrict__ W, int c, PHL& P) {
-  const float4* w4 = reinterpret_cast<const float4*>(W + 16 * (size_t)c);
-  const float4 a = __ldg(w4), b = __ldg(w4 + 1), d = __ldg(w4 + 2), e = __ldg(w4 + 3);
+  const float4* w4 = reinterpret_cast<const float4*>(W + 12 * (size_t)c);
+  const float4 a = __ldg(w4), b = __ldg(w4 + 1), d = __ldg(w4 + 2);
   P.h[0] = a.x; P.h[1] = a.y; P.h[2] = a.z; P.h[3] = a.w; P.h[4] = b.x; P.h[5] = b.y;
   P.l[0] = b.z; P.l[1] = b.w; P.l[2] = d.x; P.l[3] = d.y; P.l[4] = d.z; P.l[5] = d.w;
-  P.s = e.x;
+  P.s = sqrtf(P.h[0] + P.l[0]);
 }
 
 // Roe flow from means / jumps in flux-difference form (the interior faces of the FP32 flux,
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kThreads) k_bface32(
   double2* F2 = reinterpret_cast<double2*>(F + 6 * (size_t)f);
   if (type == FOS_BC_WALL && !all64) {
     const float4 na = __ldg(faceNA32 + f);
-    const float4* w4 = reinterpret_cast<const float4*>(Whl + 16 * (size_t)lr.x);
+    const float4* w4 = reinterpret_cast<const float4*>(Whl + 12 * (size_t)lr.x);
     const float4 a = __ldg(w4), b = __ldg(w4 + 1);  // (rho, u, v, w), (H, p, ...) hi parts
     const float un = a.y * na.x + a.z * na.y + a.w * na.z;
     const float q2 = a.y * a.y + a.z * a.z + a.w * a.w;
