@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "fos_internal.h"
+#include "fos_device.cuh"
 
 struct fos_ilut {
   int n = 0, lfil = 0, device = 0;
@@ -66,7 +67,11 @@ fos_ilut::~fos_ilut() {
 
 namespace {
 
-constexpr int kWarps = 4;                 // warps (rows in flight) per CTA
+constexpr int kWarps = 4;                 // the capacity limit is that of four rows in a CTA
+#ifndef FOS_ILUT_WARPS
+#define FOS_ILUT_WARPS 5
+#endif
+constexpr int kMaxWarps = 16;             // rows of a CTA: FOS_ILUT_WARPS where they fit
 constexpr long kSpinLimit = 1L << 23;     // polls of a dependency flag before giving up
 constexpr int kErrCapacity = -1, kErrZeroRow = -5, kErrTimeout = -6;
 
@@ -79,16 +84,68 @@ __device__ __forceinline__ void st_release(int* p, int v) {
   asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Spin until flag[j] >= epoch; false when the limit ran out or another warp already gave
-// up (the error word is set), so no wait outlives a failure.
-__device__ __forceinline__ bool wait_row(const int* flag, int j, int epoch, int* ctr, long spin) {
+// The rows a warp knows to be published: bit l of mask is row base + l.
+struct Known {
+  int base;
+  unsigned mask;
+  __device__ __forceinline__ bool has(int j) const {
+    const unsigned d = (unsigned)(j - base);
+    return d < 32u && (mask >> d & 1u);
+  }
+};
+// The warp spins until row j < top is published (flag >= epoch), looking at the 32 rows from j on:
+// the pivots that follow are mostly among them and need no look of their own.  False when the
+// limit ran out or another warp already gave up (the error word is set), so no wait outlives a
+// failure.  The lanes' acquires, ordered before the others' reads by the syncwarp, come after
+// the publishing warps' releases.
+__device__ __forceinline__ bool wait_row(const int* flag, int j, int top, int epoch, int* ctr,
+                                         long spin, int lane, Known& known) {
   for (long it = 0; it < spin; it++) {
-    if (ld_acquire(flag + j) >= epoch) return true;
-    if (*(volatile int*)(ctr + 3) == kErrTimeout) return false;
-    if (it > 8) __nanosleep(32);
+    const bool mine = j + lane < top && ld_acquire(flag + j + lane) >= epoch;
+    const unsigned m = __ballot_sync(~0u, mine);
+    if (m & 1u) {
+      known.base = j;
+      known.mask = m;
+      __syncwarp();
+      return true;
+    }
+    if ((it & 15) == 15) {
+      if (__any_sync(~0u, *(volatile int*)(ctr + 3) == kErrTimeout)) return false;
+      __nanosleep(32);
+    }
   }
   atomicCAS(ctr + 3, 0, kErrTimeout);
   return false;
+}
+// The wait for a row that a warp of this CTA publishes in shared memory
+__device__ __forceinline__ bool wait_local(const int* flag, int* ctr, long spin) {
+  for (long it = 0; it < spin; it++) {
+    const int f = *(const volatile int*)flag;
+    if (__all_sync(~0u, f != 0)) {
+      __threadfence_block();
+      return true;
+    }
+    if ((it & 1023) == 1023 && __any_sync(~0u, *(volatile int*)(ctr + 3) == kErrTimeout)) return false;
+  }
+  atomicCAS(ctr + 3, 0, kErrTimeout);
+  return false;
+}
+
+// |v| > t for t >= 0, by integer comparison (an FP64 one takes the FP64 pipe); false for NaN
+__device__ __forceinline__ bool abs_above(double v, double t) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+  return b <= 0x7ff0000000000000ull && b > (unsigned long long)__double_as_longlong(t);
+}
+// 1 / w correctly rounded, the division's bits.  For a reciprocal within one unit in the last place
+// (rcp64) one step with two fused multiply-adds rounds correctly unless w's significand is all
+// ones (Markstein, IBM J. Res. Dev. 34, 1990): 5 dependent FP64 instructions of 64 clocks instead
+// of the operator's nine or more, on the chain of rows.  The other cases take the operator.
+__device__ __forceinline__ double recip_rn(double w) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(w);
+  const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+  if (e < 64u || e > 1982u || (b & 0xfffffffffffffull) == 0xfffffffffffffull) return 1.0 / w;
+  const double x = rcp64(w);
+  return fma(fma(-w, x, 1.0), x, x);
 }
 
 __device__ __forceinline__ void set_error(int* ctr, int code, int row) {
@@ -118,33 +175,81 @@ __device__ __forceinline__ void hinsert(int* hkey, int* hpos, unsigned mask, int
   }
 }
 
-// SPARSKIT qsplit (ilut.f:2376-2434) on one lane: the ncut largest |a| first.
-__device__ __forceinline__ void qsplit(double* a, int* ind, int n, int ncut) {
+__device__ __forceinline__ unsigned lanes_below(int lane) { return (1u << lane) - 1u; }
+
+// SPARSKIT qsplit (ilut.f:2376-2434): the ncut largest |a| first, by the warp, every element where
+// the sequential routine leaves it.  A pass over [first, last] with key |a(first)| walks
+// j = first + 1, ... and swaps element j to the end of the larger ones when it is larger.  In
+// slots t = j - first: the larger elements end up in order in slots 1, 2, ...; the others form a
+// queue behind them whose front goes to slot t whenever x_t is larger.  So with c_t the number of
+// larger elements before t, slot t receives x_t, or for a larger x_t what slot c_t + 1 held, and
+// the final content of a slot is found by following those links back to a smaller element.  sa,
+// si, src: scratch of n.  One lane took 20 us for a row whose U part outgrew lfil, on the chain of
+// rows; a pass is a few hundred clocks.
+__device__ __forceinline__ void qsplit(double* a, int* ind, int n, int ncut, double* sa, int* si,
+                                       int* src, int lane) {
   int first = 0, last = n - 1;
   const int cut = ncut - 1;
   if (cut < first || cut > last) return;
   for (;;) {
-    int mid = first;
-    const double key = fabs(a[mid]);
-    for (int j = first + 1; j <= last; j++)
-      if (fabs(a[j]) > key) {
-        mid++;
-        const double t = a[mid]; a[mid] = a[j]; a[j] = t;
-        const int it = ind[mid]; ind[mid] = ind[j]; ind[j] = it;
+    const double key = fabs(a[first]);
+    const int m = last - first;
+    int larger = 0;
+    for (int t0 = 1; t0 <= m; t0 += 32) {
+      const int t = t0 + lane;
+      double v = 0.0;
+      bool g = false;
+      if (t <= m) {
+        v = a[first + t];
+        g = abs_above(v, key);
+        sa[t] = v;
+        si[t] = ind[first + t];
       }
-    const double t = a[mid]; a[mid] = a[first]; a[first] = t;
-    const int it = ind[mid]; ind[mid] = ind[first]; ind[first] = it;
+      const unsigned bg = __ballot_sync(~0u, g);
+      if (t <= m) src[t] = g ? larger + __popc(bg & lanes_below(lane)) + 1 : t;
+      larger += __popc(bg);
+    }
+    __syncwarp();
+    for (int t = 1 + lane; t <= m; t += 32) {
+      if (abs_above(sa[t], key)) {
+        a[first + src[t]] = sa[t];
+        ind[first + src[t]] = si[t];
+      }
+      if (t > larger) {
+        int q = t;
+        while (src[q] != q) q = src[q];
+        a[first + t] = sa[q];
+        ind[first + t] = si[q];
+      }
+    }
+    __syncwarp();
+    const int mid = first + larger;
+    if (lane == 0) {
+      const double v = a[mid]; a[mid] = a[first]; a[first] = v;
+      const int i = ind[mid]; ind[mid] = ind[first]; ind[first] = i;
+    }
+    __syncwarp();
     if (mid == cut) return;
     if (mid > cut) last = mid - 1; else first = mid + 1;
   }
 }
 
-__device__ __forceinline__ unsigned lanes_below(int lane) { return (1u << lane) - 1u; }
+// One row per warp, the rows of a CTA consecutive; shared memory per warp: lval, uval [cap]
+// doubles, lcol, ucol [cap] ints, hash keys and positions [4 cap] ints (56 cap bytes).  At most
+// 2 cap keys go into the hash, so at least half of its slots stay empty and every probe
+// sequence ends.
+// What bounds it is the chain of rows (nearly every row of the Euler P reads the row just
+// above): from a row's last update to the next row's.  Rows of one CTA hand over in shared memory
+// (pivot, U part and flag); only the first of them waits for another CTA's release through the L2.
+// A finished row's first 64 U entries, pivot and count are read at once.  Measured on P of
+// 20,160 tetrahedra (100,800 rows): @@
+struct IlutShared {
+  int group;
+  int flag[kMaxWarps], cnt[kMaxWarps], lev[kMaxWarps];  // a finished row: set last, U entries, level
+  double dinv[kMaxWarps];
+};
 
-// One row per warp; shared memory per warp: lval, uval [cap] doubles, lcol, ucol [cap] ints,
-// hash keys and positions [4 cap] ints (56 cap bytes).  At most 2 cap keys go into the hash,
-// so at least half of its slots stay empty and every probe sequence ends.
-__global__ void __launch_bounds__(32 * kWarps) k_ilut_factor(
+__global__ void __launch_bounds__(32 * kMaxWarps, 1) k_ilut_factor(
     int n, const int* __restrict__ ia, const int* __restrict__ ja, const double* __restrict__ a,
     int lfil, double droptol, int cap, int epoch, int* __restrict__ Lcol,
     double* __restrict__ Lval, int* __restrict__ Lcnt, int* __restrict__ Ucol,
@@ -155,6 +260,8 @@ __global__ void __launch_bounds__(32 * kWarps) k_ilut_factor(
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned hmask = 4u * cap - 1u;
+  __shared__ IlutShared sh;
+  const int nw = blockDim.x >> 5;
   unsigned char* base = smem + (size_t)wid * 56 * cap;
   double* lval = reinterpret_cast<double*>(base);
   double* uval = lval + cap;
@@ -164,10 +271,14 @@ __global__ void __launch_bounds__(32 * kWarps) k_ilut_factor(
   int* hpos = hkey + 4 * cap;
   const size_t slot = (size_t)(lfil > 0 ? lfil : 1);
   for (;;) {
-    int ii = 0;
-    if (lane == 0) ii = atomicAdd(ctr, 1);
-    ii = __shfl_sync(~0u, ii, 0);
-    if (ii >= n) return;
+    __syncthreads();  // the rows of the last group have been read
+    if (threadIdx.x == 0) sh.group = atomicAdd(ctr, 1);
+    if (lane == 0) sh.flag[wid] = 0;
+    __syncthreads();
+    const int g0 = sh.group * nw;  // the group's first row
+    const int ii = g0 + wid;
+    if (g0 >= n) return;
+    if (ii >= n) continue;
     for (int k = lane; k < 4 * cap; k += 32) hkey[k] = -1;
     const int j1 = ia[ii], j2 = ia[ii + 1];
     double tnorm = 0.0;
@@ -215,69 +326,125 @@ __global__ void __launch_bounds__(32 * kWarps) k_ilut_factor(
     // largest L-graph level among the rows of stored multipliers (a superset of the kept
     // ones, so 1 + lev is a valid level for the sweeps' claim order)
     int jj = 0, lev = 0;
+    Known known = {0, 0u};
+    // the U row of the pivot expected next (jp, -1: none): its first 64 entries, two to a lane,
+    // its pivot, count and level
+    int jp = -1, pc0 = 0, pc1 = 0, pn = 0, plev = 0;
+    double pd = 0.0, pv0 = 0.0, pv1 = 0.0;
+    auto fetch = [&](int j) {
+      const int* uc = Ucol + (size_t)j * slot;
+      const double* uv = Uval + (size_t)j * slot;
+      jp = j;
+      pd = dinv[j];
+      pn = Ucnt[j];
+      plev = levL[j];
+      if (lane < (int)slot) { pc0 = uc[lane]; pv0 = uv[lane]; }  // (entries past the count unused)
+      if (lane + 32 < (int)slot) { pc1 = uc[lane + 32]; pv1 = uv[lane + 32]; }
+    };
     while (ok && jj < lenl) {
-      int best = INT_MAX, bidx = -1;
-      for (int k = jj + lane; k < lenl; k += 32)
-        if (lcol[k] < best) { best = lcol[k]; bidx = k; }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const int ob = __shfl_xor_sync(~0u, best, o), oi = __shfl_xor_sync(~0u, bidx, o);
-        if (ob < best) { best = ob; bidx = oi; }
+      // the smallest remaining column, and the next one as far as it is known now
+      int m1 = INT_MAX, m2 = INT_MAX, k1 = 0;
+      for (int k = jj + lane; k < lenl; k += 32) {
+        const int cl = lcol[k];
+        if (cl < m1) { m2 = m1; m1 = cl; k1 = k; }
+        else if (cl < m2) m2 = cl;
       }
-      const int jrow = best, k = bidx;
-      if (lane == 0 && k != jj) {
+      const int jrow = __reduce_min_sync(~0u, m1);
+      const unsigned who = __ballot_sync(~0u, m1 == jrow);
+      const int k = __shfl_sync(~0u, k1, __ffs(who) - 1);
+      const int jnext = __reduce_min_sync(~0u, m1 == jrow ? m2 : m1);
+      if (k != jj) {  // swap entries jj and k, their hash positions looked up by two lanes
         const int cj = lcol[jj];
-        lcol[jj] = jrow; lcol[k] = cj;
-        const double t = lval[jj]; lval[jj] = lval[k]; lval[k] = t;
-        int pos;
-        unsigned s1, s2;
-        hfind(hkey, hpos, hmask, jrow, pos, s1);
-        hfind(hkey, hpos, hmask, cj, pos, s2);
-        hpos[s1] = ~jj;
-        hpos[s2] = ~k;
+        const double vj = lval[jj], vk = lval[k];
+        __syncwarp();
+        if (lane < 2) {
+          int pos;
+          unsigned sl;
+          hfind(hkey, hpos, hmask, lane == 0 ? jrow : cj, pos, sl);
+          const int to = lane == 0 ? jj : k;
+          hpos[sl] = ~to;
+          lcol[to] = lane == 0 ? jrow : cj;
+          lval[to] = lane == 0 ? vk : vj;
+        }
       }
       __syncwarp();
-      // lane 0 waits for the pivot row; every lane then acquires the flag itself, which
-      // orders its reads of the row after the pivot warp's release
-      bool ready = false;
-      if (lane == 0) ready = wait_row(done, jrow, epoch, ctr, spin);
-      if (!__shfl_sync(~0u, ready, 0)) { ok = false; break; }
-      (void)ld_acquire(done + jrow);
-      const double fact = __dmul_rn(lval[jj], dinv[jrow]);
-      if (fabs(fact) <= droptol) { jj++; __syncwarp(); continue; }
-      lev = max(lev, levL[jrow]);
-      const int ulen = Ucnt[jrow];
-      const int* uc = Ucol + (size_t)jrow * slot;
-      const double* uv = Uval + (size_t)jrow * slot;
-      for (int c = 0; c < ulen; c += 32) {
-        const int idx = c + lane;
-        const bool valid = idx < ulen;
-        int j = 0, pos = 0;
-        unsigned sl = 0;
-        double s = 0.0;
-        bool found = false;
-        if (valid) {
-          j = uc[idx];
-          s = __dmul_rn(fact, uv[idx]);
-          found = hfind(hkey, hpos, hmask, j, pos, sl);
-        }
-        const bool fill = valid && !found;
-        const unsigned bu = __ballot_sync(~0u, fill && j >= ii);
-        const unsigned bl = __ballot_sync(~0u, fill && j < ii);
-        if (valid && found) {
-          if (pos >= 0) uval[pos] = __dsub_rn(uval[pos], s);
-          else lval[~pos] = __dsub_rn(lval[~pos], s);
-        } else if (fill) {
-          if (j >= ii) {
-            const int p = lenu + __popc(bu & lanes_below(lane));
-            if (p < cap) { ucol[p] = j; uval[p] = -s; hinsert(hkey, hpos, hmask, j, p); }
-          } else {
-            const int p = lenl + __popc(bl & lanes_below(lane));
-            if (p < cap) { lcol[p] = j; lval[p] = -s; hinsert(hkey, hpos, hmask, j, ~p); }
+      const bool local = jrow >= g0;
+      const double lj = lval[jj];
+      double dj, v0, v1;
+      int ulen, lv, c0, c1;
+      const int* uc;
+      const double* uv;
+      if (local) {  // a row of this CTA: in the shared memory of its warp
+        const int w = jrow - g0;
+        if (!wait_local(sh.flag + w, ctr, spin)) { ok = false; break; }
+        dj = *(volatile double*)(sh.dinv + w);
+        ulen = *(volatile int*)(sh.cnt + w);
+        lv = *(volatile int*)(sh.lev + w);
+        unsigned char* ob = smem + (size_t)w * 56 * cap;
+        uv = reinterpret_cast<double*>(ob) + cap + 1;
+        uc = reinterpret_cast<int*>(ob + 16 * (size_t)cap) + cap + 1;
+        c0 = c1 = 0;
+        v0 = v1 = 0.0;
+        if (lane < ulen) { c0 = uc[lane]; v0 = uv[lane]; }
+        if (lane + 32 < ulen) { c1 = uc[lane + 32]; v1 = uv[lane + 32]; }
+      } else {
+        uc = Ucol + (size_t)jrow * slot;
+        uv = Uval + (size_t)jrow * slot;
+        if (jp != jrow) {
+          if (!known.has(jrow) && !wait_row(done, jrow, g0, epoch, ctr, spin, lane, known)) {
+            ok = false;
+            break;
           }
+          fetch(jrow);
         }
-        lenu += __popc(bu);
-        lenl += __popc(bl);
+        dj = pd; ulen = pn; lv = plev;
+        c0 = pc0; c1 = pc1; v0 = pv0; v1 = pv1;
+        jp = -1;
+      }
+      // on its way while this pivot is worked off; a fill-in may come before it, then it is unused
+      if (jnext < g0 && known.has(jnext)) fetch(jnext);
+      const double fact = __dmul_rn(lj, dj);
+      if (fabs(fact) <= droptol) { jj++; __syncwarp(); continue; }
+      lev = max(lev, lv);
+      // row update, 64 entries at a time: a row's columns are distinct, so the second 32 are
+      // looked up before the first 32 append their fill-ins; positions go in ilut's order
+      for (int c = 0; c < ulen; c += 64) {
+        if (c > 0) {
+          if (c + lane < ulen) { c0 = uc[c + lane]; v0 = uv[c + lane]; }
+          if (c + 32 + lane < ulen) { c1 = uc[c + 32 + lane]; v1 = uv[c + 32 + lane]; }
+        }
+        const bool in0 = c + lane < ulen, in1 = c + 32 + lane < ulen;
+        int p0 = 0, p1 = 0;
+        unsigned sl;
+        const bool f0 = in0 && hfind(hkey, hpos, hmask, c0, p0, sl);
+        const bool f1 = in1 && hfind(hkey, hpos, hmask, c1, p1, sl);
+        const double s0 = __dmul_rn(fact, v0), s1 = __dmul_rn(fact, v1);
+        __syncwarp();
+        auto update = [&](bool found, int pos, double sv) {
+          if (found) {
+            double* t = pos >= 0 ? uval + pos : lval + ~pos;
+            *t = __dsub_rn(*t, sv);
+          }
+        };
+        update(f0, p0, s0);
+        update(f1, p1, s1);
+        auto append = [&](bool fill, int j, double sv) {
+          const unsigned bu = __ballot_sync(~0u, fill && j >= ii);
+          const unsigned bl = __ballot_sync(~0u, fill && j < ii);
+          if (fill) {
+            if (j >= ii) {
+              const int q = lenu + __popc(bu & lanes_below(lane));
+              if (q < cap) { ucol[q] = j; uval[q] = -sv; hinsert(hkey, hpos, hmask, j, q); }
+            } else {
+              const int q = lenl + __popc(bl & lanes_below(lane));
+              if (q < cap) { lcol[q] = j; lval[q] = -sv; hinsert(hkey, hpos, hmask, j, ~q); }
+            }
+          }
+          lenu += __popc(bu);
+          lenl += __popc(bl);
+        };
+        append(in0 && !f0, c0, s0);
+        append(in1 && !f1, c1, s1);
         __syncwarp();
       }
       if (lenl > cap || lenu > cap) { ok = false; break; }
@@ -293,8 +460,14 @@ __global__ void __launch_bounds__(32 * kWarps) k_ilut_factor(
         Ucnt[ii] = 0;
         dinv[ii] = 0.0;
         levL[ii] = 1;
+        sh.cnt[wid] = 0;
+        sh.dinv[wid] = 0.0;
+        sh.lev[wid] = 1;
         __threadfence();
-        if (ii != withhold) st_release(done + ii, epoch);
+        if (ii != withhold) {
+          *(volatile int*)(sh.flag + wid) = 1;
+          st_release(done + ii, epoch);
+        }
       }
       __syncwarp();
       continue;
@@ -302,13 +475,16 @@ __global__ void __launch_bounds__(32 * kWarps) k_ilut_factor(
     // U part first (the rows below wait for it): drop |w| <= droptol * tnorm keeping the
     // order, keep the largest (ilut.f:258-287), publish U and the inverted pivot
     const double thr = __dmul_rn(droptol, tnorm);
+    double w0 = uval[0];
+    if (w0 == 0.0) w0 = __dmul_rn(__dadd_rn(0.0001, droptol), tnorm);
+    const double di = recip_rn(w0);
     int cnt = 0;
     for (int c = 1; c < lenu; c += 32) {
       const int idx = c + lane;
       const bool valid = idx < lenu;
       const double v = valid ? uval[idx] : 0.0;
       const int col = valid ? ucol[idx] : 0;
-      const bool keep = valid && fabs(v) > thr;
+      const bool keep = valid && abs_above(v, thr);
       const unsigned b = __ballot_sync(~0u, keep);
       __syncwarp();
       if (keep) {
@@ -321,17 +497,25 @@ __global__ void __launch_bounds__(32 * kWarps) k_ilut_factor(
     }
     const int lenu2 = cnt + 1;
     const int keepu = min(lenu2, lfil);
-    if (lane == 0) qsplit(uval + 1, ucol + 1, lenu2 - 1, keepu);
+    // (the hash is done with: its room holds the scratch of the quick-splits)
+    double* sa = reinterpret_cast<double*>(hkey);
+    int* si = reinterpret_cast<int*>(sa + cap);
+    qsplit(uval + 1, ucol + 1, lenu2 - 1, keepu, sa, si, si + cap, lane);
     __syncwarp();
     const int nu = max(keepu - 1, 0);
+    if (lane == 0) {  // for the rows of this CTA (the U part is in place, ordered by the syncwarp)
+      sh.dinv[wid] = di;
+      sh.cnt[wid] = nu;
+      sh.lev[wid] = lev + 1;
+      __threadfence_block();
+      if (ii != withhold) *(volatile int*)(sh.flag + wid) = 1;
+    }
     for (int k = lane; k < nu; k += 32) {
       Ucol[(size_t)ii * slot + k] = ucol[1 + k];
       Uval[(size_t)ii * slot + k] = uval[1 + k];
     }
     if (lane == 0) {
-      double w0 = uval[0];
-      if (w0 == 0.0) w0 = __dmul_rn(__dadd_rn(0.0001, droptol), tnorm);
-      dinv[ii] = 1.0 / w0;
+      dinv[ii] = di;
       Ucnt[ii] = nu;
       levL[ii] = lev + 1;
     }
@@ -341,7 +525,7 @@ __global__ void __launch_bounds__(32 * kWarps) k_ilut_factor(
     // L part afterwards, off the rows-below path: the lfil largest multipliers (:236-254);
     // only the sweeps read it, after this kernel
     const int keepl = min(len, lfil);
-    if (lane == 0) qsplit(lval, lcol, len, keepl);
+    qsplit(lval, lcol, len, keepl, sa, si, si + cap, lane);
     __syncwarp();
     for (int k = lane; k < keepl; k += 32) {
       Lcol[(size_t)ii * slot + k] = lcol[k];
@@ -634,23 +818,25 @@ int fos_ilut_factor_on(fos_ilut* f, const int* ia, const int* ja, const double* 
     }
   }
   for (;;) {
-    const size_t smem = (size_t)kWarps * 56 * f->cap;
-    if (smem > (size_t)smem_max) {
+    const size_t row_smem = (size_t)56 * f->cap;
+    if (kWarps * row_smem > (size_t)smem_max) {
       fos_set_error("fos_ilut_factor_dev: a row outgrew the largest working capacity (" +
                     std::to_string(f->cap / 2) + " entries of L and of U)");
       return -1;
     }
+    const int rows = (int)std::min<size_t>(FOS_ILUT_WARPS, ((size_t)smem_max - 1024) / row_smem);
+    const size_t smem = rows * row_smem;
     FOS_CUDA(cudaFuncSetAttribute(k_ilut_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem));
     FOS_CUDA(cudaMemsetAsync(f->d_ctr, 0, 5 * sizeof(int), s));
     f->fepoch++;
-    const int grid = grid_for((const void*)k_ilut_factor, 32 * kWarps, smem, kWarps, f->n);
-    k_ilut_factor<<<grid, 32 * kWarps, smem, s>>>(f->n, ia, ja, a, f->lfil, droptol, f->cap,
-                                                  f->fepoch, f->d_Lcol, f->d_Lval, f->d_Lcnt,
-                                                  f->d_Ucol, f->d_Uval, f->d_Ucnt, f->d_dinv,
-                                                  f->d_levL, f->d_done, f->d_ctr,
-                                                  f->spin_limit > 0 ? f->spin_limit : kSpinLimit,
-                                                  f->withhold);
+    const int grid = grid_for((const void*)k_ilut_factor, 32 * rows, smem, rows, f->n);
+    k_ilut_factor<<<grid, 32 * rows, smem, s>>>(f->n, ia, ja, a, f->lfil, droptol, f->cap, f->fepoch,
+                                                f->d_Lcol, f->d_Lval, f->d_Lcnt, f->d_Ucol,
+                                                f->d_Uval, f->d_Ucnt, f->d_dinv, f->d_levL,
+                                                f->d_done, f->d_ctr,
+                                                f->spin_limit > 0 ? f->spin_limit : kSpinLimit,
+                                                f->withhold);
     f->launches++;
     FOS_CUDA(cudaGetLastError());
     FOS_CUDA(cudaMemcpyAsync(f->h_ctr, f->d_ctr, 8 * sizeof(int), cudaMemcpyDeviceToHost, s));
