@@ -136,6 +136,12 @@ __device__ __forceinline__ bool abs_above(double v, double t) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
   return b <= 0x7ff0000000000000ull && b > (unsigned long long)__double_as_longlong(t);
 }
+// |v| <= t; false for NaN
+__device__ __forceinline__ bool abs_within(double v, double t) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+  const unsigned long long c = (unsigned long long)__double_as_longlong(t);
+  return c <= 0x7ff0000000000000ull ? b <= c : fabs(v) <= t;
+}
 // 1 / w correctly rounded, the division's bits.  For a reciprocal within one unit in the last place
 // (rcp64) one step with two fused multiply-adds rounds correctly unless w's significand is all
 // ones (Markstein, IBM J. Res. Dev. 34, 1990): 5 dependent FP64 instructions of 64 clocks instead
@@ -185,12 +191,52 @@ __device__ __forceinline__ unsigned lanes_below(int lane) { return (1u << lane) 
 // larger elements before t, slot t receives x_t, or for a larger x_t what slot c_t + 1 held, and
 // the final content of a slot is found by following those links back to a smaller element.  sa,
 // si, src: scratch of n.  One lane took 20 us for a row whose U part outgrew lfil, on the chain of
-// rows; a pass is a few hundred clocks.
+// rows.  Up to 65 elements the links come from the ballots of the comparisons, without scratch.
+// passes over at most 65 elements
+__device__ __forceinline__ void qsplit_tail(double* a, int* ind, int first, int last, int cut,
+                                            int lane) {
+  for (;;) {
+    const double key = a[first];
+    const int m = last - first, t0 = 1 + lane, t1 = 33 + lane;  // the lane's two slots
+    const double w0 = t0 <= m ? a[first + t0] : 0.0, w1 = t1 <= m ? a[first + t1] : 0.0;
+    const int i0 = t0 <= m ? ind[first + t0] : 0, i1 = t1 <= m ? ind[first + t1] : 0;
+    const int ikey = ind[first];
+    const bool g0 = t0 <= m && abs_above(w0, fabs(key)), g1 = t1 <= m && abs_above(w1, fabs(key));
+    const unsigned long long G = (unsigned long long)__ballot_sync(~0u, g0) |
+                                 (unsigned long long)__ballot_sync(~0u, g1) << 32;  // bit t - 1
+    const int larger = __popcll(G);
+    auto before = [&](int t) { return __popcll(G & ((1ull << (t - 1)) - 1ull)); };
+    auto source = [&](int t) {  // the slot whose element ends up in slot t > larger
+      while (G >> (t - 1) & 1ull) t = before(t) + 1;
+      return t;
+    };
+    double r0 = 0.0, r1 = 0.0;
+    int k0 = 0, k1 = 0;
+    if (t0 > larger && t0 <= m) { const int q = source(t0); r0 = a[first + q]; k0 = ind[first + q]; }
+    if (t1 > larger && t1 <= m) { const int q = source(t1); r1 = a[first + q]; k1 = ind[first + q]; }
+    __syncwarp();
+    // larger elements in order to slots 1 ..., the last of them to the pivot's place, which goes
+    // to slot `larger`; then the others
+    if (g0) { const int d = before(t0) + 1, e = first + (d == larger ? 0 : d); a[e] = w0; ind[e] = i0; }
+    if (g1) { const int d = before(t1) + 1, e = first + (d == larger ? 0 : d); a[e] = w1; ind[e] = i1; }
+    if (t0 > larger && t0 <= m) { a[first + t0] = r0; ind[first + t0] = k0; }
+    if (t1 > larger && t1 <= m) { a[first + t1] = r1; ind[first + t1] = k1; }
+    if (lane == 0) { a[first + larger] = key; ind[first + larger] = ikey; }
+    __syncwarp();
+    const int mid = first + larger;
+    if (mid == cut) return;
+    if (mid > cut) last = mid - 1; else first = mid + 1;
+  }
+}
 __device__ __forceinline__ void qsplit(double* a, int* ind, int n, int ncut, double* sa, int* si,
                                        int* src, int lane) {
   int first = 0, last = n - 1;
   const int cut = ncut - 1;
   if (cut < first || cut > last) return;
+  if (last - first <= 64) {
+    qsplit_tail(a, ind, first, last, cut, lane);
+    return;
+  }
   for (;;) {
     const double key = fabs(a[first]);
     const int m = last - first;
@@ -231,6 +277,10 @@ __device__ __forceinline__ void qsplit(double* a, int* ind, int n, int ncut, dou
     __syncwarp();
     if (mid == cut) return;
     if (mid > cut) last = mid - 1; else first = mid + 1;
+    if (last - first <= 64) {
+      qsplit_tail(a, ind, first, last, cut, lane);
+      return;
+    }
   }
 }
 
@@ -292,6 +342,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) k_ilut_factor(
       ok = false;
     }
     tnorm = tnorm / (double)(j2 - j1);
+    const double thr = __dmul_rn(droptol, tnorm);
     __syncwarp();
     if (ok) {
       // unpack: L in CSR order, U with the diagonal first, then CSR order
@@ -383,10 +434,10 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) k_ilut_factor(
         unsigned char* ob = smem + (size_t)w * 56 * cap;
         uv = reinterpret_cast<double*>(ob) + cap + 1;
         uc = reinterpret_cast<int*>(ob + 16 * (size_t)cap) + cap + 1;
-        c0 = c1 = 0;
-        v0 = v1 = 0.0;
-        if (lane < ulen) { c0 = uc[lane]; v0 = uv[lane]; }
-        if (lane + 32 < ulen) { c1 = uc[lane + 32]; v1 = uv[lane + 32]; }
+        c0 = uc[lane];  // (cap >= 256: in the arrays; entries past ulen unused)
+        v0 = uv[lane];
+        c1 = uc[lane + 32];
+        v1 = uv[lane + 32];
       } else {
         uc = Ucol + (size_t)jrow * slot;
         uv = Uval + (size_t)jrow * slot;
@@ -404,7 +455,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) k_ilut_factor(
       // on its way while this pivot is worked off; a fill-in may come before it, then it is unused
       if (jnext < g0 && known.has(jnext)) fetch(jnext);
       const double fact = __dmul_rn(lj, dj);
-      if (fabs(fact) <= droptol) { jj++; __syncwarp(); continue; }
+      if (abs_within(fact, droptol)) { jj++; __syncwarp(); continue; }
       lev = max(lev, lv);
       // row update, 64 entries at a time: a row's columns are distinct, so the second 32 are
       // looked up before the first 32 append their fill-ins; positions go in ilut's order
@@ -474,25 +525,22 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) k_ilut_factor(
     }
     // U part first (the rows below wait for it): drop |w| <= droptol * tnorm keeping the
     // order, keep the largest (ilut.f:258-287), publish U and the inverted pivot
-    const double thr = __dmul_rn(droptol, tnorm);
     double w0 = uval[0];
-    if (w0 == 0.0) w0 = __dmul_rn(__dadd_rn(0.0001, droptol), tnorm);
+    if (abs_within(w0, 0.0)) w0 = __dmul_rn(__dadd_rn(0.0001, droptol), tnorm);
     const double di = recip_rn(w0);
     int cnt = 0;
-    for (int c = 1; c < lenu; c += 32) {
-      const int idx = c + lane;
-      const bool valid = idx < lenu;
-      const double v = valid ? uval[idx] : 0.0;
-      const int col = valid ? ucol[idx] : 0;
-      const bool keep = valid && abs_above(v, thr);
-      const unsigned b = __ballot_sync(~0u, keep);
+    for (int c = 1; c < lenu; c += 64) {  // (64 at a time: one wait on the reads, one on the writes)
+      const int a0 = c + lane, a1 = c + 32 + lane;
+      const double x0 = a0 < lenu ? uval[a0] : 0.0, x1 = a1 < lenu ? uval[a1] : 0.0;
+      const int q0 = a0 < lenu ? ucol[a0] : 0, q1 = a1 < lenu ? ucol[a1] : 0;
+      const bool keep0 = a0 < lenu && abs_above(x0, thr), keep1 = a1 < lenu && abs_above(x1, thr);
+      const unsigned b0 = __ballot_sync(~0u, keep0), b1 = __ballot_sync(~0u, keep1);
+      const int d0 = 1 + cnt + __popc(b0 & lanes_below(lane));
+      const int d1 = 1 + cnt + __popc(b0) + __popc(b1 & lanes_below(lane));
       __syncwarp();
-      if (keep) {
-        const int d = 1 + cnt + __popc(b & lanes_below(lane));
-        uval[d] = v;
-        ucol[d] = col;
-      }
-      cnt += __popc(b);
+      if (keep0) { uval[d0] = x0; ucol[d0] = q0; }
+      if (keep1) { uval[d1] = x1; ucol[d1] = q1; }
+      cnt += __popc(b0) + __popc(b1);
       __syncwarp();
     }
     const int lenu2 = cnt + 1;
