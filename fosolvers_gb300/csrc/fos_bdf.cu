@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "fos_internal.h"
+#include "fos_device.cuh"
 
 
 // Default scale of the finite-difference increment s = eps (1 + ||y||)/||v||.
@@ -49,29 +50,6 @@ __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
-}
-
-// Sums of eight accumulators over a warp by halving what each lane holds: 9 FP64 additions per
-// lane where eight butterflies take 40 (an FP64 instruction holds its quarter of an SM for 64
-// clocks, so on small grids the trees were most of a dot product).  Lane l then has sum l / 4.
-__device__ __forceinline__ double warp_sum8(const double (&v)[8], int lane) {
-  double a[4], b[2], c;
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const double keep = (lane & 16) ? v[j + 4] : v[j], send = (lane & 16) ? v[j] : v[j + 4];
-    a[j] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-  }
-#pragma unroll
-  for (int j = 0; j < 2; j++) {
-    const double keep = (lane & 8) ? a[j + 2] : a[j], send = (lane & 8) ? a[j] : a[j + 2];
-    b[j] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-  }
-  {
-    const double keep = (lane & 4) ? b[1] : b[0], send = (lane & 4) ? b[0] : b[1];
-    c = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-  }
-  c += __shfl_xor_sync(0xffffffffu, c, 2);
-  return c + __shfl_xor_sync(0xffffffffu, c, 1);
 }
 
 // block-reduce NV accumulators into part[l * gridDim.x + blockIdx.x] (any block size up to kT)
