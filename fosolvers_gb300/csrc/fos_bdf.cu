@@ -94,10 +94,22 @@ __global__ void __launch_bounds__(kT) k_mdot(long n, const double* __restrict__ 
   double acc[NV];
 #pragma unroll
   for (int l = 0; l < NV; l++) acc[l] = 0.0;
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const double wi = w[i];
+  const long step = (long)gridDim.x * blockDim.x;
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 2 * step) {
+    const bool two = i + step < n;  // two unknowns at a time: their loads in flight together
+    double v[2][NV], wi[2] = {w[i], two ? w[i + step] : 0.0};
 #pragma unroll
-    for (int l = 0; l < NV; l++) acc[l] += V[(size_t)l * ldv + i] * wi;
+    for (int l = 0; l < NV; l++) v[0][l] = V[(size_t)l * ldv + i];
+    if (two) {
+#pragma unroll
+      for (int l = 0; l < NV; l++) v[1][l] = V[(size_t)l * ldv + i + step];
+    }
+#pragma unroll
+    for (int l = 0; l < NV; l++) acc[l] += v[0][l] * wi[0];
+    if (two) {
+#pragma unroll
+      for (int l = 0; l < NV; l++) acc[l] += v[1][l] * wi[1];
+    }
   }
   block_reduce_store<NV>(acc, part);
 }
@@ -120,20 +132,28 @@ __global__ void __launch_bounds__(kT) k_update(long n, const double* __restrict_
   double acc[NA];
 #pragma unroll
   for (int l = 0; l < NA; l++) acc[l] = 0.0;
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    double vv[NV];
-    double wi = w[i];
+  const long step = (long)gridDim.x * blockDim.x;
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 2 * step) {
+    const bool two = i + step < n;  // two unknowns at a time, as in k_mdot
+    double vv[2][NV], wi[2] = {w[i], two ? w[i + step] : 0.0};
 #pragma unroll
-    for (int l = 0; l < NV; l++) {
-      vv[l] = V[(size_t)l * ldv + i];
-      wi -= hs[l] * vv[l];
-    }
-    w[i] = wi;
-    if (MODE != 1) {
+    for (int l = 0; l < NV; l++) vv[0][l] = V[(size_t)l * ldv + i];
+    if (two) {
 #pragma unroll
-      for (int l = 0; l < NV; l++) acc[l] += vv[l] * wi;
+      for (int l = 0; l < NV; l++) vv[1][l] = V[(size_t)l * ldv + i + step];
     }
-    if (MODE != 0) acc[NA - 1] += wi * wi;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      if (u == 1 && !two) break;
+#pragma unroll
+      for (int l = 0; l < NV; l++) wi[u] -= hs[l] * vv[u][l];
+      w[i + u * step] = wi[u];
+      if (MODE != 1) {
+#pragma unroll
+        for (int l = 0; l < NV; l++) acc[l] += vv[u][l] * wi[u];
+      }
+      if (MODE != 0) acc[NA - 1] += wi[u] * wi[u];
+    }
   }
   block_reduce_store<NA>(acc, part);
 }
@@ -377,16 +397,15 @@ struct Driver {
     ilu_ref_rate = (its > 0 && bnorm > 0.0 && res > 0.0) ? std::pow(res / bnorm, 1.0 / its) : 0.0;
   }
 
-  // Blocks and threads of the kernels that sum over all unknowns: 128 threads a block, one block
-  // an SM, up to 16 unknowns a thread; beyond that kRedBlocks blocks of kT.  With the large
-  // shape everywhere a thread of a small grid summed one element and the block's trees were the
-  // rest (184,320 unknowns, 15 vectors: 34 us a multi-dot, 13 us this way).
-  int rblocks = kRedBlocks, rthreads = kT;
+  // Blocks of the kernels that sum over all unknowns: one block of kT an SM up to 8 unknowns a
+  // thread, beyond that kRedBlocks.  With the large shape everywhere a thread of a small grid
+  // summed one element and the block's trees were the rest (184,320 unknowns, 15 vectors: 34 us a
+  // multi-dot, 10 us this way; 22 us with 128 threads and one unknown at a time, which leaves
+  // too few loads in flight).
+  int rblocks = kRedBlocks;
   void set_shape() {
-    const long few = 152L * 128 * 16;
-    if (wk.N > few) return;
-    rthreads = 128;
-    rblocks = (int)std::max<long>(1, std::min<long>(152, (wk.N + 127) / 128));
+    const long few = 152L * kT * 8;
+    if (wk.N <= few) rblocks = (int)std::min<long>(152, (wk.N + kT - 1) / kT);
   }
   // k_final over wk.part into device out, and into host (page-locked) when given
   int reduce(int nv, double* out, double* host = nullptr, const int* flag = nullptr) {
@@ -397,7 +416,7 @@ struct Driver {
   int mdot(int nv, const double* V, long ldv, const double* w) {
     switch (nv) {
 #define FOS_MDOT(K) \
-  case K: fos_launch(c, k_mdot<K>, rblocks, rthreads, wk.N, V, ldv, w, wk.part); break;
+  case K: fos_launch(c, k_mdot<K>, rblocks, kT, wk.N, V, ldv, w, wk.part); break;
       FOS_MDOT(1) FOS_MDOT(2) FOS_MDOT(3) FOS_MDOT(4) FOS_MDOT(5) FOS_MDOT(6) FOS_MDOT(7)
       FOS_MDOT(8) FOS_MDOT(9) FOS_MDOT(10) FOS_MDOT(11) FOS_MDOT(12) FOS_MDOT(13) FOS_MDOT(14)
       FOS_MDOT(15) FOS_MDOT(16) FOS_MDOT(17) FOS_MDOT(18) FOS_MDOT(19) FOS_MDOT(20) FOS_MDOT(21)
@@ -413,7 +432,7 @@ struct Driver {
   int update(int nv, const double* V, long ldv, const double* h, double* w, const Coef& s2) {
     switch (nv) {
 #define FOS_UPD(K) \
-  case K: fos_launch(c, k_update<K, MODE>, rblocks, rthreads, wk.N, V, ldv, h, s2, w, wk.part); break;
+  case K: fos_launch(c, k_update<K, MODE>, rblocks, kT, wk.N, V, ldv, h, s2, w, wk.part); break;
       FOS_UPD(1) FOS_UPD(2) FOS_UPD(3) FOS_UPD(4) FOS_UPD(5) FOS_UPD(6) FOS_UPD(7) FOS_UPD(8)
       FOS_UPD(9) FOS_UPD(10) FOS_UPD(11) FOS_UPD(12) FOS_UPD(13) FOS_UPD(14) FOS_UPD(15)
       FOS_UPD(16) FOS_UPD(17) FOS_UPD(18) FOS_UPD(19) FOS_UPD(20) FOS_UPD(21) FOS_UPD(22)
@@ -515,7 +534,7 @@ struct Driver {
       int rc = fos_residual_launch(c, y, nullptr, nullptr, nullptr, wk.f, 0.0, 0.0, 0);
       if (rc) return rc;
       st.n_rhs++;
-      fos_launch(c, k_newton_res, rblocks, rthreads, N, (const double*)y, (const double*)wk.f,
+      fos_launch(c, k_newton_res, rblocks, kT, N, (const double*)y, (const double*)wk.f,
                  hist, gamma, wk.b, wk.V, wk.part);
       if ((rc = reduce(2, wk.sc, c->h_scal, c->d_flag))) return rc;
       FOS_CUDA(cudaStreamSynchronize(c->stream));
@@ -965,7 +984,7 @@ struct Adapt {
   }
   // ||a||_WRMS with weights from w
   int wrms(const double* a, const double* w, double rtol, double atol, double* out) {
-    fos_launch(c, k_wrms_part, dr.rblocks, dr.rthreads, N, a, w, rtol, atol, wk.part);
+    fos_launch(c, k_wrms_part, dr.rblocks, kT, N, a, w, rtol, atol, wk.part);
     if (int rc = dr.reduce(1, wk.sc + 5 * kMaxVec, c->h_scal)) return rc;
     FOS_CUDA(cudaStreamSynchronize(c->stream));
     *out = std::sqrt(c->h_scal[0] / (double)N);
