@@ -171,12 +171,14 @@ __global__ void k_final(int nv, int np, const double* __restrict__ part, double*
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = sh[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++) t += sh[w];
-    out[l] = t;
-    if (host) host[l] = t;
-    if (flag && l == 0) host[nv] = *flag ? 1.0 : 0.0;
+  if (threadIdx.x < 32) {
+    double t = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
+    t = warp_sum(t);
+    if (threadIdx.x == 0) {
+      out[l] = t;
+      if (host) host[l] = t;
+      if (flag && l == 0) host[nv] = *flag ? 1.0 : 0.0;
+    }
   }
 }
 
@@ -401,15 +403,18 @@ struct Driver {
   // thread, beyond that kRedBlocks.  With the large shape everywhere a thread of a small grid
   // summed one element and the block's trees were the rest (184,320 unknowns, 15 vectors: 34 us a
   // multi-dot, 10 us this way; 22 us with 128 threads and one unknown at a time, which leaves
-  // too few loads in flight).
+  // too few loads in flight).  Not with the FP32 flux: there a sum in another order moves the
+  // state by an FP64 rounding and some face's FP32 terms by theirs, which is seen at 1e-9 of a
+  // step's result, so its sums keep their order at every size.
   int rblocks = kRedBlocks;
   void set_shape() {
     const long few = 152L * kT * 8;
-    if (wk.N <= few) rblocks = (int)std::min<long>(152, (wk.N + kT - 1) / kT);
+    if (wk.N <= few && !(c->flags & FOS_FLUX_FP32))
+      rblocks = (int)std::min<long>(152, (wk.N + kT - 1) / kT);
   }
   // k_final over wk.part into device out, and into host (page-locked) when given
   int reduce(int nv, double* out, double* host = nullptr, const int* flag = nullptr) {
-    fos_launch(c, k_final, nv, 128, nv, rblocks, wk.part, out, host, flag);
+    fos_launch(c, k_final, nv, 256, nv, rblocks, wk.part, out, host, flag);
     FOS_LAUNCH_CHECK();
     return 0;
   }

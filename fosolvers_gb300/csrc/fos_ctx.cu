@@ -5,7 +5,7 @@
 // Device layout (internal cell order after renumbering):
 //   state vectors      SoA by variable, 5*nC doubles (N_Vector layout)
 //   faceLR  int2[nF]   interior faces (L, R) sorted by (min, max) cell id, then the
-//                      boundary faces (L, condition row) by condition and cell; L/R keep the reference
+//                      boundary faces (L, condition row); L/R keep the reference
 //                      orientation (normal points from L to R)
 //   faceNA  double2[2*nF]  (nx, ny), (nz, area)
 //   crow/cent          per-cell CSR of its faces, entry = face<<1 | (cell is R),
@@ -34,7 +34,7 @@ fos_ctx::~fos_ctx() {
                   d_flag, d_prow, d_pcol, d_pdiag, d_cdiag, d_ipos, d_ord, d_fslot, d_Jraw,
                   d_LU, d_LU32, d_lrows_f, d_lrows_b, d_upd_ptr, d_upd, d_ilu_tmp, d_Jb, d_ierr,
                   d_closure32, d_pia, d_pja, d_pa, d_vol, d_ilut_x, d_plst, d_pdu, d_fsel,
-                  d_yJ, d_cnb, d_cna32, d_pnbL, d_pnbU, d_cslot};
+                  d_yJ, d_cnb, d_cna32, d_pnbL, d_pnbU, d_cslot, d_bord};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h_scal) cudaFreeHost(h_scal);
@@ -242,12 +242,7 @@ extern "C" int fos_ctx_create(fos_ctx** out, int nC, int nE, int nPi, int nPb, c
     if (a1 != b1) return a1 < b1;
     return a < b;
   });
-  // boundary faces by condition, then by cell: a warp then takes one branch of ghost_state, whose
-  // branches cost up to five interior faces of FP64 work each (residual at 41x37x33x6 with six
-  // conditions: 160 -> 150 us)
-  auto bc_of = [&](int i) { return brow[i - nPi] > 0 ? bcType[brow[i - nPi] - 1] : (int)FOS_BC_WALL; };
   std::sort(forder.begin() + nPi, forder.end(), [&](int a, int b) {
-    if (bc_of(a) != bc_of(b)) return bc_of(a) < bc_of(b);
     if (keyL(a) != keyL(b)) return keyL(a) < keyL(b);
     return a < b;
   });
@@ -268,6 +263,14 @@ extern "C" int fos_ctx_create(fos_ctx** out, int nC, int nE, int nPi, int nPb, c
     faceNA32[f] = make_float4((float)normP[3 * i], (float)normP[3 * i + 1],
                               (float)normP[3 * i + 2], (float)aP[i]);
   }
+  // boundary faces by condition, then by cell: the order in which the kernels of boundary faces take
+  // them, so that a warp runs one branch of ghost_state, whose branches cost up to five interior
+  // faces of FP64 work each (residual at 41x37x33x6 with six conditions: 160 -> 150 us, and 136
+  // with these blocks, the longest, launched first)
+  std::vector<int> bord(nPb);
+  std::iota(bord.begin(), bord.end(), nPi);
+  auto bc_of = [&](int f) { return faceLR[f].y > 0 ? bcType[faceLR[f].y - 1] : (int)FOS_BC_WALL; };
+  std::stable_sort(bord.begin(), bord.end(), [&](int a, int b) { return bc_of(a) < bc_of(b); });
   std::vector<int> crow(nC + 1, 0), cent;
   for (int f = 0; f < nP; f++) {
     crow[faceLR[f].x + 1]++;
@@ -326,6 +329,7 @@ extern "C" int fos_ctx_create(fos_ctx** out, int nC, int nE, int nPi, int nPb, c
   FOS_TRY(upload(&c->d_old2new, c->old2new.data(), nC));
   FOS_TRY(upload(&c->d_new2old, c->new2old.data(), nC));
   FOS_TRY(upload(&c->d_faceLR, faceLR.data(), nP));
+  FOS_TRY(upload(&c->d_bord, bord.data(), nPb));
   FOS_TRY(upload(&c->d_faceNA, faceNA.data(), 2 * (size_t)nP));
   FOS_TRY(upload(&c->d_faceNA32, faceNA32.data(), nP));
   FOS_TRY(upload(&c->d_crow, crow.data(), nC + 1));

@@ -56,6 +56,7 @@ struct fos_ctx {
   int* d_old2new = nullptr;
   int* d_new2old = nullptr;
   int2* d_faceLR = nullptr;   // [nF] (L, R) internal ids; boundary faces: (L, bc row)
+  int* d_bord = nullptr;      // [nFb] the boundary faces by condition, then by cell
   double2* d_faceNA = nullptr;  // [2*nF] (nx, ny), (nz, aP)
   float4* d_faceNA32 = nullptr; // [nF]  (nx, ny, nz, aP) for the FP32 flux
   int* d_crow = nullptr;      // [nC+1] cell -> face entries

@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kT) k_jac_ghost64(int nFi, int nF, int nC,
 }
 
 // FP64 form: FP64 primitives and geometry
-__global__ void __launch_bounds__(kT) k_jac_face(int nFi, int nF, int nC,
+__global__ void __launch_bounds__(kT) k_jac_face(int nFi, int nF, int nC, const int* __restrict__ bord,
                                                  const int2* __restrict__ faceLR,
                                                  const double2* __restrict__ faceNA,
                                                  const double* __restrict__ W,
@@ -262,8 +262,9 @@ __global__ void __launch_bounds__(kT) k_jac_face(int nFi, int nF, int nC,
                                                  double g, double r, double* __restrict__ J,
                                                  double* __restrict__ Jb) {
   pdl_entry();
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  int f = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;  // boundary faces first
   if (f >= nF) return;
+  if (f >= nFi) f = bord[f - nFi];
   const int2 lr = faceLR[f];
   const double2 n01 = faceNA[2 * (size_t)f], n2a = faceNA[2 * (size_t)f + 1];
   const double n[3] = {n01.x, n01.y, n2a.x};
@@ -1484,7 +1485,7 @@ static int jac_assemble_t(fos_ctx* c, const double* y) {
   } else {
     double* Jb = reinterpret_cast<double*>(c->d_Jb);
     if (int rc = fos_prim_launch(c, y)) return rc;
-    fos_launch(c, k_jac_face, nb(c->nF), kT, c->nFi, c->nF, c->nC,
+    fos_launch(c, k_jac_face, nb(c->nF), kT, c->nFi, c->nF, c->nC, (const int*)c->d_bord,
                (const int2*)c->d_faceLR, (const double2*)c->d_faceNA, (const double*)c->d_W, y,
                (const int*)c->d_fslot, (const int*)c->d_bcT, (const double*)c->d_bcP, c->maxP,
                c->gamm, c->r, J, Jb);
@@ -1619,7 +1620,9 @@ static int ilu_apply_t(fos_ctx* c, const TF* LU, const double* r, double* z, dou
                (const TF*)yv, zv);
   }
   if (d_zsq) {
-    const int blocks = std::min(kRedBlocks, nb(c->nC, kRedThreads));
+    // (the FP32 flux keeps the order of this sum at every size)
+    const int blocks = (c->flags & FOS_FLUX_FP32) ? kRedBlocks
+                                                  : std::min(kRedBlocks, nb(c->nC, kRedThreads));
     fos_launch(c, k_ilu_out_sq<TF>, blocks, kRedThreads, c->nC, (const int*)c->d_ipos,
                (const TF*)zv, z, c->d_red);
     FOS_LAUNCH_CHECK();

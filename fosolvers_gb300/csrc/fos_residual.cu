@@ -122,13 +122,17 @@ __global__ void __launch_bounds__(kThreads) k_prim64(int nC, const double* __res
 }
 
 __global__ void __launch_bounds__(kThreads) k_face64(
-    int nFi, int nF, int nC, const int2* __restrict__ faceLR, const double2* __restrict__ faceNA,
+    int nFi, int nF, int nC, const int* __restrict__ bord, const int2* __restrict__ faceLR,
+    const double2* __restrict__ faceNA,
     const double* __restrict__ W, const double* __restrict__ y, const double* __restrict__ v,
     const double* __restrict__ d_s, const int* __restrict__ bcT, const double* __restrict__ bcP,
     int maxP, double g, double r, double* __restrict__ F) {
   pdl_entry();
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  // last blocks first: the boundary faces, which are dear, do not end up in the last wave, and the
+  // primitives written last by k_prim64 are read while they are in the L2
+  int f = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
   if (f >= nF) return;
+  if (f >= nFi) f = __ldg(bord + f - nFi);
   const int2 lr = __ldg(faceLR + f);
   const double2 n01 = __ldg(faceNA + 2 * (size_t)f), n2a = __ldg(faceNA + 2 * (size_t)f + 1);
   const double nx = n01.x, ny = n01.y, nz = n2a.x, aP = n2a.y;
@@ -367,14 +371,16 @@ __device__ __forceinline__ void roe_split_mj(T rm, T dr, T um, T du, T vm, T dv,
 //   other conditions (and walls too with FOS_FLUX_HYBRID, all64): k_face64's FP64 flow
 //     (interior and ghost primitives from the conserved variables) minus the own flux, in FP64.
 __global__ void __launch_bounds__(kThreads) k_bface32(
-    int nFi, int nF, int nC, const int2* __restrict__ faceLR, const double2* __restrict__ faceNA,
+    int nFi, int nF, int nC, const int* __restrict__ bord, const int2* __restrict__ faceLR,
+    const double2* __restrict__ faceNA,
     const float4* __restrict__ faceNA32, const float* __restrict__ Whl, float gm1f,
     const double* __restrict__ y, const double* __restrict__ v, const double* __restrict__ d_s,
     const int* __restrict__ bcT, const double* __restrict__ bcP, int maxP, double g, double r,
     double* __restrict__ F, int all64) {
   pdl_entry();
-  const int f = nFi + blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nF) return;
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= nF - nFi) return;
+  const int f = __ldg(bord + idx);
   const int2 lr = __ldg(faceLR + f);
   const int row = lr.y;
   const int type = row > 0 ? bcT[row - 1] : FOS_BC_WALL;
@@ -414,13 +420,21 @@ __global__ void __launch_bounds__(kThreads) k_bface32(
   F2[2] = make_double2(flow[4] - m * L.H, 0.0);
 }
 
+// the term of boundary face f (cell is L): the FP64 difference of k_bface32, negated
+__device__ __forceinline__ void boundary_term(const double* __restrict__ Fb, int f, double t[5]) {
+  const double2* F2 = reinterpret_cast<const double2*>(Fb + 6 * (size_t)f);
+  const double2 a0 = __ldg(F2), a1 = __ldg(F2 + 1), a2 = __ldg(F2 + 2);
+  t[0] = neg_bits(a0.x); t[1] = neg_bits(a0.y); t[2] = neg_bits(a1.x);
+  t[3] = neg_bits(a1.y); t[4] = neg_bits(a2.x);
+}
+
 // Fused interior flux + cell gather for the FP32 flux (one pass, no face-flow array for
 // interior faces).  Thread per cell: each interior face of the cell is evaluated in the
 // face's own orientation (L = faceLR.x, R = faceLR.y) from the FP32 (hi, lo) means and
 // jumps, FP32 instructions only, so
 // the two cells of a face compute bit-identical (dF, dw) and the scheme stays exactly
-// conservative; the cell then takes -(dF - dw) (cell is L) or -(dF + dw) (cell is R) in
-// FP64, in ascending ELL order.  Boundary faces read the FP64 differences k_bface32 wrote.
+// conservative; the cell then sums -(dF - dw) (cell is L) or -(dF + dw) (cell is R) in
+// ascending ELL order.  Boundary faces read the FP64 differences k_bface32 wrote.
 // Each face is evaluated twice -- cheap FP32 arithmetic in exchange for the 2 x 48 B per face
 // a face-flow array costs in HBM traffic.  Cells that are not closed (Sc non-null: warped
 // faces) also take the own-flux sum the difference form leaves out, -F(u_c).S_c.
@@ -440,7 +454,8 @@ __global__ void __launch_bounds__(kThreads) k_cell32(
     const double2* __restrict__ faceNA64, unsigned char* __restrict__ fsel, float theta,
     double gm1d) {
   pdl_entry();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  // last blocks first: what k_prim_hl wrote and read last is still in the L2
+  const int c = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
   if (c >= nC) return;
   int e[kW], nbr[kW];
   load_ell<kW>(ell, c, e);
@@ -452,11 +467,13 @@ __global__ void __launch_bounds__(kThreads) k_cell32(
   // arithmetic (where negation is exact), so the sums are plain additions.
   // The FP64 flux terms of kHyb are summed in FP64.  Without it every interior term is an FP32
   // number, and the sum is carried as an FP32 pair (error-free TwoSum, its errors summed: about
-  // 48 bits, what the primitives carry) and widened once: 5 FP64 additions a cell instead of 15
-  // (30 for a hexahedron with its closure term), and half the widenings, on a kernel whose FP64
-  // pipe was the bound (a Jv's 25 FP64 instructions took 79 of 109 us at 64^3 x 6: now 15).
-  // The error against 64-bit values is that of the FP32 terms, the same as with FP64 sums.
+  // 48 bits, what the primitives carry; the sum of four such terms is nearly always exact in
+  // either) and widened once, before the boundary faces' FP64 terms and the closure term: 5 FP64
+  // additions a cell instead of 15, and half the widenings, on a kernel whose FP64 pipe was the
+  // bound (a Jv's 25 FP64 instructions took 79 of 109 us at 64^3 x 6: now 15).  The error against
+  // 64-bit values is that of the FP32 terms, the same as with FP64 sums.
   double acc[5];
+  int kb = kW;  // the first boundary face's slot
   float as[5], ae[5];
   auto add = [&](int q, bool first, float t) {
     if (first) {
@@ -529,23 +546,34 @@ __global__ void __launch_bounds__(kThreads) k_cell32(
           else add(q, k == 0, tq);
         }
       }
-    } else {  // boundary face (cell is L): the FP64 difference of k_bface32, negated
-      const double2* F2 = reinterpret_cast<const double2*>(Fb + 6 * (size_t)f);
-      const double2 a0 = __ldg(F2), a1 = __ldg(F2 + 1), a2 = __ldg(F2 + 2);
-      t[0] = neg_bits(a0.x); t[1] = neg_bits(a0.y); t[2] = neg_bits(a1.x);
-      t[3] = neg_bits(a1.y); t[4] = neg_bits(a2.x);
-      if constexpr (!kHyb) {
+    } else if constexpr (kHyb) {
+      boundary_term(Fb, f, t);
+    } else {
+      if (k == 0) {  // (a cell without interior faces)
 #pragma unroll
-        for (int q = 0; q < 5; q++) {
-          const df2 d = df_from_double(t[q]);
-          add(q, k == 0, d.h);
-          ae[q] += d.l;
-        }
+        for (int q = 0; q < 5; q++) as[q] = ae[q] = 0.0f;
       }
+      kb = min(kb, k);
     }
     if constexpr (kHyb) {
 #pragma unroll
       for (int q = 0; q < 5; q++) acc[q] = k == 0 ? t[q] : acc[q] + t[q];
+    }
+  }
+  if constexpr (!kHyb) {
+#pragma unroll
+    for (int q = 0; q < 5; q++)  // (an infinite sum has no rounding error: TwoSum's is a NaN)
+      acc[q] = f2d_bits(as[q]) + f2d_bits(fabsf(as[q]) <= 3.402823466e38f ? ae[q] : 0.0f);
+    // the boundary faces come after the interior ones in ELL order (a loop of its own, so that
+    // cells without any do not issue its FP64 additions predicated off)
+#pragma unroll 1
+    for (int k = kb; k < kW; k++) {
+      const int ek = __ldg(ell + (size_t)kW * c + k);
+      if (ek < 0) break;
+      double t[5];
+      boundary_term(Fb, ek >> 1, t);
+#pragma unroll
+      for (int q = 0; q < 5; q++) acc[q] += t[q];
     }
   }
   // own flux through the closure vector (kSc: the grid has cells whose faces do not close):
@@ -557,14 +585,7 @@ __global__ void __launch_bounds__(kThreads) k_cell32(
     const float own[5] = {t, fmaf(t, P.h[1], P.h[5] * S.x), fmaf(t, P.h[2], P.h[5] * S.y),
                           fmaf(t, P.h[3], P.h[5] * S.z), t * P.h[4]};
 #pragma unroll
-    for (int q = 0; q < 5; q++) {
-      if constexpr (kHyb) acc[q] -= f2d_bits(own[q]);
-      else add(q, false, -own[q]);
-    }
-  }
-  if constexpr (!kHyb) {
-#pragma unroll
-    for (int q = 0; q < 5; q++) acc[q] = f2d_bits(as[q]) + f2d_bits(ae[q]);
+    for (int q = 0; q < 5; q++) acc[q] -= f2d_bits(own[q]);
   }
   gather_epilogue<kE>(nC, c, acc, __ldg(invV + c), vv, fy, d_s, a, out, flag);
 }
@@ -641,19 +662,19 @@ __global__ void k_sum_final(const double* __restrict__ part, int np, double* __r
 // s, 1/s and b/s of the Jv (scal[1..3]; the epilogue reads them as d_s[0..2]) from ||v||^2, the
 // sum of part[0..np), which goes to scal[0] (np = 0: it is there already); one block, its scalar
 // arithmetic by one thread
-__global__ void __launch_bounds__(256) k_sigma(double* scal, const double* __restrict__ part,
-                                               int np, double ynorm, double eps, double b) {
+__global__ void __launch_bounds__(1024) k_sigma(double* scal, const double* __restrict__ part,
+                                                int np, double ynorm, double eps, double b) {
   pdl_entry();
-  __shared__ double sh[8];
+  __shared__ double sh[32];
   double vn2 = 0.0;
-  if (np > 0) {
+  if (np > 0) {  // (the sum of k_sum_final, in its order)
     double q = 0.0;
     for (int i = threadIdx.x; i < np; i += blockDim.x) q += part[i];
     q = warp_sum(q);
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = q;
     __syncthreads();
-    if (threadIdx.x == 0)
-      for (int w = 0; w < (int)(blockDim.x >> 5); w++) vn2 += sh[w];
+    if (threadIdx.x >= 32) return;
+    vn2 = warp_sum(threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0);
   }
   if (threadIdx.x != 0) return;
   if (np > 0) scal[0] = vn2;
@@ -689,7 +710,7 @@ int fos_residual_launch(fos_ctx* c, const double* y, const double* v, const doub
     const bool hyb = (c->flags & FOS_FLUX_HYBRID) != 0;
     if (c->nFb)
       fos_launch(c, k_bface32, nblk(c->nFb), kThreads, c->nFi, c->nF, c->nC,
-                 (const int2*)c->d_faceLR, (const double2*)c->d_faceNA,
+                 (const int*)c->d_bord, (const int2*)c->d_faceLR, (const double2*)c->d_faceNA,
                  (const float4*)c->d_faceNA32, (const float*)c->d_Whl, (float)gm1, y, v, d_s,
                  (const int*)c->d_bcT, (const double*)c->d_bcP, c->maxP, c->gamm, c->r, c->d_F,
                  hyb ? 1 : 0);
@@ -701,7 +722,7 @@ int fos_residual_launch(fos_ctx* c, const double* y, const double* v, const doub
   } else {
     if (v) fos_launch(c, k_prim64<true>, nblk(c->nC), kThreads, c->nC, y, v, d_s, gm1, c->d_W);
     else fos_launch(c, k_prim64<false>, nblk(c->nC), kThreads, c->nC, y, v, d_s, gm1, c->d_W);
-    fos_launch(c, k_face64, nblk(c->nF), kThreads, c->nFi, c->nF, c->nC,
+    fos_launch(c, k_face64, nblk(c->nF), kThreads, c->nFi, c->nF, c->nC, (const int*)c->d_bord,
                (const int2*)c->d_faceLR, (const double2*)c->d_faceNA, (const double*)c->d_W, y, v,
                d_s, (const int*)c->d_bcT, (const double*)c->d_bcP, c->maxP, c->gamm, c->r,
                c->d_F);
@@ -728,13 +749,15 @@ int fos_prim_launch(fos_ctx* c, const double* y) {
 }
 
 // blocks of the sum of squares: about eight elements a thread (more, and smaller, sums on a small
-// vector would be trees), kRedBlocks at most
-static int sumsq_blocks(long n) {
+// vector would be trees), kRedBlocks at most; with the FP32 flux always, so that its products,
+// which see the last bit of the increment, keep the order of the sum
+static int sumsq_blocks(const fos_ctx* c, long n) {
+  if (c->flags & FOS_FLUX_FP32) return kRedBlocks;
   return (int)std::max<long>(1, std::min<long>(kRedBlocks, n / (8L * kRedThreads)));
 }
 
 int fos_norm2_dev(fos_ctx* c, const double* x, long n, double* d_out_sq) {
-  const int np = sumsq_blocks(n);
+  const int np = sumsq_blocks(c, n);
   fos_launch(c, k_sumsq_part, np, kRedThreads, x, n, c->d_red);
   fos_launch(c, k_sum_final, 1, 1024, c->d_red, np, d_out_sq);
   FOS_LAUNCH_CHECK();
@@ -748,14 +771,14 @@ int fos_sum_partials(fos_ctx* c, int np, double* d_out) {
 }
 
 int fos_jv_sigma(fos_ctx* c, double* d_scal, int np, double ynorm, double eps, double b) {
-  fos_launch(c, k_sigma, 1, np > 0 ? 256 : 32, d_scal, (const double*)c->d_red, np, ynorm, eps, b);
+  fos_launch(c, k_sigma, 1, np > 0 ? 1024 : 32, d_scal, (const double*)c->d_red, np, ynorm, eps, b);
   FOS_LAUNCH_CHECK();
   return 0;
 }
 
 int fos_norm2_sigma(fos_ctx* c, const double* x, long n, double* d_scal, double ynorm, double eps,
                     double b) {
-  const int np = sumsq_blocks(n);
+  const int np = sumsq_blocks(c, n);
   fos_launch(c, k_sumsq_part, np, kRedThreads, x, n, c->d_red);
   return fos_jv_sigma(c, d_scal, np, ynorm, eps, b);
 }
@@ -853,7 +876,7 @@ extern "C" int fos_euler_rhs_dev_static(const fos_ctx* c, double t, const double
     k_prim_hl<false><<<nblk(c->nC), kThreads, 0, s>>>(c->nC, y, nullptr, nullptr, gm1, Whl);
     const bool hyb = (c->flags & FOS_FLUX_HYBRID) != 0;
     if (c->nFb)
-      k_bface32<<<nblk(c->nFb), kThreads, 0, s>>>(c->nFi, c->nF, c->nC, c->d_faceLR,
+      k_bface32<<<nblk(c->nFb), kThreads, 0, s>>>(c->nFi, c->nF, c->nC, c->d_bord, c->d_faceLR,
                                                   c->d_faceNA, c->d_faceNA32, Whl, (float)gm1, y,
                                                   nullptr, nullptr, c->d_bcT, c->d_bcP, c->maxP,
                                                   c->gamm, c->r, F, hyb ? 1 : 0);
@@ -866,7 +889,7 @@ extern "C" int fos_euler_rhs_dev_static(const fos_ctx* c, double t, const double
     double* W = reinterpret_cast<double*>(bytes);
     double* F = reinterpret_cast<double*>(bytes + kStaticCellBytes);
     k_prim64<false><<<nblk(c->nC), kThreads, 0, s>>>(c->nC, y, nullptr, nullptr, gm1, W);
-    k_face64<<<nblk(c->nF), kThreads, 0, s>>>(c->nFi, c->nF, c->nC, c->d_faceLR, c->d_faceNA, W,
+    k_face64<<<nblk(c->nF), kThreads, 0, s>>>(c->nFi, c->nF, c->nC, c->d_bord, c->d_faceLR, c->d_faceNA, W,
                                               y, nullptr, nullptr, c->d_bcT, c->d_bcP, c->maxP,
                                               c->gamm, c->r, F);
     gather_kernel(c->ell_w, kEpiRhs)<<<nblk(c->nC), kThreads, 0, s>>>(
