@@ -74,20 +74,34 @@ __device__ __forceinline__ void load_a(const unsigned short* A, int lda, int r0,
   a[2] = p0[4];
   a[3] = p1[4];
 }
-// B fragment when k is contiguous: element (k, n) at B[n * ldn + k] (ldn, k0 even)
-__device__ __forceinline__ void load_b_kc(const unsigned short* B, int ldn, int k0, int n0,
-                                          unsigned b[2]) {
-  const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
-  const unsigned* p = reinterpret_cast<const unsigned*>(B + (n0 + g) * ldn + k0 + 2 * t);
-  b[0] = p[0];
-  b[1] = p[4];
-}
 __device__ __forceinline__ void load_b(const unsigned short* B, int sk, int sn, int k0, int n0,
                                        unsigned b[2]) {
   const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
   const unsigned short* p = B + (k0 + 2 * t) * sk + (n0 + g) * sn;
   b[0] = pack2(p[0], p[sk]);
   b[1] = pack2(p[8 * sk], p[9 * sk]);
+}
+
+// four 8x8 BF16 matrices, the rows at the addresses of lanes 0-7, 8-15, 16-23 and 24-31: the
+// A fragment of a 16 x 16 tile, or the B fragments of two 16 x 8 tiles stored n-major
+// (16-byte aligned rows; 272-byte row strides keep the eight rows in different banks)
+__device__ __forceinline__ void ldmatrix4(const unsigned short* p, unsigned r[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p))
+               : "memory");
+}
+
+// copies into shared memory that do not wait (both addresses aligned to the size)
+template <int kBytes, typename T>
+__device__ __forceinline__ void cp_async(T* dst, const T* src) {
+  static_assert(kBytes == sizeof(T), "one element");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)), "l"(src), "n"(kBytes)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() {  // for the thread's own copies
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 struct GnnScales {
@@ -111,7 +125,10 @@ __device__ __forceinline__ void gate2(const float* __restrict__ Gc, float ex, fl
 // Input layer, 256 cells per CTA.  Phase 1: thread per cell computes the 16 features into
 // shared memory.  Phase 2: a warp per cell, lane l owns hidden channels 2l, 2l+1 with its
 // two rows of W0 (and b0) in registers as pairs: 16 packed FMAs per cell and lane, and the
-// BF16 row of h0 leaves as one coalesced 128-byte store.
+// BF16 row of h0 leaves as one coalesced 128-byte store.  The next chunk's 11 doubles a cell are
+// copied into shared memory during phase 2, and W0 comes through shared memory (511,104 cells:
+// 65 -> 41 us; about half of the issue slots and of the shared-memory wavefronts are used, the
+// rest is the features' chains of divisions and logarithms between two barriers).
 __global__ void __launch_bounds__(256) k_gnn_in(int nC, const double* __restrict__ y,
                                                 const double* __restrict__ v,
                                                 const double* __restrict__ invV, float gam_dt,
@@ -122,13 +139,30 @@ __global__ void __launch_bounds__(256) k_gnn_in(int nC, const double* __restrict
                                                 unsigned short* __restrict__ h0) {
   pdl_entry();
   __shared__ __align__(16) float xs[256][NIN];
+  __shared__ double in[11][256];  // the next chunk's y, v, 1/volume
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int f0 = 2 * lane;
+  const int nchunk = (nC + 255) / 256;
+  auto fetch = [&](int chunk) {
+    const int i = chunk * 256 + threadIdx.x;
+    if (chunk >= nchunk || i >= nC) return;  // (a later chunk number may overflow i)
+#pragma unroll
+    for (int q = 0; q < 5; q++) {
+      cp_async<8>(&in[q][threadIdx.x], y + (size_t)q * nC + i);
+      cp_async<8>(&in[5 + q][threadIdx.x], v + (size_t)q * nC + i);
+    }
+    cp_async<8>(&in[10][threadIdx.x], invV + i);
+  };
+  fetch(blockIdx.x);
+  // W0 through shared memory, channel-minor: a lane's own rows read from global memory would
+  // touch a line a lane and load (rows of 66 keep the transposing stores in different banks)
+  float* ws = &xs[0][0];
+  for (int k = threadIdx.x; k < H * NIN; k += 256) ws[66 * (k % NIN) + k / NIN] = Wb[OFF_W0 + k];
+  __syncthreads();
   float2 w[NIN];
 #pragma unroll
-  for (int k = 0; k < NIN; k++) w[k] = make_float2(Wb[OFF_W0 + NIN * f0 + k], Wb[OFF_W0 + NIN * (f0 + 1) + k]);
+  for (int k = 0; k < NIN; k++) w[k] = *reinterpret_cast<const float2*>(&ws[66 * k + f0]);
   const float2 bias = make_float2(Wb[OFF_B0 + f0], Wb[OFF_B0 + f0 + 1]);
-  const int nchunk = (nC + 255) / 256;
   for (int chunk = blockIdx.x; chunk < nchunk; chunk += gridDim.x) {  // persistent
   const int c0 = chunk * 256;
   __syncthreads();  // the previous chunk's features are consumed
@@ -139,18 +173,22 @@ __global__ void __launch_bounds__(256) k_gnn_in(int nC, const double* __restrict
     for (int k = 0; k < NIN; k++) x[k] = 0.0f;
     if (i < nC) {
       const GnnScales s = *sc;
-      x[0] = d2f_trunc(y[i]) / s.sy[0];
-      x[1] = d2f_trunc(y[(size_t)nC + i]) / s.sy[1];
-      x[2] = d2f_trunc(y[2 * (size_t)nC + i]) / s.sy[1];
-      x[3] = d2f_trunc(y[3 * (size_t)nC + i]) / s.sy[1];
-      x[4] = d2f_trunc(y[4 * (size_t)nC + i]) / s.sy[2];
+      cp_async_wait();  // (its own copies)
+      const float r = d2f_trunc(in[0][threadIdx.x]);
+      const float mx = d2f_trunc(in[1][threadIdx.x]), my = d2f_trunc(in[2][threadIdx.x]),
+                  mz = d2f_trunc(in[3][threadIdx.x]), E = d2f_trunc(in[4][threadIdx.x]);
+      const float iv = d2f_trunc(in[10][threadIdx.x]);
+      float vq[5];
 #pragma unroll
-      for (int q = 0; q < 5; q++) x[5 + q] = d2f_trunc(v[(size_t)q * nC + i]) / s.sv[q];
-      const float iv = d2f_trunc(invV[i]);
+      for (int q = 0; q < 5; q++) vq[q] = d2f_trunc(in[5 + q][threadIdx.x]);
+      x[0] = r / s.sy[0];
+      x[1] = mx / s.sy[1];
+      x[2] = my / s.sy[1];
+      x[3] = mz / s.sy[1];
+      x[4] = E / s.sy[2];
+#pragma unroll
+      for (int q = 0; q < 5; q++) x[5 + q] = vq[q] / s.sv[q];
       x[10] = -logf(iv) - s.lvmean;
-      const float r = d2f_trunc(y[i]);
-      const float mx = d2f_trunc(y[(size_t)nC + i]), my = d2f_trunc(y[2 * (size_t)nC + i]),
-                  mz = d2f_trunc(y[3 * (size_t)nC + i]), E = d2f_trunc(y[4 * (size_t)nC + i]);
       const float q2 = (mx * mx + my * my + mz * mz) / (r * r);
       const float p = (gas_g - 1.0f) * (E - 0.5f * r * q2);
       const float cs = sqrtf(fmaxf(gas_g * p / r, 0.0f));
@@ -168,6 +206,7 @@ __global__ void __launch_bounds__(256) k_gnn_in(int nC, const double* __restrict
           make_float4(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
   }
   __syncthreads();
+  fetch(chunk + gridDim.x);
   // four cells per step (rows r0, r0 + 8, r0 + 16, r0 + 24): independent FMA chains
   constexpr int U = 4;
   for (int r0 = warp; r0 < 256; r0 += 8 * U) {
@@ -196,6 +235,16 @@ __global__ void __launch_bounds__(256) k_gnn_in(int nC, const double* __restrict
   }
 }
 
+// edge features of ELL entry ent with the face's normal and area na, seen from its cell
+__device__ __forceinline__ void edge_features(int ent, float4 na, float inv_amean, float& ex,
+                                              float& ey, float& ez, float& ea) {
+  const float sgn = (ent & 1) ? -1.0f : 1.0f;  // cell is R: outward normal is -n
+  const float a = na.w * inv_amean;
+  ex = sgn * na.x * a;
+  ey = sgn * na.y * a;
+  ez = sgn * na.z * a;
+  ea = a;
+}
 // edge features of ELL entry ent seen from cell i; returns the neighbour cell or -1
 __device__ __forceinline__ int edge_of(int ent, const int2* __restrict__ faceLR, int nFi,
                                        const float4* __restrict__ faceNA, float inv_amean,
@@ -204,30 +253,35 @@ __device__ __forceinline__ int edge_of(int ent, const int2* __restrict__ faceLR,
   const int f = ent >> 1;
   if (f >= nFi) return -1;  // boundary face: no neighbour
   const int2 lr = faceLR[f];
-  const float4 na = faceNA[f];
-  const float sgn = (ent & 1) ? -1.0f : 1.0f;  // cell is R: outward normal is -n
-  const float a = na.w * inv_amean;
-  ex = sgn * na.x * a;
-  ey = sgn * na.y * a;
-  ez = sgn * na.z * a;
-  ea = a;
+  edge_features(ent, faceNA[f], inv_amean, ex, ey, ez, ea);
   return (ent & 1) ? lr.x : lr.y;
 }
 
 // One message-passing layer, persistent over tiles of 64 cells (128 threads):
 //   A. edge phase: the 256 (cell, ELL slot) pairs of the tile -> neighbour index and edge
-//      features in shared memory (all independent loads, one pass);
-//   B. gather + gate (CUDA cores, FP32): warp w takes cells w, w+4, ..., four cells per
-//      step, so 20 rows of h (128 B each) are in flight per warp;
-//   C. [h; bf16(m)] A^T on the tensor cores (mma.sync m16n8k16, BF16 in, FP32 accumulate);
+//      features in shared memory.  Contexts with the per-cell slot copies (FP32 flux or ILU)
+//      have them copied there during the previous tile's phase C, coalesced; the others go from
+//      the ELL entry to the face arrays, two latencies in a row (the network applied to 511,104
+//      cells: 324 us that way, 310 with the copies);
+//   B. gather + gate (CUDA cores, FP32): half a warp a cell, four channels a lane, eight cells per
+//      step, so 40 rows of h (128 B each) are in flight per warp (with 4 cells per step 89 us a
+//      layer, with 8 80 us; a cell per warp reads the edge features twice as often);
+//   C. [h; bf16(m)] A^T on the tensor cores (mma.sync m16n8k16, BF16 in, FP32 accumulate), the
+//      fragments by ldmatrix.  Not tcgen05: its order of accumulation would flip BF16 roundings
+//      of h, and the matrix unit is busy 17% of the time;
 //   D. bias + relu -> BF16 into the warp's own rows of the tile, then coalesced 16-byte stores.
 // The layer weights are loaded once per CTA.  HEAD (last layer) also applies the output
 // head z = s_v (v / s_v + D h3 + d) from the tile in shared memory, so h3 is stored only
-// when training keeps it.  Optionally keeps bf16(m) for the backward pass.
+// when training keeps it; its v arrive in shared memory during the gather.  Optionally keeps
+// bf16(m) for the backward pass.
+// 511,104 cells: 95 -> 80 us a layer and 122 -> 92 with the head.  Bound by the L1: 70% of its
+// wavefronts (2150 a tile: operands of C 640, rows of h 400, edge features 256), 5 CTAs an SM
+// by registers (4 with 126 registers: 83 us); HBM would take 24 us.
 template <bool HEAD>
-__global__ void __launch_bounds__(kT) k_gnn_layer(
+__global__ void __launch_bounds__(kT, 5) k_gnn_layer(
     int nC, int nFi, const int* __restrict__ ell, const int2* __restrict__ faceLR,
-    const float4* __restrict__ faceNA, const GnnScales* __restrict__ sc,
+    const float4* __restrict__ faceNA, const int* __restrict__ cnb,
+    const float4* __restrict__ cna, const GnnScales* __restrict__ sc,
     const float* __restrict__ Wl,            // layer block of the bf16-rounded FP32 weights
     const unsigned short* __restrict__ Ab,   // layer A in BF16 bits, 64 x 128 row-major
     const unsigned short* __restrict__ hin, unsigned short* __restrict__ hout,
@@ -239,9 +293,23 @@ __global__ void __launch_bounds__(kT) k_gnn_layer(
   __shared__ __align__(16) unsigned short As[H][RS];
   __shared__ float bs[H];
   __shared__ __align__(16) int nbr[kTile][4];
+  __shared__ int ent[kTile][4];
   __shared__ float4 ef[kTile][4];
+  __shared__ double vs[HEAD ? 5 : 1][kTile];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
+  const int ntiles = (nC + kTile - 1) / kTile;
+  auto fetch = [&](int tile) {  // a tile's slot copies on their way into shared memory
+    if (!cna || tile >= ntiles) return;
+    for (int p = threadIdx.x; p < kTile * 4; p += kT) {
+      const int r = p >> 2, k = p & 3, i = tile * kTile + r;
+      if (i >= nC) break;  // (and so are the thread's next cells)
+      cp_async<4>(&ent[r][k], ell + 4 * (size_t)i + k);
+      cp_async<4>(&nbr[r][k], cnb + 4 * (size_t)i + k);
+      cp_async<16>(&ef[r][k], cna + (size_t)k * nC + i);
+    }
+  };
+  fetch(blockIdx.x);
   for (int k = threadIdx.x; k < H * (2 * H / 8); k += kT) {
     const int r = k / (2 * H / 8), c = k % (2 * H / 8);
     *reinterpret_cast<uint4*>(&As[r][8 * c]) = reinterpret_cast<const uint4*>(Ab)[k];
@@ -249,81 +317,104 @@ __global__ void __launch_bounds__(kT) k_gnn_layer(
   for (int k = threadIdx.x; k < H; k += kT) bs[k] = Wl[L_B + k];
   const GnnScales s = *sc;
   const float inv_amean = 1.0f / s.amean;
-  const int f0 = 2 * lane;
-  // the lane's gate rows G[f0], G[f0 + 1] and c[f0], c[f0 + 1] in registers, as pairs
-  const float2 gx = make_float2(Wl[L_G + 4 * f0 + 0], Wl[L_G + 4 * f0 + 4]);
-  const float2 gy = make_float2(Wl[L_G + 4 * f0 + 1], Wl[L_G + 4 * f0 + 5]);
-  const float2 gz = make_float2(Wl[L_G + 4 * f0 + 2], Wl[L_G + 4 * f0 + 6]);
-  const float2 ga = make_float2(Wl[L_G + 4 * f0 + 3], Wl[L_G + 4 * f0 + 7]);
-  const float2 gc = make_float2(Wl[L_C + f0], Wl[L_C + f0 + 1]);
-  // output head (last layer): B fragments of D^T (k = hidden channel, n = field) and d
-  unsigned dfr[4][2] = {{0u, 0u}, {0u, 0u}, {0u, 0u}, {0u, 0u}};
-  float dq[2] = {0.0f, 0.0f};
-  if (HEAD) {
+  // the lane's four gate rows G[4 l16 ..] and c[4 l16 ..] in registers, as pairs
+  const int half = lane >> 4, l16 = lane & 15;
+  float2 gx[2], gy[2], gz[2], ga[2], gc[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int f0 = 4 * l16 + 2 * h;
+    gx[h] = make_float2(Wl[L_G + 4 * f0 + 0], Wl[L_G + 4 * f0 + 4]);
+    gy[h] = make_float2(Wl[L_G + 4 * f0 + 1], Wl[L_G + 4 * f0 + 5]);
+    gz[h] = make_float2(Wl[L_G + 4 * f0 + 2], Wl[L_G + 4 * f0 + 6]);
+    ga[h] = make_float2(Wl[L_G + 4 * f0 + 3], Wl[L_G + 4 * f0 + 7]);
+    gc[h] = make_float2(Wl[L_C + f0], Wl[L_C + f0 + 1]);
+  }
+  // output head (last layer): B fragments of D^T (k = hidden channel, n = field) and d, in shared
+  // memory because the gather needs the registers
+  __shared__ uint2 dfr[HEAD ? 4 : 1][32];
+  __shared__ float ds[8];
+  if (HEAD && warp == 0) {
     const int n = g;  // field of this lane's B column
 #pragma unroll
     for (int kk = 0; kk < 4; kk++) {
       const int k0 = 16 * kk + 2 * t;
       auto w = [&](int k) { return n < 5 ? bf(Wb[OFF_D + H * n + k]) : (unsigned short)0; };
-      dfr[kk][0] = pack2(w(k0), w(k0 + 1));
-      dfr[kk][1] = pack2(w(k0 + 8), w(k0 + 9));
+      dfr[kk][lane] = make_uint2(pack2(w(k0), w(k0 + 1)), pack2(w(k0 + 8), w(k0 + 9)));
     }
-    dq[0] = 2 * t < 5 ? Wb[OFF_DB + 2 * t] : 0.0f;
-    dq[1] = 2 * t + 1 < 5 ? Wb[OFF_DB + 2 * t + 1] : 0.0f;
+    if (lane < 8) ds[lane] = lane < 5 ? Wb[OFF_DB + lane] : 0.0f;
   }
-  const int ntiles = (nC + kTile - 1) / kTile;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int c0 = tile * kTile;
-    // A. edges of the tile
+    // A. edges of the tile (each thread finishes the slots that it fetched itself)
+    cp_async_wait();
     for (int p = threadIdx.x; p < kTile * 4; p += kT) {
       const int r = p >> 2, k = p & 3, i = c0 + r;
       int j = -1;
       float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       if (i < nC) {
         float ex, ey, ez, ea;
-        j = edge_of(ell[4 * (size_t)i + k], faceLR, nFi, faceNA, inv_amean, ex, ey, ez, ea);
+        if (cna) {
+          const int en = ent[r][k];
+          if (en >= 0 && (en >> 1) < nFi) {
+            j = nbr[r][k];
+            edge_features(en, ef[r][k], inv_amean, ex, ey, ez, ea);
+          }
+        } else {
+          j = edge_of(ell[4 * (size_t)i + k], faceLR, nFi, faceNA, inv_amean, ex, ey, ez, ea);
+        }
         if (j >= 0) e = make_float4(ex, ey, ez, ea);
       }
       nbr[r][k] = j;
       ef[r][k] = e;
     }
     __syncthreads();  // edges ready; the previous tile's output rows are stored
-    // B. gather + gate, four cells per step; gate and message as packed FP32 FMAs
-    //    (missing neighbours contribute (c + 0) * 0, which leaves the sum unchanged)
+    if (HEAD)  // the tile's v, needed at its end
+      for (int p = threadIdx.x; p < 5 * kTile; p += kT) {
+        const int q = p / kTile, i = c0 + p % kTile;
+        if (i < nC) cp_async<8>(&vs[q][p % kTile], v + (size_t)q * nC + i);
+      }
+    // B. gather + gate, a cell per half warp (four channels a lane), 2 U cells per step; gate and
+    //    message as packed FP32 FMAs (missing neighbours contribute (c + 0) * 0, which leaves
+    //    the sum unchanged)
     constexpr int U = 4;
-    for (int r0 = warp; r0 < kTile; r0 += 4 * U) {
-      unsigned hv[U][4], hs[U];
+    for (int r0 = 2 * warp + half; r0 < kTile; r0 += 8 * U) {
+      uint2 hv[U][4], hs[U];
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        const int r = r0 + 4 * u, i = c0 + r;
+        const int r = r0 + 8 * u, i = c0 + r;
         const int4 nb = *reinterpret_cast<const int4*>(&nbr[r][0]);
         const int js[4] = {nb.x, nb.y, nb.z, nb.w};
-        hs[u] = i < nC ? reinterpret_cast<const unsigned*>(hin + (size_t)H * i)[lane] : 0u;
+        auto row = [&](int j) { return reinterpret_cast<const uint2*>(hin + (size_t)H * j)[l16]; };
+        hs[u] = i < nC ? row(i) : make_uint2(0u, 0u);
 #pragma unroll
-        for (int k = 0; k < 4; k++)
-          hv[u][k] = js[k] >= 0 ? reinterpret_cast<const unsigned*>(hin + (size_t)H * js[k])[lane] : 0u;
+        for (int k = 0; k < 4; k++) hv[u][k] = js[k] >= 0 ? row(js[k]) : make_uint2(0u, 0u);
       }
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        const int r = r0 + 4 * u, i = c0 + r;
-        float2 m = make_float2(0.0f, 0.0f);
+        const int r = r0 + 8 * u, i = c0 + r;
+        float2 m[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
 #pragma unroll
         for (int k = 0; k < 4; k++) {
           const float4 e = ef[r][k];
-          float2 gg = __ffma2_rn(gx, make_float2(e.x, e.x), gc);
-          gg = __ffma2_rn(gy, make_float2(e.y, e.y), gg);
-          gg = __ffma2_rn(gz, make_float2(e.z, e.z), gg);
-          gg = __ffma2_rn(ga, make_float2(e.w, e.w), gg);
-          const unsigned hb = hv[u][k];
-          m = __ffma2_rn(gg, make_float2(__uint_as_float(hb << 16), __uint_as_float(hb & 0xffff0000u)), m);
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            float2 gg = __ffma2_rn(gx[h], make_float2(e.x, e.x), gc[h]);
+            gg = __ffma2_rn(gy[h], make_float2(e.y, e.y), gg);
+            gg = __ffma2_rn(gz[h], make_float2(e.z, e.z), gg);
+            gg = __ffma2_rn(ga[h], make_float2(e.w, e.w), gg);
+            const unsigned hb = h ? hv[u][k].y : hv[u][k].x;
+            m[h] = __ffma2_rn(gg, make_float2(__uint_as_float(hb << 16), __uint_as_float(hb & 0xffff0000u)), m[h]);
+          }
         }
-        const unsigned ms = pack2(bf(m.x), bf(m.y));
-        if (mkeep && i < nC) reinterpret_cast<unsigned*>(mkeep + (size_t)H * i)[lane] = ms;
-        reinterpret_cast<unsigned*>(&Xs[r][0])[lane] = hs[u];
-        reinterpret_cast<unsigned*>(&Xs[r][H])[lane] = ms;
+        const uint2 ms = make_uint2(pack2(bf(m[0].x), bf(m[0].y)), pack2(bf(m[1].x), bf(m[1].y)));
+        if (mkeep && i < nC) reinterpret_cast<uint2*>(mkeep + (size_t)H * i)[l16] = ms;
+        reinterpret_cast<uint2*>(&Xs[r][0])[l16] = hs[u];
+        reinterpret_cast<uint2*>(&Xs[r][H])[l16] = ms;
       }
     }
+    if (HEAD) cp_async_wait();
     __syncthreads();
+    fetch(tile + gridDim.x);  // this tile's edges are consumed
     // C. tensor cores: rows 16*warp .. +15 of the tile, all 64 outputs, K = 128
     float acc[8][4];
 #pragma unroll
@@ -333,13 +424,15 @@ __global__ void __launch_bounds__(kT) k_gnn_layer(
 #pragma unroll
     for (int kk = 0; kk < 2 * H; kk += 16) {
       unsigned a[4];
-      load_a(&Xs[0][0], RS, 16 * warp, kk, a);
+      // lanes 0-15 point at the 16 rows, lanes 16-31 at their second 16 bytes
+      ldmatrix4(&Xs[16 * warp + (lane & 15)][kk + 8 * (lane >> 4)], a);
 #pragma unroll
-      for (int nt = 0; nt < 8; nt++) {
-        unsigned b[2];
-        // B(k, n) = A_l(n, k): k contiguous along the rows of As
-        load_b_kc(&As[0][0], RS, kk, 8 * nt, b);
+      for (int nt = 0; nt < 8; nt += 2) {
+        unsigned b[4];
+        // B(k, n) = A_l(n, k): k contiguous along the rows of As; two 8-column tiles a load
+        ldmatrix4(&As[8 * nt + (lane & 7) + 8 * (lane >> 4)][kk + (lane & 8)], b);
         mma16816(acc[nt], a, b);
+        mma16816(acc[nt + 1], a, b + 2);
       }
     }
     // D. bias + relu -> BF16.  The m16n8 accumulator layout of output columns 16 kk .. +15
@@ -375,7 +468,9 @@ __global__ void __launch_bounds__(kT) k_gnn_layer(
 #pragma unroll
       for (int kk = 0; kk < 4; kk++) {
         const unsigned a[4] = {ob[2 * kk][0], ob[2 * kk][1], ob[2 * kk + 1][0], ob[2 * kk + 1][1]};
-        mma16816(o, a, dfr[kk]);
+        const uint2 d = dfr[kk][lane];
+        const unsigned b[2] = {d.x, d.y};
+        mma16816(o, a, b);
       }
 #pragma unroll
       for (int e = 0; e < 4; e++) {
@@ -383,7 +478,7 @@ __global__ void __launch_bounds__(kT) k_gnn_layer(
         const int i = c0 + 16 * warp + g + ((e & 2) ? 8 : 0);
         if (q < 5 && i < nC) {
           const float svq = sc->sv[q];
-          const float zh = d2f_trunc(v[(size_t)q * nC + i]) / svq + (o[e] + dq[e & 1]);
+          const float zh = d2f_trunc(vs[q][i - c0]) / svq + (o[e] + ds[q]);
           if (zhat) zhat[(size_t)8 * i + q] = zh;
           if (z) z[(size_t)q * nC + i] = f2d_bits(zh * svq);
         }
@@ -434,21 +529,23 @@ __global__ void __launch_bounds__(256) k_gnn_scale_part(int nC, int nF, const do
   if (threadIdx.x < 10) {
     float s = 0.0f;
     for (int k = 0; k < (int)(blockDim.x >> 5); k++) s += sh[k][threadIdx.x];
-    part[10 * blockIdx.x + threadIdx.x] = s;
+    part[gridDim.x * threadIdx.x + blockIdx.x] = s;
   }
 }
-__global__ void k_gnn_scale_final(int nC, int nF, int np, const float* __restrict__ part,
-                                  GnnScales* __restrict__ sc) {
+// a warp per sum: lane l sums partials l, l+32, ... (fixed order), then a shuffle tree
+__global__ void __launch_bounds__(320) k_gnn_scale_final(int nC, int nF, int np,
+                                                         const float* __restrict__ part,
+                                                         GnnScales* __restrict__ sc) {
   pdl_entry();
-  // one warp: lane l sums partials l, l+32, ... (fixed order), then a shuffle tree
-  const int lane = threadIdx.x & 31;
-  float s[10] = {0};
-  for (int b = lane; b < np; b += 32)
-#pragma unroll
-    for (int k = 0; k < 10; k++) s[k] += part[10 * b + k];
-#pragma unroll
-  for (int k = 0; k < 10; k++) s[k] = warp_sumf(s[k]);
-  if (lane != 0) return;
+  __shared__ float s[10];
+  const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+  float t = 0.0f;
+#pragma unroll 8
+  for (int b = lane; b < np; b += 32) t += part[np * k + b];
+  t = warp_sumf(t);
+  if (lane == 0) s[k] = t;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   const float tiny = 1e-30f;
   GnnScales o;
   o.sy[0] = sqrtf(s[0] / nC) + tiny;
@@ -869,7 +966,7 @@ int gnn_forward(fos_gnn* g, fos_ctx* c, const double* y, const double* v, double
   const int nC = c->nC;
   fos_launch(c, k_gnn_scale_part, kScaleBlocks, 256, nC, c->nF, y, v, (const double*)c->d_invV,
              (const float4*)c->d_faceNA32, g->scp);
-  fos_launch(c, k_gnn_scale_final, 1, 32, nC, c->nF, kScaleBlocks, (const float*)g->scp, g->sc);
+  fos_launch(c, k_gnn_scale_final, 1, 320, nC, c->nF, kScaleBlocks, (const float*)g->scp, g->sc);
   fos_launch(c, k_gnn_in, std::max(1, std::min(nblk(nC, 256), g->in_ctas)), 256, nC, y, v, (const double*)c->d_invV,
              (float)gamma, (float)c->gamm, (const float*)g->wb, (const GnnScales*)g->sc, train ? g->X0 : (float*)nullptr,
              g->h[0]);
@@ -879,7 +976,8 @@ int gnn_forward(fos_gnn* g, fos_ctx* c, const double* y, const double* v, double
     const int grid = std::max(1, std::min(ntiles, g->layer_ctas));
     auto kern = last ? k_gnn_layer<true> : k_gnn_layer<false>;
     fos_launch(c, kern, grid, kT, nC, c->nFi, (const int*)c->d_ell,
-               (const int2*)c->d_faceLR, (const float4*)c->d_faceNA32, (const GnnScales*)g->sc,
+               (const int2*)c->d_faceLR, (const float4*)c->d_faceNA32, (const int*)c->d_cnb,
+               (const float4*)c->d_cna32, (const GnnScales*)g->sc,
                (const float*)(g->wb + OFF_L0 + l * L_SIZE),
                (const unsigned short*)(g->Ab + l * H * 2 * H), (const unsigned short*)g->h[l],
                (last && !train) ? (unsigned short*)nullptr : g->h[l + 1],

@@ -101,3 +101,31 @@ def test_krylov_sums_both_shapes(cuda, cells, dims, precond):
     y, st = gpu_run(c, precond=precond, **kw)
     assert st["n_lin_iters"] > st["n_newton"]
     assert rel_err(y, y_ref) <= 1e-10
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (3, 3, 3), (4, 4, 4), (7, 6, 5)])
+def test_gnn_edges_from_slots_equal_edges_from_faces(cuda, dims):
+    """Tiles of 64 cells (partial, full, several) and chunks of 256: a context with the per-cell
+    copies of the face data gives the bits of one without, which is within 2e-2 of the
+    reference (BF16 roundings)."""
+    import torch
+    from fosolvers_gb300.learned import GNN
+    from oracle import gnn_ref as R
+    g = GNN(seed=2)
+    w = g.params()
+    w[R.OFF_D:R.OFF_DB] = 0.05 * np.random.default_rng(5).standard_normal(R.OFF_DB - R.OFF_D)
+    g.set_params(w)
+    z = []
+    for flags in (0, FLUX_FP32):
+        c = Case(with_all_conditions(box("tet", dims)), flags=flags)
+        y = perturbed(c.y0, c.nC, 6)
+        v = np.random.default_rng(6).standard_normal(c.N)
+        yi, vi, zi, zr = (torch.empty(c.N, dtype=torch.float64, device="cuda") for _ in range(4))
+        c.gpu.to_internal(torch.from_numpy(y).cuda(), yi)
+        c.gpu.to_internal(torch.from_numpy(v).cuda(), vi)
+        g.apply_dev(c.gpu, yi, vi, zi, 2e-3)
+        c.gpu.to_reference(zi, zr)
+        z.append(zr.cpu().numpy())
+    assert np.array_equal(z[0], z[1])
+    ref = R.forward(R.split(w), R.Graph(c.grid), y, v, 2e-3)
+    assert np.linalg.norm(z[0] - ref) <= 2e-2 * np.linalg.norm(ref - v)
