@@ -4,7 +4,9 @@
 // SPARSKIT's ilut (ITSOL/ilut.f:38-382) and applies it with lusol (:2272-2320).  Here the
 // same algorithm runs one warp per row:
 //
-//   factor  rows are claimed in increasing order from an atomic ticket.  A row's working
+//   factor  blocks of five consecutive rows are claimed in increasing order from an atomic
+//           ticket, a warp a row; the rows of a block hand over to one another in shared
+//           memory, the others through global memory.  A row's working
 //           copy (L part, U part, and a column -> position hash) lives in shared memory;
 //           its L entries are eliminated in increasing column order, each waiting (bounded
 //           spin) until the pivot row's own warp has published it.  A warp only waits on
@@ -13,7 +15,8 @@
 //           performs, in the same order, with the FMA contraction ilut does not have
 //           written out (__dmul_rn / __dsub_rn): given the same CSR the factors are
 //           bit-identical to SPARSKIT's.  Fill-in positions follow ilut's append order
-//           (ballot prefix counts), and the quick-split runs on one lane.
+//           (ballot prefix counts), and the quick-split is ilut's, swap for swap, run by the
+//           whole warp.
 //   solve   the forward and backward sweeps of lusol, groups of five rows claimed level by level
 //           of the graphs of groups, each unknown published by its own store and polled by
 //           the groups that read it; the row sums are fixed-order warp reductions.
