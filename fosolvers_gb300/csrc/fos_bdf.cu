@@ -414,7 +414,8 @@ struct Driver {
   }
   // k_final over wk.part into device out, and into host (page-locked) when given
   int reduce(int nv, double* out, double* host = nullptr, const int* flag = nullptr) {
-    fos_launch(c, k_final, nv, 256, nv, rblocks, wk.part, out, host, flag);
+    const int threads = std::min(256, (rblocks + 31) / 32 * 32);  // (idle warps would add zeros)
+    fos_launch(c, k_final, nv, threads, nv, rblocks, wk.part, out, host, flag);
     FOS_LAUNCH_CHECK();
     return 0;
   }
