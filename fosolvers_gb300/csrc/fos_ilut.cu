@@ -140,10 +140,14 @@ __device__ __forceinline__ bool wait_local(const int* flag, int* ctr, long spin)
   return false;
 }
 
-// |v| > t for t >= 0, by integer comparison (an FP64 one takes the FP64 pipe); false for NaN
+// |v| > t, by integer comparison (an FP64 one takes the FP64 pipe) where t is not negative: bits of
+// numbers without a sign order as the numbers do, and NaN's are above infinity's.  A t with its
+// sign bit set (a drop tolerance of -0.0, or below, which keeps every entry) or NaN takes the FP64
+// comparison.
 __device__ __forceinline__ bool abs_above(double v, double t) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-  return b <= 0x7ff0000000000000ull && b > (unsigned long long)__double_as_longlong(t);
+  const unsigned long long c = (unsigned long long)__double_as_longlong(t);
+  return c <= 0x7ff0000000000000ull ? b <= 0x7ff0000000000000ull && b > c : fabs(v) > t;
 }
 // |v| <= t; false for NaN
 __device__ __forceinline__ bool abs_within(double v, double t) {

@@ -1,0 +1,47 @@
+"""ILUT at the edges of its arguments: what ilut and lusol do there, the GPU class does too
+(factors bit for bit the oracle's, solves within 1e-12, as in the tests of ordinary arguments)."""
+import numpy as np
+import pytest
+
+from fosolvers_gb300 import mesh as M
+from fosolvers_gb300.euler import PREC_ILUT
+from helpers import Case, perturbed
+from oracle import pyoracle as O
+from test_gpu_ilut import assert_same_factors, gpu_ilu, oracle_ilut
+from test_oracle_kat import _random_csr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("droptol", [-0.0, -1e-6, -np.inf])
+@pytest.mark.parametrize("n,density,lfil", [(40, 0.15, 39), (200, 0.05, 10), (203, 0.3, 60)])
+def test_drop_tolerance_below_zero_keeps_every_entry(cuda, n, density, lfil, droptol):
+    """ilut drops |w| <= droptol |row| only, so nothing at a negative tolerance (zeros stored in
+    the matrix neither), and -0.0 is 0."""
+    _, a, ja, ia = _random_csr(n, density, n)
+    a[::7] = np.where(np.abs(a[::7]) < 2.0, 0.0, a[::7])  # stored zeros off the diagonal
+    ref = oracle_ilut(n, a, ja, ia, lfil, droptol)
+    assert len(ref[0]) > 3 * n  # (an empty U would leave about 2 n)
+    p = gpu_ilu(n, a, ja, ia, lfil, droptol)
+    assert_same_factors(p, ref)
+    if np.isfinite(droptol):
+        y = np.random.default_rng(n).normal(size=n)
+        xr = O.lusol(n, y, *ref)
+        assert np.abs(p.solve(y) - xr).max() <= 1e-12 * np.abs(xr).max()
+
+
+def test_context_drop_tolerance_of_minus_zero(cuda):
+    """A context accepts -0.0 (it is not below 0) and preconditions as with 0."""
+    m = M.box_mesh(4, 3, 5, jitter=0.1, seed=1, cells="tet")
+    wl = M.Workload("box", m, M.sine_state(m.centroids(), 1), np.zeros(0, np.int32),
+                    np.zeros(0, np.int32), np.zeros((0, 5)), order=2, dt=5e-4, nsteps=1)
+    c = Case(wl, flags=PREC_ILUT)
+    y = perturbed(c.y0, c.nC, 2)
+    r = np.random.default_rng(2).normal(size=c.N)
+    z = []
+    for droptol in (0.0, -0.0):
+        c.gpu.set_ilut(30, droptol)
+        assert c.gpu.pset(0.0, y, None, 0, 5e-3)[0] == 0
+        z.append(np.zeros_like(r))
+        assert c.gpu.psol(0.0, y, None, r, z[-1], 5e-3) == 0
+    assert np.array_equal(z[0], z[1])
