@@ -656,7 +656,9 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
                                                     int* __restrict__ ctr, long spin,
                                                     int withhold) {
   pdl_entry();
-  __shared__ double in_group[8][kGroup][kGroup];  // the entries between rows of the warp's group
+  // the entries between rows of the warp's group (kPending, no number that is stored: no entry; a
+  // stored zero counts, its product with an unknown that is not finite is a NaN)
+  __shared__ double in_group[8][kGroup][kGroup];
   const int lane = threadIdx.x & 31;
   double (*cg)[kGroup] = in_group[threadIdx.x >> 5];
   const size_t slot = (size_t)(lfil > 0 ? lfil : 1);
@@ -669,7 +671,8 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
     const int r0 = perm[t] * kGroup, nr = min(kGroup, n - r0);
     const double own = lane < nr ? rhs[r0 + lane] : 0.0;  // before the polls: its load overlaps them
     const double di = kBwd && lane < nr ? dinv[r0 + lane] : 1.0;
-    if (lane < kGroup * kGroup) cg[lane / kGroup][lane % kGroup] = 0.0;
+    if (lane < kGroup * kGroup)
+      cg[lane / kGroup][lane % kGroup] = __longlong_as_double((long long)kPending);
     __syncwarp();
     const int cl = lane < nr ? cnt[r0 + lane] : 0;
     const int longest = __reduce_max_sync(~0u, cl);
@@ -696,6 +699,7 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
           const int q = j[h][r];
           if (q >= r0 && q < r0 + nr) {
             cg[r][q - r0] = a[h][r];
+            a[h][r] = 0.0;
             j[h][r] = -1;
           }
           v[h][r] = j[h][r] >= 0 ? ld_poll(out + j[h][r]) : 0.0;
@@ -747,7 +751,7 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
       for (int q = 0; q < kGroup; q++)
         if (kBwd ? q > r : q < r) {
           const double e = cg[r][q];
-          if (__double_as_longlong(e) != 0) s = fma(-e, w[q], s);  // (no entry: w may be NaN)
+          if (!pending(e)) s = fma(-e, w[q], s);
         }
       w[r] = kBwd ? s * __shfl_sync(~0u, di, r) : s;
       if (!kBwd && r0 + r == withhold)  // (its readers in the group are left without it too)

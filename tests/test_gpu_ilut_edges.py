@@ -45,3 +45,31 @@ def test_context_drop_tolerance_of_minus_zero(cuda):
         z.append(np.zeros_like(r))
         assert c.gpu.psol(0.0, y, None, r, z[-1], 5e-3) == 0
     assert np.array_equal(z[0], z[1])
+
+
+@pytest.mark.parametrize("upper", [False, True], ids=["L", "U"])
+@pytest.mark.parametrize("entry,y11", [(0.0, np.inf), (0.0, np.nan), (np.inf, 12.0)])
+def test_factors_and_unknowns_that_are_not_finite(cuda, entry, y11, upper):
+    """A negative tolerance keeps zeros in the factors, and 0 x inf is a NaN in the rows that have
+    them, in lusol as here; an infinite entry makes its row infinite, not a NaN.  Rows depend on
+    the rows three away (mostly of their group of five) and seven away."""
+    n = 23
+    ia, ja, a = [1], [], []
+    for i in range(n):
+        cols = {i: 2.0}
+        for d in (3, 7):
+            j = i + d if upper else i - d
+            if 0 <= j < n:
+                cols[j] = entry if entry == 0.0 or j == 11 else 0.25
+        ja += [j + 1 for j in sorted(cols)]
+        a += [cols[j] for j in sorted(cols)]
+        ia.append(len(ja) + 1)
+    a, ja, ia = np.array(a), np.array(ja, np.int32), np.array(ia, np.int32)
+    ref = oracle_ilut(n, a, ja, ia, 5, -1.0)
+    p = gpu_ilu(n, a, ja, ia, 5, -1.0)
+    assert_same_factors(p, ref)
+    y = np.arange(1.0, n + 1)
+    y[11] = y11
+    xr = O.lusol(n, y, *ref)
+    assert (~np.isfinite(xr)).sum() > 3 and np.isfinite(xr).sum() > 3
+    np.testing.assert_allclose(p.solve(y), xr, rtol=1e-12)
