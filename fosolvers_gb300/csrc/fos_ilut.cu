@@ -771,7 +771,8 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
 template <bool kBwd>
 __global__ void __launch_bounds__(256) k_ilut_levels(int n, int lfil, const int* __restrict__ col,
                                                      const int* __restrict__ cnt, int* lev,
-                                                     int* __restrict__ ctr, long spin) {
+                                                     int* __restrict__ ctr, long spin,
+                                                     int withhold) {
   pdl_entry();
   const int lane = threadIdx.x & 31;
   const size_t slot = (size_t)(lfil > 0 ? lfil : 1);
@@ -826,7 +827,8 @@ __global__ void __launch_bounds__(256) k_ilut_levels(int n, int lfil, const int*
         for (int r = 0; r < kGroup; r++) mx = max(mx, v[h][r]);
     }
     mx = __reduce_max_sync(~0u, mx);
-    if (lane == 0) asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(lev + g), "r"(mx + 1) : "memory");
+    if (lane == 0 && (withhold < r0 || withhold >= r0 + nr))
+      asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(lev + g), "r"(mx + 1) : "memory");
   }
 }
 
@@ -923,7 +925,8 @@ static int solve_orders(fos_ilut* f, cudaStream_t s) {
     FOS_CUDA(cudaMemsetAsync(f->d_ctr, 0, 4 * sizeof(int), s));
     FOS_CUDA(cudaMemsetAsync(d_perm, 0, sizeof(int) * ng, s));  // the levels, for now
     kernel<<<grid_for((const void*)kernel, 256, 0, 8, std::min(ng, 2432)), 256, 0, s>>>(
-        n, f->lfil, d_col, d_cnt, d_perm, f->d_ctr, kSpinLimit);
+        n, f->lfil, d_col, d_cnt, d_perm, f->d_ctr, f->spin_limit > 0 ? f->spin_limit : kSpinLimit,
+        f->withhold);
     f->launches++;
     FOS_CUDA(cudaGetLastError());
     FOS_CUDA(cudaMemcpyAsync(lev.data(), d_perm, sizeof(int) * ng, cudaMemcpyDeviceToHost, s));
@@ -998,6 +1001,7 @@ int fos_ilut_factor_on(fos_ilut* f, const int* ia, const int* ja, const double* 
       return -1;
     }
   }
+  f->factored = false;  // until the factors and the sweeps' orders are complete
   for (;;) {
     const size_t row_smem = (size_t)56 * f->cap;
     if (kWarps * row_smem > (size_t)smem_max) {
@@ -1027,9 +1031,10 @@ int fos_ilut_factor_on(fos_ilut* f, const int* ia, const int* ja, const double* 
       f->cap *= 2;
       continue;
     }
-    f->factored = err == 0;
-    if (f->factored)
+    if (err == 0) {
       if (int rc = solve_orders(f, s)) return rc;
+      f->factored = true;
+    }
     if (err == kErrZeroRow) {
       fos_set_error("fos_ilut_factor_dev: zero row " + std::to_string(row + 1));
       return -5;

@@ -211,7 +211,8 @@ typedef struct fos_ilut fos_ilut;
  * lfil < 0 returns -4 (ilut's ierr) */
 int fos_ilut_create(fos_ilut** out, int n, int lfil);
 /* factor (factILU): returns 0, -5 on a zero row (ilut's ierr), -6 if a dependency wait ran
- * out, -1 on bad arguments.  Synchronises the stream. */
+ * out, -1 on bad arguments.  Synchronises the stream.  After a failure solves are refused (a
+ * malformed matrix, which is found first, leaves an earlier factorisation as it was). */
 int fos_ilut_factor_dev(fos_ilut* f, const int* ia, const int* ja, const double* a,
                         double droptol, void* stream);
 /* x = (LU)^{-1} y (solveILU / lusol), device vectors, x may equal y; asynchronous */
@@ -221,9 +222,10 @@ int fos_ilut_status(fos_ilut* f);
 /* Failure injection (tests of the bounded waits; no counterpart in the reference): every
  * dependency wait of the following factor and solve calls gives up after `polls` polls
  * (<= 0: the default 2^23), and row `withhold_row` (>= 0) is never published -- the factor
- * does not release it and the forward sweep does not store its unknown -- so every wait on
- * it runs out: fos_ilut_factor_dev returns -6 and a solve leaves fos_ilut_status at -6 with
- * NaN in the rows that waited.  withhold_row = -1 publishes every row again. */
+ * does not release it, the ordering of the sweeps does not store its level and the forward sweep
+ * not its unknown -- so every wait on it runs out: fos_ilut_factor_dev returns -6 (solves are then
+ * refused) and a solve leaves fos_ilut_status at -6 with NaN in the rows that waited.
+ * withhold_row = -1 publishes every row again. */
 int fos_ilut_set_wait_limit(fos_ilut* f, long polls, int withhold_row);
 /* the factors in ilut's MSR layout on the host (1-based values): alu(1:n) the inverted
  * diagonal, jlu(1:n+1) row pointers, ju(1:n) the start of each U row; returns the used

@@ -73,3 +73,35 @@ def test_factors_and_unknowns_that_are_not_finite(cuda, entry, y11, upper):
     xr = O.lusol(n, y, *ref)
     assert (~np.isfinite(xr)).sum() > 3 and np.isfinite(xr).sum() > 3
     np.testing.assert_allclose(p.solve(y), xr, rtol=1e-12)
+
+
+@pytest.mark.parametrize("first", [False, True], ids=["refactor", "first"])
+def test_solves_are_refused_after_the_ordering_ran_out(cuda, first):
+    """Upper triangular: no row waits in the factor, but the claim order of the backward sweep
+    waits for the level of a row that is withheld.  The factor call reports it and a solve has no
+    order to go by; published again, the same object factors and solves."""
+    n = 1000
+    ia = np.concatenate([[1], np.cumsum(np.minimum(n - np.arange(n), 7)) + 1]).astype(np.int32)
+    ja = np.concatenate([np.arange(i, min(n, i + 7)) + 1 for i in range(n)]).astype(np.int32)
+    a = np.random.default_rng(1).normal(size=len(ja))
+    a[ia[:-1] - 1] = 9.0
+    ref = oracle_ilut(n, a, ja, ia, 9, 0.0)
+    y = np.random.default_rng(2).normal(size=n)
+    xr = O.lusol(n, y, *ref)
+    import torch
+    from fosolvers_gb300.ilut import ILU
+    dev = lambda x, t: torch.from_numpy(np.ascontiguousarray(x, t)).cuda()
+    csr = (dev(ia - 1, np.int32), dev(ja - 1, np.int32), dev(a, np.float64))
+    p = ILU(n, 9)
+    if not first:
+        p.factor_csr(*csr, 0.0)
+        assert np.abs(p.solve(y) - xr).max() <= 1e-12 * np.abs(xr).max()
+    p.set_wait_limit(polls=4096, withhold_row=700)
+    with pytest.raises(RuntimeError, match="dependency wait ran out"):
+        p.factor_csr(*csr, 0.0)
+    with pytest.raises(RuntimeError, match="no factorisation"):
+        p.solve(y)
+    p.set_wait_limit(0, -1)
+    p.factor_csr(*csr, 0.0)
+    assert_same_factors(p, ref)
+    assert np.abs(p.solve(y) - xr).max() <= 1e-12 * np.abs(xr).max()
