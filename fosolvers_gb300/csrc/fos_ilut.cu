@@ -140,14 +140,20 @@ __device__ __forceinline__ bool wait_local(const int* flag, int* ctr, long spin)
   return false;
 }
 
-// |v| > t, by integer comparison (an FP64 one takes the FP64 pipe) where t is not negative: bits of
-// numbers without a sign order as the numbers do, and NaN's are above infinity's.  A t with its
-// sign bit set (a drop tolerance of -0.0, or below, which keeps every entry) or NaN takes the FP64
-// comparison.
-__device__ __forceinline__ bool abs_above(double v, double t) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-  const unsigned long long c = (unsigned long long)__double_as_longlong(t);
-  return c <= 0x7ff0000000000000ull ? b <= 0x7ff0000000000000ull && b > c : fabs(v) > t;
+// |v| > t by integer comparison (an FP64 one takes the FP64 pipe, and these stand on the chain of
+// rows): bits of numbers without a sign order as the numbers do, and a NaN's are above infinity's.
+// t as the bits to compare with: those of a negative t, which every |v| exceeds, are a negative
+// integer; -0.0 counts as 0, and nothing exceeds a NaN.
+__device__ __forceinline__ long long threshold_bits(double t) {
+  const long long c = __double_as_longlong(t), mag = c & 0x7fffffffffffffffll;
+  return mag > 0x7ff0000000000000ll ? LLONG_MAX : mag == 0 ? 0 : c;
+}
+__device__ __forceinline__ long long abs_bits(double v) {
+  return __double_as_longlong(v) & 0x7fffffffffffffffll;
+}
+__device__ __forceinline__ bool abs_above(double v, long long t) {
+  const long long b = abs_bits(v);
+  return b <= 0x7ff0000000000000ll && b > t;
 }
 // |v| <= t; false for NaN
 __device__ __forceinline__ bool abs_within(double v, double t) {
@@ -214,7 +220,8 @@ __device__ __forceinline__ void qsplit_tail(double* a, int* ind, int first, int 
     const double w0 = t0 <= m ? a[first + t0] : 0.0, w1 = t1 <= m ? a[first + t1] : 0.0;
     const int i0 = t0 <= m ? ind[first + t0] : 0, i1 = t1 <= m ? ind[first + t1] : 0;
     const int ikey = ind[first];
-    const bool g0 = t0 <= m && abs_above(w0, fabs(key)), g1 = t1 <= m && abs_above(w1, fabs(key));
+    const long long akey = abs_bits(key);
+    const bool g0 = t0 <= m && abs_above(w0, akey), g1 = t1 <= m && abs_above(w1, akey);
     const unsigned long long G = (unsigned long long)__ballot_sync(~0u, g0) |
                                  (unsigned long long)__ballot_sync(~0u, g1) << 32;  // bit t - 1
     const int larger = __popcll(G);
@@ -251,7 +258,7 @@ __device__ __forceinline__ void qsplit(double* a, int* ind, int n, int ncut, dou
     return;
   }
   for (;;) {
-    const double key = fabs(a[first]);
+    const long long key = abs_bits(a[first]);
     const int m = last - first;
     int larger = 0;
     for (int t0 = 1; t0 <= m; t0 += 32) {
@@ -355,7 +362,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) k_ilut_factor(
       ok = false;
     }
     tnorm = tnorm / (double)(j2 - j1);
-    const double thr = __dmul_rn(droptol, tnorm);
+    const long long thr = threshold_bits(__dmul_rn(droptol, tnorm));
     __syncwarp();
     if (ok) {
       // unpack: L in CSR order, U with the diagonal first, then CSR order
