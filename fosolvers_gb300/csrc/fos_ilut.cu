@@ -48,9 +48,10 @@ struct fos_ilut {
   int* d_levL = nullptr;   // level of every row in the L graph, published by the factor
   int* d_permF = nullptr;  // row groups by forward / backward level: the solves' claim order
   int* d_permB = nullptr;
-  int nlevF = 0, nlevB = 0;  // levels of the L and U graphs of rows (-1: not counted yet)
+  int nlevF = 0, nlevB = 0;  // levels of the L and U graphs of rows
   int ngF = 0, ngB = 0;      // and of the graphs of row groups
   int* d_ctr = nullptr;    // [0] factor ticket [1] forward [2] backward [3] error [4] error row
+                           // [5] malformed row [6] most levels
   int* h_ctr = nullptr;    // pinned copy
   int fepoch = 0;
   int cap = 256;           // working-row capacity (entries of L and of U)
@@ -77,9 +78,9 @@ constexpr int kWarps = 4;                 // the capacity limit is that of four 
 #endif
 constexpr int kMaxWarps = 16;             // rows of a CTA: FOS_ILUT_WARPS where they fit
 constexpr long kSpinLimit = 1L << 23;     // polls of a dependency flag before giving up
-__device__ __forceinline__ int ld_relaxed(const int* p) {
-  int v;
-  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ unsigned long long ld_level(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
 constexpr int kErrCapacity = -1, kErrZeroRow = -5, kErrTimeout = -6;
@@ -772,14 +773,18 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
 }
 
 // Levels of the graph of row groups: 1 + the largest level among the other groups that a group's
-// stored entries read (0: none yet, the value every level starts from).  The sweeps' own scheme
-// with integers: a warp per group, claimed in the natural order of the sweep, which every
-// dependency respects.  (From the columns on the host it took 8 ms for 100,800 rows.)
+// stored entries read.  The sweeps' own scheme with integers: a warp per group, claimed in the
+// natural order of the sweep, which every dependency respects; a row publishes one word (0: not
+// yet), its group's level in the low half and, for U, its own level in the graph of rows in the
+// high half.  top: the most levels of a row, of L from levL, where the factor kernel left them.
+// (From the columns on the host both U orders took 8 ms for 100,800 rows.)
 template <bool kBwd>
 __global__ void __launch_bounds__(256) k_ilut_levels(int n, int lfil, const int* __restrict__ col,
-                                                     const int* __restrict__ cnt, int* lev,
-                                                     int* __restrict__ ctr, long spin,
-                                                     int withhold) {
+                                                     const int* __restrict__ cnt,
+                                                     const int* __restrict__ levL,
+                                                     unsigned long long* pub, int* __restrict__ lev,
+                                                     int* __restrict__ top, int* __restrict__ ctr,
+                                                     long spin, int withhold) {
   pdl_entry();
   const int lane = threadIdx.x & 31;
   const size_t slot = (size_t)(lfil > 0 ? lfil : 1);
@@ -792,27 +797,38 @@ __global__ void __launch_bounds__(256) k_ilut_levels(int n, int lfil, const int*
     const int g = kBwd ? ng - 1 - t : t, r0 = g * kGroup, nr = min(kGroup, n - r0);
     const int cl = lane < nr ? cnt[r0 + lane] : 0;
     const int longest = __reduce_max_sync(~0u, cl);
-    int mx = 0;
+    int mx = 0, row[kGroup];
+    unsigned own[kGroup];  // the entries inside the group, a bit each
+#pragma unroll
+    for (int r = 0; r < kGroup; r++) row[r] = 0, own[r] = 0u;
     for (int k0 = 0; k0 < longest; k0 += 64) {
-      int j[2][kGroup], v[2][kGroup];
+      int j[2][kGroup];
+      unsigned long long v[2][kGroup];
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
         for (int r = 0; r < kGroup; r++) {
           const int k = k0 + 32 * h + lane;
           const bool in = r < nr && k < __shfl_sync(~0u, cl, r);
-          j[h][r] = in ? col[(size_t)(r0 + r) * slot + k] / kGroup : g;
+          j[h][r] = in ? col[(size_t)(r0 + r) * slot + k] : -1;
         }
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int r = 0; r < kGroup; r++) v[h][r] = j[h][r] != g ? ld_relaxed(lev + j[h][r]) : -1;
+        for (int r = 0; r < kGroup; r++) {
+          const int q = j[h][r];
+          if (q >= r0 && q < r0 + nr) {
+            own[r] |= 1u << (q - r0);
+            j[h][r] = -1;
+          }
+          v[h][r] = j[h][r] >= 0 ? ld_level(pub + j[h][r]) : 0ull;
+        }
       for (long it = 0;; it++) {
         bool wait = false;
 #pragma unroll
         for (int h = 0; h < 2; h++)
 #pragma unroll
-          for (int r = 0; r < kGroup; r++) wait |= v[h][r] == 0;
+          for (int r = 0; r < kGroup; r++) wait |= j[h][r] >= 0 && v[h][r] == 0ull;
         if (!__any_sync(~0u, wait)) break;
         if (it >= spin) {
           atomicCAS(ctr + 3, 0, kErrTimeout);
@@ -826,16 +842,44 @@ __global__ void __launch_bounds__(256) k_ilut_levels(int n, int lfil, const int*
         for (int h = 0; h < 2; h++)
 #pragma unroll
           for (int r = 0; r < kGroup; r++)
-            if (v[h][r] == 0) v[h][r] = ld_relaxed(lev + j[h][r]);
+            if (j[h][r] >= 0 && v[h][r] == 0ull) v[h][r] = ld_level(pub + j[h][r]);
       }
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int r = 0; r < kGroup; r++) mx = max(mx, v[h][r]);
+        for (int r = 0; r < kGroup; r++) {
+          mx = max(mx, (int)(unsigned)v[h][r]);
+          row[r] = max(row[r], (int)(v[h][r] >> 32));
+        }
     }
-    mx = __reduce_max_sync(~0u, mx);
-    if (lane == 0 && (withhold < r0 || withhold >= r0 + nr))
-      asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(lev + g), "r"(mx + 1) : "memory");
+    mx = __reduce_max_sync(~0u, mx) + 1;
+    int most;
+    if constexpr (kBwd) {
+#pragma unroll
+      for (int r = kGroup - 1; r >= 0; r--) {
+        const unsigned in = __reduce_or_sync(~0u, own[r]);
+        int l = __reduce_max_sync(~0u, row[r]);
+#pragma unroll
+        for (int q = r + 1; q < kGroup; q++)
+          if (in >> q & 1u) l = max(l, row[q]);
+        row[r] = l + 1;
+      }
+      most = row[0];
+#pragma unroll
+      for (int r = 1; r < kGroup; r++) most = max(most, row[r]);
+    } else {
+      most = __reduce_max_sync(~0u, lane < nr ? levL[r0 + lane] : 0);
+    }
+#pragma unroll
+    for (int r = 0; r < kGroup; r++)
+      if (lane == r && r < nr && r0 + r != withhold)
+        asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(pub + r0 + r),
+                     "l"((unsigned long long)(kBwd ? row[r] : 0) << 32 | (unsigned)mx)
+                     : "memory");
+    if (lane == 0) {
+      lev[g] = mx;
+      atomicMax(top, most);
+    }
   }
 }
 
@@ -928,16 +972,17 @@ extern "C" void fos_ilut_destroy(fos_ilut* f) { delete f; }
 static int solve_orders(fos_ilut* f, cudaStream_t s) {
   const int n = f->n, ng = (n + kGroup - 1) / kGroup;
   std::vector<int> lev(ng), perm(ng);
-  auto order = [&](auto kernel, const int* d_col, const int* d_cnt, int* d_perm, int* nlev) -> int {
-    FOS_CUDA(cudaMemsetAsync(f->d_ctr, 0, 4 * sizeof(int), s));
-    FOS_CUDA(cudaMemsetAsync(d_perm, 0, sizeof(int) * ng, s));  // the levels, for now
+  auto order = [&](auto kernel, const int* d_col, const int* d_cnt, int* d_perm, int* nlev,
+                   int* nlev_rows) -> int {
+    FOS_CUDA(cudaMemsetAsync(f->d_ctr, 0, 7 * sizeof(int), s));
+    FOS_CUDA(cudaMemsetAsync(f->d_z, 0, sizeof(double) * n, s));  // (refilled before every solve)
     kernel<<<grid_for((const void*)kernel, 256, 0, 8, std::min(ng, 2432)), 256, 0, s>>>(
-        n, f->lfil, d_col, d_cnt, d_perm, f->d_ctr, f->spin_limit > 0 ? f->spin_limit : kSpinLimit,
-        f->withhold);
+        n, f->lfil, d_col, d_cnt, f->d_levL, reinterpret_cast<unsigned long long*>(f->d_z), d_perm,
+        f->d_ctr + 6, f->d_ctr, f->spin_limit > 0 ? f->spin_limit : kSpinLimit, f->withhold);
     f->launches++;
     FOS_CUDA(cudaGetLastError());
     FOS_CUDA(cudaMemcpyAsync(lev.data(), d_perm, sizeof(int) * ng, cudaMemcpyDeviceToHost, s));
-    FOS_CUDA(cudaMemcpyAsync(f->h_ctr, f->d_ctr, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    FOS_CUDA(cudaMemcpyAsync(f->h_ctr, f->d_ctr, 7 * sizeof(int), cudaMemcpyDeviceToHost, s));
     FOS_CUDA(cudaStreamSynchronize(s));
     if (f->h_ctr[3]) {
       fos_set_error("fos_ilut_factor_dev: a dependency wait ran out");
@@ -951,39 +996,12 @@ static int solve_orders(fos_ilut* f, cudaStream_t s) {
     FOS_CUDA(cudaMemcpyAsync(d_perm, perm.data(), sizeof(int) * ng, cudaMemcpyHostToDevice, s));
     FOS_CUDA(cudaStreamSynchronize(s));
     *nlev = nl;
+    *nlev_rows = f->h_ctr[6];
     return 0;
   };
-  if (int rc = order(k_ilut_levels<false>, f->d_Lcol, f->d_Lcnt, f->d_permF, &f->ngF)) return rc;
-  f->nlevF = f->nlevB = -1;  // the rows' levels are counted when asked for
-  return order(k_ilut_levels<true>, f->d_Ucol, f->d_Ucnt, f->d_permB, &f->ngB);
-}
-
-// Levels of the graphs of rows (fos_ilut_info): L's from the factor kernel, U's from the stored
-// columns, fetched in chunks of rows from the bottom up so host memory stays small.
-static int count_levels(fos_ilut* f) {
-  const int n = f->n;
-  const size_t slot = (size_t)std::max(f->lfil, 1);
-  std::vector<int> lev(n);
-  FOS_CUDA(cudaMemcpy(lev.data(), f->d_levL, sizeof(int) * n, cudaMemcpyDeviceToHost));
-  f->nlevF = *std::max_element(lev.begin(), lev.end());
-  const int chunk = (int)std::max<size_t>(1, (size_t)(16u << 20) / (slot * sizeof(int)));
-  std::vector<int> cnt(chunk), col(slot * chunk);
-  int nu = 0;
-  for (int hi = n; hi > 0; hi -= chunk) {
-    const int lo = std::max(0, hi - chunk), m = hi - lo;
-    FOS_CUDA(cudaMemcpy(cnt.data(), f->d_Ucnt + lo, sizeof(int) * m, cudaMemcpyDeviceToHost));
-    FOS_CUDA(cudaMemcpy(col.data(), f->d_Ucol + slot * lo, sizeof(int) * slot * m,
-                        cudaMemcpyDeviceToHost));
-    for (int i = hi - 1; i >= lo; i--) {  // rows above i are final: U columns are > i
-      int mx = 0;
-      const int* c = col.data() + slot * (i - lo);
-      for (int k = 0; k < cnt[i - lo]; k++) mx = std::max(mx, lev[c[k]]);
-      lev[i] = mx + 1;
-      nu = std::max(nu, mx + 1);
-    }
-  }
-  f->nlevB = nu;
-  return 0;
+  if (int rc = order(k_ilut_levels<false>, f->d_Lcol, f->d_Lcnt, f->d_permF, &f->ngF, &f->nlevF))
+    return rc;
+  return order(k_ilut_levels<true>, f->d_Ucol, f->d_Ucnt, f->d_permB, &f->ngB, &f->nlevB);
 }
 
 int fos_ilut_factor_on(fos_ilut* f, const int* ia, const int* ja, const double* a,
@@ -1174,8 +1192,6 @@ extern "C" long fos_ilut_copy(const fos_ilut* f, double* alu, int* jlu, int* ju,
 
 extern "C" int fos_ilut_info(const fos_ilut* f, long* out) {
   if (!f || !out) return -1;
-  if (f->nlevF < 0)
-    if (int rc = count_levels(const_cast<fos_ilut*>(f))) return rc;
   out[0] = f->n;
   out[1] = f->lfil;
   out[2] = f->cap;

@@ -105,3 +105,33 @@ def test_solves_are_refused_after_the_ordering_ran_out(cuda, first):
     p.factor_csr(*csr, 0.0)
     assert_same_factors(p, ref)
     assert np.abs(p.solve(y) - xr).max() <= 1e-12 * np.abs(xr).max()
+
+
+@pytest.mark.parametrize("n,density", [(5, 0.3), (203, 0.02), (701, 0.01)])
+def test_levels_are_read_while_a_stream_is_captured(cuda, n, density):
+    """fos_ilut_info reads what the factor call left: the levels of the graphs of rows, equal to
+    those counted from the factors, also while a stream that waits for the default one is being
+    captured (when work on the default stream is an error and ends the capture)."""
+    import ctypes as C
+    from fosolvers_gb300 import _lib
+    rt = C.CDLL("libcudart.so.13")  # (the one that torch has loaded)
+    _, a, ja, ia = _random_csr(n, density, 3)
+    p = gpu_ilu(n, a, ja, ia, n, 0.0)
+    info = (C.c_long * 6)()
+    stream, graph = C.c_void_p(), C.c_void_p()
+    assert rt.cudaStreamCreate(C.byref(stream)) == 0
+    assert rt.cudaStreamBeginCapture(stream, 0) == 0
+    rc = _lib.lib().fos_ilut_info(p.handle, info)
+    ended = rt.cudaStreamEndCapture(stream, C.byref(graph))
+    rt.cudaGetLastError()
+    if ended == 0:
+        rt.cudaGraphDestroy(graph)
+    rt.cudaStreamDestroy(stream)
+    assert (rc, ended) == (0, 0)
+    _, jlu, ju = p.msr()
+    lo, up = np.zeros(n, int), np.zeros(n, int)
+    for i in range(n):
+        lo[i] = 1 + max([lo[c - 1] for c in jlu[jlu[i] - 1:ju[i] - 1]], default=0)
+    for i in reversed(range(n)):
+        up[i] = 1 + max([up[c - 1] for c in jlu[ju[i] - 1:jlu[i + 1] - 1]], default=0)
+    assert (info[4], info[5]) == (lo.max(), up.max())
