@@ -15,8 +15,7 @@
 // form, from per-cell FP32 (hi, lo) primitive pairs (k_prim_hl), and fuses the interior
 // faces into the cell gather (k_cell32: each interior face evaluated by both of its cells,
 // bit-identically); boundary faces go through k_bface32 (ghost state and flow in FP64,
-// stored as the difference from the cell's own flux).  Sums are in FP64, or in FP32 pairs
-// that are widened once (k_cell32), with the same results.
+// stored as the difference from the cell's own flux).  Sums are in FP64 in both variants.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -434,7 +433,7 @@ __device__ __forceinline__ void boundary_term(const double* __restrict__ Fb, int
 // face's own orientation (L = faceLR.x, R = faceLR.y) from the FP32 (hi, lo) means and
 // jumps, FP32 instructions only, so
 // the two cells of a face compute bit-identical (dF, dw) and the scheme stays exactly
-// conservative; the cell then sums -(dF - dw) (cell is L) or -(dF + dw) (cell is R) in
+// conservative; the cell then sums -(dF - dw) (cell is L) or -(dF + dw) (cell is R) in FP64, in
 // ascending ELL order.  Boundary faces read the FP64 differences k_bface32 wrote.
 // Each face is evaluated twice -- cheap FP32 arithmetic in exchange for the 2 x 48 B per face
 // a face-flow array costs in HBM traffic.  Cells that are not closed (Sc non-null: warped
@@ -463,29 +462,10 @@ __global__ void __launch_bounds__(kThreads) k_cell32(
   load_ell<kW>(cnb, c, nbr);  // the cells across the faces: no wait on the face arrays
   PHL P;
   load_hl(W, c, P);
-  // Accumulation in ELL order; the first face initialises the sums (every cell has at least
-  // one face, and ELL rows are padded at the end).  The terms come negated from the face
+  // FP64 accumulation in ELL order; the first face initialises the sums (every cell has at
+  // least one face, and ELL rows are padded at the end).  The terms come negated from the face
   // arithmetic (where negation is exact), so the sums are plain additions.
-  // The FP64 flux terms of kHyb are summed in FP64.  Without it every interior term is an FP32
-  // number, and the sum is carried as an FP32 pair (error-free TwoSum, its errors summed: about
-  // 48 bits, what the primitives carry; the sum of four such terms is nearly always exact in
-  // either) and widened once, before the boundary faces' FP64 terms and the closure term: 5 FP64
-  // additions a cell instead of 15, and half the widenings, on a kernel whose FP64 pipe was the
-  // bound (a Jv's 25 FP64 instructions took 79 of 109 us at 64^3 x 6: now 15).  The error against
-  // 64-bit values is that of the FP32 terms, the same as with FP64 sums.
   double acc[5];
-  int kb = kW;  // the first boundary face's slot
-  float as[5], ae[5];
-  auto add = [&](int q, bool first, float t) {
-    if (first) {
-      as[q] = t;
-      ae[q] = 0.0f;
-    } else {
-      const df2 r = df_two_sum(as[q], t);
-      as[q] = r.h;
-      ae[q] += r.l;
-    }
-  };
 #pragma unroll
   for (int k = 0; k < kW; k++) {
     if (k > 0 && e[k] < 0) continue;
@@ -541,42 +521,13 @@ __global__ void __launch_bounds__(kThreads) k_cell32(
                             -sw * (Q.s - P.s), P.s + Q.s, P.s * Q.s, na.x, na.y, na.z, na.w,
                             gm1, dF, dw);
 #pragma unroll
-        for (int q = 0; q < 5; q++) {
-          const float tq = fmaf(-sw, dw[q], -dF[q]);
-          if constexpr (kHyb) t[q] = f2d_bits(tq);
-          else add(q, k == 0, tq);
-        }
+        for (int q = 0; q < 5; q++) t[q] = f2d_bits(fmaf(-sw, dw[q], -dF[q]));
       }
-    } else if constexpr (kHyb) {
-      boundary_term(Fb, f, t);
     } else {
-      if (k == 0) {  // (a cell without interior faces)
-#pragma unroll
-        for (int q = 0; q < 5; q++) as[q] = ae[q] = 0.0f;
-      }
-      kb = min(kb, k);
+      boundary_term(Fb, f, t);
     }
-    if constexpr (kHyb) {
 #pragma unroll
-      for (int q = 0; q < 5; q++) acc[q] = k == 0 ? t[q] : acc[q] + t[q];
-    }
-  }
-  if constexpr (!kHyb) {
-#pragma unroll
-    for (int q = 0; q < 5; q++)  // (an infinite sum has no rounding error: TwoSum's is a NaN)
-      acc[q] = f2d_bits(as[q]) + f2d_bits(fabsf(as[q]) <= 3.402823466e38f ? ae[q] : 0.0f);
-    // the boundary faces come after the interior ones in ELL order (a loop of its own, so that
-    // cells without any do not issue its FP64 additions predicated off; inside the loop above
-    // they took the kernel from 64 registers to 71: Jv at 80^3 x 6 286 us, here 270)
-#pragma unroll 1
-    for (int k = kb; k < kW; k++) {
-      const int ek = __ldg(ell + (size_t)kW * c + k);
-      if (ek < 0) break;
-      double t[5];
-      boundary_term(Fb, ek >> 1, t);
-#pragma unroll
-      for (int q = 0; q < 5; q++) acc[q] += t[q];
-    }
+    for (int q = 0; q < 5; q++) acc[q] = k == 0 ? t[q] : acc[q] + t[q];
   }
   // own flux through the closure vector (kSc: the grid has cells whose faces do not close):
   // rho u.S, rho u u.S + p S, rho H u.S.  A compile-time switch: as a run-time branch the
