@@ -205,16 +205,28 @@ __device__ __forceinline__ bool finite_bits(double x) {
 // 1/a and 1/sqrt(a) in FP64: the special-function unit's approximation (about 20 bits, full
 // binary64 range, not an FP64-pipe instruction) and one step of Householder's cubically
 // convergent iteration, which takes the seed's error to about 2^-60, so the result carries
-// the rounding of its last operation.  Three and five FP64 instructions, where the division
-// and square root operators issue about ten each.  No special cases: a zero, infinite or
-// (after flushing) subnormal argument gives a non-finite result.
-__device__ __forceinline__ double rcp64(double a) {
+// the rounding of its last operation (the correctly rounded value or its neighbour): three and
+// five FP64 instructions.  For normal numbers whose reciprocals are normal; in the flux and its
+// Jacobian a zero or an infinity (a density, a squared speed of sound) ends in results that are
+// not finite whichever way it is divided by.
+__device__ __forceinline__ double rcp64_normal(double a) {
   double x;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
   const double e = fma(-a, x, 1.0);  // 1/a = x (1 + e + e^2 + ...)
   return fma(x, fma(e, e, e), x);
 }
-// also root = sqrt(a), from the same seed (one more instruction)
+// the same with 1/0, 1/inf and 1/NaN as the division has them (the seed itself, which takes
+// subnormal numbers for zeros): pivots, where an infinite one makes a row of zeros and spoils no
+// other.  Two selects (set-up and apply on 47x45x43 hexahedra 509 us with them and without; 523 with a branch
+// to the division)
+__device__ __forceinline__ double rcp64(double a) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  const double e = fma(-a, x, 1.0);
+  const double v = fma(x, fma(e, e, e), x);
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x00100000u >= 0x7fe00000u ? x : v;
+}
+// 1/sqrt(a), also root = sqrt(a), from the same seed (one more instruction)
 __device__ __forceinline__ double rsqrt64(double a, double& root) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
@@ -223,6 +235,18 @@ __device__ __forceinline__ double rsqrt64(double a, double& root) {
   const double q = e * fma(0.375, e, 0.5);
   root = fma(t, q, t);
   return fma(y, q, y);
+}
+
+// 1 / w correctly rounded, the division's bits.  For a reciprocal within one unit in the last place
+// (rcp64_normal) one step with two fused multiply-adds rounds correctly unless w's significand is all
+// ones (Markstein, IBM J. Res. Dev. 34, 1990): 5 dependent FP64 instructions of 64 clocks instead
+// of the operator's nine or more, on the chain of rows.  The other cases take the operator.
+__device__ __forceinline__ double recip_rn(double w) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(w);
+  const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+  if (e < 64u || e > 1982u || (b & 0xfffffffffffffull) == 0xfffffffffffffull) return 1.0 / w;
+  const double x = rcp64_normal(w);
+  return fma(fma(-w, x, 1.0), x, x);
 }
 
 // Sums of eight accumulators over a warp by halving what each lane holds: 9 FP64 additions per

@@ -162,18 +162,6 @@ __device__ __forceinline__ bool abs_within(double v, double t) {
   const unsigned long long c = (unsigned long long)__double_as_longlong(t);
   return c <= 0x7ff0000000000000ull ? b <= c : fabs(v) <= t;
 }
-// 1 / w correctly rounded, the division's bits.  For a reciprocal within one unit in the last place
-// (rcp64) one step with two fused multiply-adds rounds correctly unless w's significand is all
-// ones (Markstein, IBM J. Res. Dev. 34, 1990): 5 dependent FP64 instructions of 64 clocks instead
-// of the operator's nine or more, on the chain of rows.  The other cases take the operator.
-__device__ __forceinline__ double recip_rn(double w) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(w);
-  const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
-  if (e < 64u || e > 1982u || (b & 0xfffffffffffffull) == 0xfffffffffffffull) return 1.0 / w;
-  const double x = rcp64(w);
-  return fma(fma(-w, x, 1.0), x, x);
-}
-
 __device__ __forceinline__ void set_error(int* ctr, int code, int row) {
   if (atomicCAS(ctr + 3, 0, code) == 0) ctr[4] = row;
 }

@@ -150,7 +150,7 @@ __device__ __forceinline__ void jac_face_blocks(int f, int nFi, const double n[3
                                                 double g, const int* __restrict__ fslot,
                                                 double* __restrict__ J, double* __restrict__ Jb) {
   const double g1 = g - 1.0, h = 0.5 * aP;
-  const double wR = R.s * rcp64(L.s + R.s);
+  const double wR = R.s * rcp64_normal(L.s + R.s);
   double u[3], hn[3], g1n[3];
 #pragma unroll
   for (int i = 0; i < 3; i++) {

@@ -40,7 +40,7 @@ __device__ __forceinline__ void load_prim(const double* __restrict__ W, int c, P
 
 __device__ __forceinline__ void prim_from_cons(double rho, double mx, double my, double mz,
                                                double E, double gm1, P64& P) {
-  const double inv = rcp64(rho);
+  const double inv = rcp64_normal(rho);
   P.rho = rho;
   P.u = mx * inv; P.v = my * inv; P.w = mz * inv;
   P.p = gm1 * fma(-0.5, fma(mz, P.w, fma(my, P.v, mx * P.u)), E);
@@ -61,7 +61,7 @@ __device__ __forceinline__ void prim_from_cons(double rho, double mx, double my,
 // 317 us; the FP64 pipe is what bounds it before and after).
 __device__ __forceinline__ void roe_flow64(const P64& L, const P64& R, double nx, double ny,
                                            double nz, double aP, double gm1, double flow[5]) {
-  const double wR = R.s * rcp64(L.s + R.s);
+  const double wR = R.s * rcp64_normal(L.s + R.s);
   const double rJ = R.rho - L.rho, pJ = R.p - L.p, HJ = R.H - L.H;
   const double uJ = R.u - L.u, vJ = R.v - L.v, wJ = R.w - L.w;
   const double ua = fma(wR, uJ, L.u), va = fma(wR, vJ, L.v), wa = fma(wR, wJ, L.w);
