@@ -85,9 +85,22 @@ struct Coef {  // coefficients passed with the launch
   double c[kMaxVec];
 };
 
+// Blocks an SM that the Gram--Schmidt kernels have to leave room for.  With kRedBlocks blocks (kMany),
+// four an SM: four where two unknowns at a time fit 64 registers (up to 9 vectors), two up to the
+// longest basis, in the pass with both results (MODE 2) two up to 18.  Left to themselves they took
+// 74-80 registers with 6-8 vectors, so that three blocks an SM ran and the fourth alone, and
+// more than 128 from 17 on: the update of 11.8 M unknowns with 8, 20 and 31 vectors 264, 517 and 709
+// us, here 187, 417 and 679 (one unknown at a time 183, 508 and 700); of 1.3 M with 8 and 20 35 and
+// 71, here 27 and 57.  One block an SM (small vectors) has the registers to itself: bounds would cost
+// it up to a fifth (31 vectors, 311,000 unknowns: 22.8 -> 27.1 us).
+template <bool kMany>
+constexpr int gs_blocks(int nv, int mode = 1) {
+  return !kMany ? 1 : mode == 2 ? (nv <= 18 ? 2 : 1) : nv <= 9 ? 4 : 2;
+}
+
 // h[l] = V_l . w for l < NV (NV fixed at compile time: accumulators stay in registers)
-template <int NV>
-__global__ void __launch_bounds__(kT) k_mdot(long n, const double* __restrict__ V, long ldv,
+template <int NV, bool kMany>
+__global__ void __launch_bounds__(kT, gs_blocks<kMany>(NV)) k_mdot(long n, const double* __restrict__ V, long ldv,
                                              const double* __restrict__ w,
                                              double* __restrict__ part) {
   pdl_entry();
@@ -119,8 +132,8 @@ __global__ void __launch_bounds__(kT) k_mdot(long n, const double* __restrict__ 
 // coefficients come out of the same sweep over V).  s2 are the squared scales of
 // unnormalised basis vectors (v_l = s_l V_l), so h = V^T w gives the coefficients
 // of the projection onto the v_l.
-template <int NV, int MODE>
-__global__ void __launch_bounds__(kT) k_update(long n, const double* __restrict__ V, long ldv,
+template <int NV, int MODE, bool kMany>
+__global__ void __launch_bounds__(kT, gs_blocks<kMany>(NV, MODE)) k_update(long n, const double* __restrict__ V, long ldv,
                                                const double* __restrict__ h, const Coef s2,
                                                double* __restrict__ w,
                                                double* __restrict__ part) {
@@ -420,9 +433,12 @@ struct Driver {
     return 0;
   }
   int mdot(int nv, const double* V, long ldv, const double* w) {
+    const bool many = rblocks == kRedBlocks;
     switch (nv) {
 #define FOS_MDOT(K) \
-  case K: fos_launch(c, k_mdot<K>, rblocks, kT, wk.N, V, ldv, w, wk.part); break;
+  case K: \
+    fos_launch(c, many ? k_mdot<K, true> : k_mdot<K, false>, rblocks, kT, wk.N, V, ldv, w, wk.part); \
+    break;
       FOS_MDOT(1) FOS_MDOT(2) FOS_MDOT(3) FOS_MDOT(4) FOS_MDOT(5) FOS_MDOT(6) FOS_MDOT(7)
       FOS_MDOT(8) FOS_MDOT(9) FOS_MDOT(10) FOS_MDOT(11) FOS_MDOT(12) FOS_MDOT(13) FOS_MDOT(14)
       FOS_MDOT(15) FOS_MDOT(16) FOS_MDOT(17) FOS_MDOT(18) FOS_MDOT(19) FOS_MDOT(20) FOS_MDOT(21)
@@ -436,9 +452,13 @@ struct Driver {
   }
   template <int MODE>
   int update(int nv, const double* V, long ldv, const double* h, double* w, const Coef& s2) {
+    const bool many = rblocks == kRedBlocks;
     switch (nv) {
 #define FOS_UPD(K) \
-  case K: fos_launch(c, k_update<K, MODE>, rblocks, kT, wk.N, V, ldv, h, s2, w, wk.part); break;
+  case K: \
+    fos_launch(c, many ? k_update<K, MODE, true> : k_update<K, MODE, false>, rblocks, kT, wk.N, V, \
+               ldv, h, s2, w, wk.part); \
+    break;
       FOS_UPD(1) FOS_UPD(2) FOS_UPD(3) FOS_UPD(4) FOS_UPD(5) FOS_UPD(6) FOS_UPD(7) FOS_UPD(8)
       FOS_UPD(9) FOS_UPD(10) FOS_UPD(11) FOS_UPD(12) FOS_UPD(13) FOS_UPD(14) FOS_UPD(15)
       FOS_UPD(16) FOS_UPD(17) FOS_UPD(18) FOS_UPD(19) FOS_UPD(20) FOS_UPD(21) FOS_UPD(22)
