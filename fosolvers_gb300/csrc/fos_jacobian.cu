@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(32) k_pset32(
     __syncwarp();
     float Bv[25];
 #pragma unroll
-    for (int k = 0; k < 25; k++) Bv[k] = ops[o & 1][lane][((25 * op.y) & 3) + k];
+    for (int k = 0; k < 25; k++) Bv[k] = ops[o & 1][lane][(op.y & 3) + k];  // (25 y mod 4)
     __syncwarp();
     op_copy(LU, op2.y, ops[o & 1]);
     const int3 op3 = o + 3 < no ? upd[o0 + o + 3] : none;
