@@ -100,9 +100,9 @@ constexpr int gs_blocks(int nv, int mode = 1) {
 
 // h[l] = V_l . w for l < NV (NV fixed at compile time: accumulators stay in registers)
 template <int NV, bool kMany>
-__global__ void __launch_bounds__(kT, gs_blocks<kMany>(NV)) k_mdot(long n, const double* __restrict__ V, long ldv,
-                                             const double* __restrict__ w,
-                                             double* __restrict__ part) {
+__global__ void __launch_bounds__(kT, gs_blocks<kMany>(NV)) k_mdot(
+    long n, const double* __restrict__ V, long ldv, const double* __restrict__ w,
+    double* __restrict__ part) {
   pdl_entry();
   double acc[NV];
 #pragma unroll
@@ -127,21 +127,19 @@ __global__ void __launch_bounds__(kT, gs_blocks<kMany>(NV)) k_mdot(long n, const
   block_reduce_store<NV>(acc, part);
 }
 
-// w -= sum_l h[l] s2[l] V_l ; then part <- V_l . w (MODE 0, CGS2 second pass), ||w||^2
-// (MODE 1), or both (MODE 2: the DGKS test and, when it fails, the second pass's
-// coefficients come out of the same sweep over V).  s2 are the squared scales of
-// unnormalised basis vectors (v_l = s_l V_l), so h = V^T w gives the coefficients
-// of the projection onto the v_l.
+// w -= sum_l h[l] s2[l] V_l ; then part <- ||w||^2 (MODE 1), or V_l . w and ||w||^2 (MODE 2:
+// the DGKS test and, when it fails, the second pass's coefficients come out of the same sweep
+// over V).  s2 are the squared scales of unnormalised basis vectors (v_l = s_l V_l), so
+// h = V^T w gives the coefficients of the projection onto the v_l.
 template <int NV, int MODE, bool kMany>
-__global__ void __launch_bounds__(kT, gs_blocks<kMany>(NV, MODE)) k_update(long n, const double* __restrict__ V, long ldv,
-                                               const double* __restrict__ h, const Coef s2,
-                                               double* __restrict__ w,
-                                               double* __restrict__ part) {
+__global__ void __launch_bounds__(kT, gs_blocks<kMany>(NV, MODE)) k_update(
+    long n, const double* __restrict__ V, long ldv, const double* __restrict__ h, const Coef s2,
+    double* __restrict__ w, double* __restrict__ part) {
   pdl_entry();
   __shared__ double hs[NV];
   if (threadIdx.x < NV) hs[threadIdx.x] = h[threadIdx.x] * s2.c[threadIdx.x];
   __syncthreads();
-  constexpr int NA = MODE == 0 ? NV : MODE == 1 ? 1 : NV + 1;
+  constexpr int NA = MODE == 1 ? 1 : NV + 1;
   double acc[NA];
 #pragma unroll
   for (int l = 0; l < NA; l++) acc[l] = 0.0;
@@ -165,7 +163,7 @@ __global__ void __launch_bounds__(kT, gs_blocks<kMany>(NV, MODE)) k_update(long 
 #pragma unroll
         for (int l = 0; l < NV; l++) acc[l] += vv[u][l] * wi[u];
       }
-      if (MODE != 0) acc[NA - 1] += wi[u] * wi[u];
+      acc[NA - 1] += wi[u] * wi[u];
     }
   }
   block_reduce_store<NA>(acc, part);
@@ -416,14 +414,17 @@ struct Driver {
   // thread, beyond that kRedBlocks.  With the large shape everywhere a thread of a small grid
   // summed one element and the block's trees were the rest (184,320 unknowns, 15 vectors: 34 us a
   // multi-dot, 10 us this way; 22 us with 128 threads and one unknown at a time, which leaves
-  // too few loads in flight).  Not with the FP32 flux: there a sum in another order moves the
+  // too few loads in flight).  Measured either side of the line with 15 vectors, one block an SM
+  // against kRedBlocks: 311,000 unknowns 14 and 18 us, 700,000 25 and 28, 1.3 M 53 and 46: they cross
+  // near a million, and the line lies at the smaller size because moving it would change the
+  // order of the sums in between.  Not with the FP32 flux: there a sum in another order moves the
   // state by an FP64 rounding and some face's FP32 terms by theirs, which is seen at 1e-9 of a
   // step's result, so its sums keep their order at every size.
   int rblocks = kRedBlocks;
   void set_shape() {
-    const long few = 152L * kT * 8;
+    const long few = (long)c->sm_count * kT * 8;
     if (wk.N <= few && !(c->flags & FOS_FLUX_FP32))
-      rblocks = (int)std::min<long>(152, (wk.N + kT - 1) / kT);
+      rblocks = (int)std::min<long>(c->sm_count, (wk.N + kT - 1) / kT);
   }
   // k_final over wk.part into device out, and into host (page-locked) when given
   int reduce(int nv, double* out, double* host = nullptr, const int* flag = nullptr) {

@@ -200,6 +200,7 @@ extern "C" int fos_ctx_create(fos_ctx** out, int nC, int nE, int nPi, int nPb, c
   c->gamm = gamm; c->r = r; c->nBC = nBC; c->maxP = maxP;
   c->nFi = nPi; c->nFb = nPb; c->nF = nP;
   cudaGetDevice(&c->device);
+  cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
 
   // ---- renumbering
   std::vector<int> xadj(nC + 1, 0), adj(2 * (size_t)nPi);

@@ -76,7 +76,7 @@ constexpr int kWarps = 4;                 // the capacity limit is that of four 
 #ifndef FOS_ILUT_WARPS
 #define FOS_ILUT_WARPS 5
 #endif
-constexpr int kMaxWarps = 16;             // rows of a CTA: FOS_ILUT_WARPS where they fit
+constexpr int kMaxWarps = FOS_ILUT_WARPS;  // rows of a CTA where they fit
 constexpr long kSpinLimit = 1L << 23;     // polls of a dependency flag before giving up
 __device__ __forceinline__ unsigned long long ld_level(const unsigned long long* p) {
   unsigned long long v;

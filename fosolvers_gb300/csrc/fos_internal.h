@@ -200,7 +200,6 @@ inline void fos_launch(fos_ctx* c, void (*k)(KArgs...), dim3 g, dim3 b, Args... 
 int fos_residual_launch(fos_ctx* c, const double* y, const double* v, const double* d_s,
                         const double* fy, double* out, double a, double b, int mode);
 int fos_norm2_dev(fos_ctx* c, const double* x, long n, double* d_out_sq);
-int fos_sum_partials(fos_ctx* c, int np, double* d_out);  // sum of c->d_red[0..np) in order
 int fos_permute(fos_ctx* c, const double* in, double* out, int dir);
 // plane q (0..4) only: out + q nC from in + q nC
 int fos_permute_plane(fos_ctx* c, const double* in, double* out, int dir, int q);
@@ -227,8 +226,8 @@ int fos_jac_assemble(fos_ctx* c, const double* y);
 bool fos_pset_is_fused(const fos_ctx* c);
 int fos_pset_fused(fos_ctx* c, const double* y, double gamma);
 int fos_ilu_factor(fos_ctx* c, double gamma);
-// z = P^-1 r; with d_zsq also ||z||^2 from the same pass over z: into d_zsq (device; *np = 0), or
-// left as *np partial sums in d_red
+// z = P^-1 r; with d_zsq and np also ||z||^2: from the same pass over z as *np partial sums in d_red,
+// or (ILUT, *np = 0) in d_zsq (device)
 int fos_ilu_apply(fos_ctx* c, const double* r, double* z, double* d_zsq = nullptr,
                   int* np = nullptr);
 // fos_ilut.cu: the Euler preconditioner with ILUT (FOS_PREC_ILUT)

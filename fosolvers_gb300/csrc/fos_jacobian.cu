@@ -1412,9 +1412,6 @@ int fos_jac_setup(fos_ctx* c) {
     if (up(&c->d_pnbL, nbL) || up(&c->d_pnbU, nbU)) return -100;
   }
   if (c->ilu_colors) {
-    int sms = 0;
-    FOS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-    c->sm_count = sms;
     for (int mode : {kSwFwd, kSwTop, kSwBwd})
       FOS_CUDA(cudaFuncSetAttribute(sweep_kernel(c->ilu_nbw, mode),
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
@@ -1601,8 +1598,9 @@ static int ilu_apply_t(fos_ctx* c, const TF* LU, const double* r, double* z, dou
       }
     const int n = c->lev_f[l + 1] - c->lev_f[l];
     const int* rows = c->d_lrows_f ? c->d_lrows_f + c->lev_f[l] : nullptr;
-    auto k = top ? (c->ilu_nbw == 4 ? k_ilu_fwd<TF, true, 4> : k_ilu_fwd<TF, true, 8>)
-                 : (c->ilu_nbw == 4 ? k_ilu_fwd<TF, false, 4> : k_ilu_fwd<TF, false, 8>);
+    auto k = c->ilu_nbw == 4 ? k_ilu_fwd<TF, false, 4> : k_ilu_fwd<TF, false, 8>;
+    if constexpr (sizeof(TF) == 8)  // (only colours have a fused top level)
+      if (top) k = c->ilu_nbw == 4 ? k_ilu_fwd<TF, true, 4> : k_ilu_fwd<TF, true, 8>;
     fos_launch(c, k, nb_rows5(n), kT, n, rows, c->lev_f[l], (const int*)c->d_pnbL,
                (const int*)c->d_plst, (const int*)c->d_pdu, LU, yv, zv);
   }
@@ -1626,11 +1624,8 @@ static int ilu_apply_t(fos_ctx* c, const TF* LU, const double* r, double* z, dou
     fos_launch(c, k_ilu_out_sq<TF>, blocks, kRedThreads, c->nC, (const int*)c->d_ipos,
                (const TF*)zv, z, c->d_red);
     FOS_LAUNCH_CHECK();
-    if (np) {
-      *np = blocks;
-      return 0;
-    }
-    return fos_sum_partials(c, blocks, d_zsq);
+    *np = blocks;
+    return 0;
   }
   fos_launch(c, k_ilu_out<TF>, nb(c->nC, 256), 256, c->nC, (const int*)c->d_ipos,
              (const TF*)zv, z);

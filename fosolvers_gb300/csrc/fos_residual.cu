@@ -723,12 +723,6 @@ int fos_norm2_dev(fos_ctx* c, const double* x, long n, double* d_out_sq) {
   return 0;
 }
 
-int fos_sum_partials(fos_ctx* c, int np, double* d_out) {
-  fos_launch(c, k_sum_final, 1, sum_threads(np), (const double*)c->d_red, np, d_out);
-  FOS_LAUNCH_CHECK();
-  return 0;
-}
-
 int fos_jv_sigma(fos_ctx* c, double* d_scal, int np, double ynorm, double eps, double b) {
   fos_launch(c, k_sigma, 1, sum_threads(np), d_scal, (const double*)c->d_red, np, ynorm, eps, b);
   FOS_LAUNCH_CHECK();
