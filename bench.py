@@ -49,13 +49,13 @@ GNN_BYTES_PER_CELL = 120 + 216 + 3 * 368 + 208
 # the operation's kernels, L2 flushed before every kernel, so an upper bound); traffic
 # grows with the cell count, so the full-size figure is this times nC.  Summary and
 # command: profiles/traffic_sine64_fp32.md
-TRAFFIC_FP32_BYTES_PER_CELL = {"residual": 236.7, "jv": 405.5,
-                               "ilu_apply": 764.5, "gnn_apply": 1263.5}
+TRAFFIC_FP32_BYTES_PER_CELL = {"residual": 237.0, "jv": 406.0,
+                               "ilu_apply": 764.8, "gnn_apply": 1268.2}
 # FP64-pipe lane-instructions per cell of the FP32 form's residual (k_prim_hl<0> +
 # k_cell32 residual epilogue) and Jv (k_prim_hl<1> + k_cell32 Jv epilogue), counted by ncu
 # (sm__inst_executed_pipe_fp64 x 32 / cells; profiles/fp64_pipe_sine64.md).  GB300 retires
 # 2 FP64 lanes per clock per SM, so these put a second roof under the operations, beside HBM.
-FP64_INSTR_PER_CELL_FP32 = {"residual": 12.8, "jv": 22.8}
+FP64_INSTR_PER_CELL_FP32 = {"residual": 20.0, "jv": 30.0}
 
 
 def parse():

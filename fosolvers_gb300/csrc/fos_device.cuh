@@ -237,18 +237,6 @@ __device__ __forceinline__ double rsqrt64(double a, double& root) {
   return fma(y, q, y);
 }
 
-// 1 / w correctly rounded, the division's bits.  For a reciprocal within one unit in the last place
-// (rcp64_normal) one step with two fused multiply-adds rounds correctly unless w's significand is all
-// ones (Markstein, IBM J. Res. Dev. 34, 1990): 5 dependent FP64 instructions of 64 clocks instead
-// of the operator's nine or more, on the chain of rows.  The other cases take the operator.
-__device__ __forceinline__ double recip_rn(double w) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(w);
-  const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
-  if (e < 64u || e > 1982u || (b & 0xfffffffffffffull) == 0xfffffffffffffull) return 1.0 / w;
-  const double x = rcp64_normal(w);
-  return fma(fma(-w, x, 1.0), x, x);
-}
-
 // Sums of eight accumulators over a warp by halving what each lane holds: 9 FP64 additions per
 // lane where eight butterflies take 40 (an FP64 instruction holds its quarter of an SM for 64
 // clocks, so on small grids the trees were most of a dot product).  Lane l then has sum l / 4.

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kT) k_jac_face(int nFi, int nF, int nC, const 
 // FP32 form: FP32 arithmetic from the per-cell primitives (double-float, rounded to FP32) and
 // the FP32 face geometry, so no FP64 instruction runs on interior faces (the FP32
 // preconditioner is assembled and stored in FP32).  A cell is one 32-byte sector: the
-// residual's 64-byte (hi, lo) pairs made a gather two sectors of which a fifth is used here.
+// residual's 48-byte (hi, lo) pairs make a gather two sectors of which a fifth is used here.
 __device__ __forceinline__ PrimT<float> load_prim_f32(const float* __restrict__ Wj, int c) {
   const float4* w4 = reinterpret_cast<const float4*>(Wj + 8 * (size_t)c);
   const float4 a = __ldg(w4);
@@ -641,8 +641,8 @@ __global__ void __launch_bounds__(kT) k_ilu_factor(
 //      then the Gauss--Jordan inverse of the diagonal block, left where the operands were;
 //   C. the warp stores its 32 rows one after another, each as its two contiguous ranges (L
 //      blocks, then inverted diagonal and U blocks).
-// What bounds it is latency at few resident warps (two on a scheduler, a third of the issue
-// slots used, DRAM 33-58% busy); what is left out is load/store and address work.  An operand
+// What bounds it is latency at few resident warps (nine blocks an SM, 37% of the issue slots used and
+// DRAM 37% busy in the largest colour); what is left out is load/store and address work.  An operand
 // block is 100 bytes at a 4-byte alignment: read by each lane with 25 loads it cost 25 x 32
 // cache lookups per operation, so the warp copies the aligned 16-byte pieces that hold it, eight
 // lanes to a block.  Staging in the stored order takes the transposition and its divisions
@@ -980,8 +980,8 @@ __global__ void __launch_bounds__(kT) k_ilu_bwd(int n, const int* __restrict__ r
 // memory, two tiles in flight, and a lane reads its row's blocks from there: the factor is
 // streamed once, at full width, and marked evict-first so that the vectors the rows gather
 // from stay in the L2.  The gathers of a tile (the neighbours' finished rows, one 32-byte sector
-// each) are issued while the tile before it is computed.  DRAM bounds it (80-85% busy in the
-// large levels).  The five-lanes-per-row kernels above ask the L1 for 20 bytes at a time (88%
+// each) are issued while the tile before it is computed.  DRAM bounds it (79% of peak in the
+// largest level).  The five-lanes-per-row kernels above ask the L1 for 20 bytes at a time (88%
 // busy, DRAM at 68%); they remain for level sets, whose rows are scattered, and for FP64 factors,
 // where seven 200-byte blocks a row leave two such warps on an SM and half of its FP64 units
 // idle (hexahedra 47x45x43: 88 us in the sweeps against 51).  A lane forms the row's five sums

@@ -268,7 +268,8 @@ gather_fn gather_kernel(int ell_w, int ek) {
 // double-float arithmetic (df_*: FP32 pipe); only the Jv perturbation y + s v is FP64.
 // Layout: 12 floats (48 B) per cell = (rho, u, v, w, H, p) hi, (rho, u, v, w, H, p) lo.  sqrt(rho)
 // is formed by whoever loads the cell: a fourth 16-byte load per neighbour cost more on a kernel
-// whose L1 is 76% busy than ten FP32 instructions (FP32 Jv at 80^3 x 6 tetrahedra: 293 -> 268 us).
+// whose L1 is 76% busy than ten FP32 instructions (FP32 Jv at 80^3 x 6 tetrahedra: 293 -> 268
+// us when it was measured, 283 now).
 // kV: the state is y + s v (a Jv), else y; a compile-time switch, so a residual issues no
 // predicated-off FP64 FMAs.  kJac: for the Jacobian, which reads the pairs' FP32 sums only:
 // 8 floats (32 B, one sector) per cell = (u, v, w, H, sqrt(rho), 0, 0, 0)

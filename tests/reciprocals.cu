@@ -8,8 +8,7 @@ __global__ void k_recips(long n, const double* __restrict__ x, double* __restric
   out[i] = rcp64(x[i]);
   out[n + i] = rsqrt64(x[i], root);
   out[2 * n + i] = root;
-  out[3 * n + i] = recip_rn(x[i]);
-  out[4 * n + i] = rcp64_normal(x[i]);
+  out[3 * n + i] = rcp64_normal(x[i]);
 }
 
 extern "C" int recips(long n, const double* x, double* out) {
