@@ -1025,8 +1025,9 @@ int fos_ilut_factor_on(fos_ilut* f, const int* ia, const int* ja, const double* 
     }
     const int rows = (int)std::min<size_t>(FOS_ILUT_WARPS, ((size_t)smem_max - 1024) / row_smem);
     const size_t smem = rows * row_smem;
+    // (the same value for every object and capacity: another thread may set it before this launch)
     FOS_CUDA(cudaFuncSetAttribute(k_ilut_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
+                                  smem_max - 1024));
     FOS_CUDA(cudaMemsetAsync(f->d_ctr, 0, 5 * sizeof(int), s));
     f->fepoch++;
     const int grid = grid_for((const void*)k_ilut_factor, 32 * rows, smem, rows, f->n);

@@ -135,3 +135,38 @@ def test_levels_are_read_while_a_stream_is_captured(cuda, n, density):
     for i in reversed(range(n)):
         up[i] = 1 + max([up[c - 1] for c in jlu[ju[i] - 1:jlu[i + 1] - 1]], default=0)
     assert (info[4], info[5]) == (lo.max(), up.max())
+
+
+def test_two_threads_with_rows_of_different_lengths(cuda):
+    """Factorisations of short and of long rows (working capacities of 256 and 1024 entries, so
+    launches with different amounts of shared memory) by two threads at a time, each on a stream
+    of its own: every one succeeds, with the oracle's factors."""
+    import threading
+    import torch
+    from fosolvers_gb300.ilut import ILU
+    errors = []
+
+    def work(n, dense, rounds):
+        try:
+            A = np.diag(4.0 + np.arange(n) % 3).astype(float)
+            A[:dense] += 0.01 * (1.0 + np.arange(n) % 7)
+            a, ja = A[A != 0], np.nonzero(A)[1].astype(np.int32)
+            ia = np.concatenate([[0], np.cumsum((A != 0).sum(1))]).astype(np.int32)
+            ref = oracle_ilut(n, a, ja + 1, ia + 1, n, 0.0)
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                csr = tuple(torch.from_numpy(x).cuda() for x in (ia, ja, a))
+                stream.synchronize()
+                for _ in range(rounds):
+                    p = ILU(n, n)
+                    p.factor_csr(*csr, 0.0, stream=stream)
+                assert_same_factors(p, ref)
+        except Exception as e:  # reported by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in ((40, 2, 400), (700, 2, 60))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
