@@ -143,27 +143,31 @@ __device__ __forceinline__ void jac_block64(const double A[25], const double hn[
 // off-diagonal blocks of an interior face, or the boundary pair's diagonal term.  The FP64 pipe
 // bounds it, so the half area h is folded into the normal and the wave weights, |A~| (anfj's
 // decomposition) is built with one FMA per rank-1 term, and each block adds its side's eulerNFJ
-// to it with two: about 240 FP64 instructions a face instead of 370.  Set-up and one apply on
-// 47x45x43 hexahedra, with the diagonal kernel and the Gauss--Jordan step below: 625 -> 524 us.
+// to it with two: about 250 FP64 instructions a face instead of 370.  Set-up and one apply on
+// 47x45x43 hexahedra, with the diagonal kernel and the Gauss--Jordan step below: 625 -> 510 us.
+// Against quad arithmetic a block's mean error is 2-12% above that of |A~| and F' formed apart and
+// scaled at the end (1.34e-16 and 1.26e-16 on smooth states), and below it on neighbours that
+// differ by 10^6, because the averages are quotients of sums.
 __device__ __forceinline__ void jac_face_blocks(int f, int nFi, const double n[3], double aP,
                                                 const PrimT<double>& L, const PrimT<double>& R,
                                                 double g, const int* __restrict__ fslot,
                                                 double* __restrict__ J, double* __restrict__ Jb) {
   const double g1 = g - 1.0, h = 0.5 * aP;
-  const double wR = R.s * rcp64_normal(L.s + R.s);
+  const double inv = rcp64_normal(L.s + R.s);
   double u[3], hn[3], g1n[3];
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    u[i] = fma(wR, R.u[i] - L.u[i], L.u[i]);
+    u[i] = fma(R.s, R.u[i], L.s * L.u[i]) * inv;
     hn[i] = h * n[i];
     g1n[i] = g1 * hn[i];
   }
-  const double H = fma(wR, R.H - L.H, L.H);
+  const double H = fma(R.s, R.H, L.s * L.H) * inv;
   const double hq = 0.5 * fma(u[2], u[2], fma(u[1], u[1], u[0] * u[0]));
   const double vn = fma(u[2], n[2], fma(u[1], n[1], u[0] * n[0]));
   double c;
-  const double ic = rsqrt64(g1 * (H - hq), c);
-  const double av = fabs(vn), hav = h * av, k = 0.5 * h * ic * ic;
+  const double c2 = g1 * (H - hq);
+  (void)rsqrt64(c2, c);
+  const double av = fabs(vn), hav = h * av, k = (0.5 * h) * rcp64_normal(c2);
   const double wm = k * (fabs(vn - c) - av), wp = k * (fabs(vn + c) - av);
   const double g1q = g1 * hq, cv = c * vn;
   double lm[5], lp[5], cn[3], A[25];
