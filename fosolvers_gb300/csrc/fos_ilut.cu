@@ -51,7 +51,7 @@ struct fos_ilut {
   int nlevF = 0, nlevB = 0;  // levels of the L and U graphs of rows
   int ngF = 0, ngB = 0;      // and of the graphs of row groups
   int* d_ctr = nullptr;    // [0] factor ticket [1] forward [2] backward [3] error [4] error row
-                           // [5] malformed row [6] most levels
+                           // [5] malformed row [6] most levels [7] groups done
   int* h_ctr = nullptr;    // pinned copy
   int fepoch = 0;
   int cap = 256;           // working-row capacity (entries of L and of U)
@@ -78,12 +78,17 @@ constexpr int kWarps = 4;                 // the capacity limit is that of four 
 #endif
 constexpr int kMaxWarps = FOS_ILUT_WARPS;  // rows of a CTA where they fit
 constexpr long kSpinLimit = 1L << 23;     // polls of a dependency flag before giving up
+__device__ __forceinline__ unsigned long long timer_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
 __device__ __forceinline__ unsigned long long ld_level(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-constexpr int kErrCapacity = -1, kErrZeroRow = -5, kErrTimeout = -6;
+constexpr int kErrCapacity = -1, kErrZeroRow = -5, kErrTimeout = -6, kErrSlow = -7;
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
   int v;
@@ -766,15 +771,21 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
 // natural order of the sweep, which every dependency respects; a row publishes one word (0: not
 // yet), its group's level in the low half and, for U, its own level in the graph of rows in the
 // high half.  top: the most levels of a row, of L from levL, where the factor kernel left them.
-// (From the columns on the host both U orders took 8 ms for 100,800 rows.)
+// A link of the chain of groups takes 0.5-0.75 us here, and 100,800 rows of the Euler P 0.6 ms for both
+// orders, 8 ms from the columns on the host; but 20,000 groups that are one chain take 15 ms, on
+// the host 1.7.  So the kernel has the time that the host would take (budget_ns): beyond it, or when
+// the groups done after a quarter of it foretell that, the warps leave (kErrSlow) and the host
+// counts.
 template <bool kBwd>
 __global__ void __launch_bounds__(256) k_ilut_levels(int n, int lfil, const int* __restrict__ col,
                                                      const int* __restrict__ cnt,
                                                      const int* __restrict__ levL,
                                                      unsigned long long* pub, int* __restrict__ lev,
                                                      int* __restrict__ top, int* __restrict__ ctr,
-                                                     long spin, int withhold) {
+                                                     long spin, int withhold,
+                                                     unsigned long long budget_ns) {
   pdl_entry();
+  const unsigned long long t0 = timer_ns();
   const int lane = threadIdx.x & 31;
   const size_t slot = (size_t)(lfil > 0 ? lfil : 1);
   const int ng = (n + kGroup - 1) / kGroup;
@@ -821,10 +832,13 @@ __global__ void __launch_bounds__(256) k_ilut_levels(int n, int lfil, const int*
         if (!__any_sync(~0u, wait)) break;
         if (it >= spin) {
           atomicCAS(ctr + 3, 0, kErrTimeout);
-          break;
+          return;
         }
         if ((it & 63) == 63) {
-          if (__any_sync(~0u, *(volatile int*)(ctr + 3) == kErrTimeout)) break;
+          const unsigned long long t = timer_ns() - t0, done = *(volatile unsigned*)(ctr + 7);
+          if (__any_sync(~0u, t > budget_ns / 4 && t * ng > budget_ns * done))
+            atomicCAS(ctr + 3, 0, kErrSlow);
+          if (__any_sync(~0u, *(volatile int*)(ctr + 3) != 0)) return;
           __nanosleep(32);
         }
 #pragma unroll
@@ -868,6 +882,7 @@ __global__ void __launch_bounds__(256) k_ilut_levels(int n, int lfil, const int*
     if (lane == 0) {
       lev[g] = mx;
       atomicMax(top, most);
+      atomicAdd(ctr + 7, 1);
     }
   }
 }
@@ -957,23 +972,62 @@ extern "C" int fos_ilut_create(fos_ilut** out, int n, int lfil) {
 
 extern "C" void fos_ilut_destroy(fos_ilut* f) { delete f; }
 
+// The levels of k_ilut_levels on the host, from the stored columns (fetched in chunks of rows in the
+// sweep's order, so host memory stays small): lev by group, *most of the rows (of U; L's are levL's).
+static int levels_on_host(fos_ilut* f, bool bwd, const int* d_col, const int* d_cnt, int* lev,
+                          int* most, cudaStream_t s) {
+  const int n = f->n;
+  const size_t slot = (size_t)std::max(f->lfil, 1);
+  std::fill(lev, lev + (n + kGroup - 1) / kGroup, 1);
+  std::vector<int> row(n, 1);
+  if (!bwd)
+    FOS_CUDA(cudaMemcpyAsync(row.data(), f->d_levL, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
+  const int chunk = (int)std::min<size_t>(n, std::max<size_t>(1, (size_t)(16u << 20) / (slot * sizeof(int))));
+  std::vector<int> cnt(chunk), col(slot * chunk);
+  for (int done = 0; done < n; done += chunk) {
+    const int m = std::min(chunk, n - done), lo = bwd ? n - done - m : done;
+    FOS_CUDA(cudaMemcpyAsync(cnt.data(), d_cnt + lo, sizeof(int) * m, cudaMemcpyDeviceToHost, s));
+    FOS_CUDA(cudaMemcpyAsync(col.data(), d_col + slot * lo, sizeof(int) * slot * m,
+                             cudaMemcpyDeviceToHost, s));
+    FOS_CUDA(cudaStreamSynchronize(s));
+    for (int k = 0; k < m; k++) {  // the rows that row i reads are final
+      const int i = bwd ? lo + m - 1 - k : lo + k, g = i / kGroup;
+      const int* c = col.data() + slot * (i - lo);
+      for (int e = 0; e < cnt[i - lo]; e++) {
+        const int q = c[e] / kGroup;
+        if (q != g) lev[g] = std::max(lev[g], lev[q] + 1);
+        if (bwd) row[i] = std::max(row[i], row[c[e]] + 1);
+      }
+    }
+  }
+  *most = *std::max_element(row.begin(), row.end());
+  return 0;
+}
+
 // Claim orders of the two sweeps: groups of kGroup rows sorted (stably) by their level.
 static int solve_orders(fos_ilut* f, cudaStream_t s) {
   const int n = f->n, ng = (n + kGroup - 1) / kGroup;
   std::vector<int> lev(ng), perm(ng);
+  // what the host takes for an order: 100,000 rows of 8 slots 1.7 ms, 14,000 of 50 1.5.  (A row that
+  // is withheld is waited for until the limit on the polls.)
+  const unsigned long long host_ns = 50000ull + 5ull * n + 2ull * n * std::max(f->lfil, 1);
+  const unsigned long long budget = f->withhold >= 0 ? ~0ull : host_ns;
   auto order = [&](auto kernel, const int* d_col, const int* d_cnt, int* d_perm, int* nlev,
                    int* nlev_rows) -> int {
-    FOS_CUDA(cudaMemsetAsync(f->d_ctr, 0, 7 * sizeof(int), s));
+    FOS_CUDA(cudaMemsetAsync(f->d_ctr, 0, 8 * sizeof(int), s));
     FOS_CUDA(cudaMemsetAsync(f->d_z, 0, sizeof(double) * n, s));  // (refilled before every solve)
     kernel<<<grid_for((const void*)kernel, 256, 0, 8, std::min(ng, 2432)), 256, 0, s>>>(
         n, f->lfil, d_col, d_cnt, f->d_levL, reinterpret_cast<unsigned long long*>(f->d_z), d_perm,
-        f->d_ctr + 6, f->d_ctr, f->spin_limit > 0 ? f->spin_limit : kSpinLimit, f->withhold);
+        f->d_ctr + 6, f->d_ctr, f->spin_limit > 0 ? f->spin_limit : kSpinLimit, f->withhold, budget);
     f->launches++;
     FOS_CUDA(cudaGetLastError());
     FOS_CUDA(cudaMemcpyAsync(lev.data(), d_perm, sizeof(int) * ng, cudaMemcpyDeviceToHost, s));
     FOS_CUDA(cudaMemcpyAsync(f->h_ctr, f->d_ctr, 7 * sizeof(int), cudaMemcpyDeviceToHost, s));
     FOS_CUDA(cudaStreamSynchronize(s));
-    if (f->h_ctr[3]) {
+    if (f->h_ctr[3] == kErrSlow) {
+      if (int rc = levels_on_host(f, d_perm == f->d_permB, d_col, d_cnt, lev.data(), f->h_ctr + 6, s))
+        return rc;
+    } else if (f->h_ctr[3]) {
       fos_set_error("fos_ilut_factor_dev: a dependency wait ran out");
       return -6;
     }

@@ -170,3 +170,33 @@ def test_two_threads_with_rows_of_different_lengths(cuda):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("below,above", [(0, 7), (7, 0), (1, 1), (3, 4)])
+@pytest.mark.parametrize("n,lfil", [(40003, 8), (40003, 40)])
+def test_orders_of_chains(cuda, n, lfil, below, above):
+    """Bands: every row depends on the one next to it, so the graphs are chains, whose levels the
+    host counts where that is faster (the narrow storage) and the device elsewhere."""
+    import ctypes as C
+    from fosolvers_gb300 import _lib
+    d = np.arange(-below, above + 1)
+    ja = np.arange(n)[:, None] + d
+    inside = (ja >= 0) & (ja < n)
+    a = np.where(d == 0, 9.0, np.random.default_rng(n).uniform(-1.0, 1.0, ja.shape))[inside]
+    ia = np.concatenate([[1], 1 + np.cumsum(inside.sum(1))]).astype(np.int32)
+    ja = ja[inside].astype(np.int32) + 1
+    ref = oracle_ilut(n, a, ja, ia, lfil, 1e-3)
+    p = gpu_ilu(n, a, ja, ia, lfil, 1e-3)
+    assert_same_factors(p, ref)
+    _, jlu, ju = (x.tolist() for x in ref)
+    lo, up = [0] * (n + 1), [0] * (n + 1)
+    for i in range(n):
+        lo[i + 1] = 1 + max([lo[c] for c in jlu[jlu[i] - 1:ju[i] - 1]], default=0)
+    for i in reversed(range(n)):
+        up[i + 1] = 1 + max([up[c] for c in jlu[ju[i] - 1:jlu[i + 1] - 1]], default=0)
+    info = (C.c_long * 6)()
+    assert _lib.lib().fos_ilut_info(p.handle, info) == 0
+    assert (info[4], info[5]) == (max(lo), max(up))
+    y = np.random.default_rng(1).normal(size=n)
+    xr = O.lusol(n, y, *ref)
+    assert np.abs(p.solve(y) - xr).max() <= 1e-12 * np.abs(xr).max()
