@@ -17,8 +17,8 @@
 //           bit-identical to SPARSKIT's.  Fill-in positions follow ilut's append order
 //           (ballot prefix counts), and the quick-split is ilut's, swap for swap, run by the
 //           whole warp.
-//   solve   the forward and backward sweeps of lusol, groups of five rows claimed level by level
-//           of the graphs of groups, each unknown published by its own store and polled by
+//   solve   the forward and backward sweeps of lusol, groups of five rows or single rows claimed
+//           level by level of their graph, each unknown published by its own store and polled by
 //           the groups that read it; the row sums are fixed-order warp reductions.
 //
 // Storage: every row owns lfil slots for L and lfil for U (ilut keeps at most lfil L and
@@ -46,12 +46,14 @@ struct fos_ilut {
   int* d_done = nullptr;   // factor: epoch of the factorisation that published the row
   double* d_z = nullptr;   // forward-sweep result (kPending before each solve)
   int* d_levL = nullptr;   // level of every row in the L graph, published by the factor
-  int* d_permF = nullptr;  // row groups by forward / backward level: the solves' claim order
+  int* d_permF = nullptr;  // row groups or rows by forward / backward level: the solves' claim order
   int* d_permB = nullptr;
   int nlevF = 0, nlevB = 0;  // levels of the L and U graphs of rows
-  int ngF = 0, ngB = 0;      // and of the graphs of row groups
+  int perF = 0, perB = 0;    // rows that a warp of the forward / backward sweep takes at a time
+  int swF = 0, swB = 0;      // and levels of the graph of these
   int* d_ctr = nullptr;    // [0] factor ticket [1] forward [2] backward [3] error [4] error row
-                           // [5] malformed row [6] most levels [7] groups done
+                           // [5] malformed row [6] most levels [7] groups done [8] most levels in
+                           // the stored columns
   int* h_ctr = nullptr;    // pinned copy
   int fepoch = 0;
   int cap = 256;           // working-row capacity (entries of L and of U)
@@ -88,6 +90,7 @@ __device__ __forceinline__ unsigned long long ld_level(const unsigned long long*
   asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
+constexpr int kCtr = 9;                   // words of d_ctr
 constexpr int kErrCapacity = -1, kErrZeroRow = -5, kErrTimeout = -6, kErrSlow = -7;
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
@@ -632,7 +635,7 @@ __global__ void k_fill_pending(long n, double* __restrict__ x) {
   if (i < n) x[i] = __longlong_as_double((long long)kPending);
 }
 
-// One sweep of lusol, a warp per group of kGroup consecutive rows:
+// One sweep of lusol, a warp per group of kG consecutive rows (kGroup, or 1: see one_at_a_time):
 //   forward (ilut.f:2300-2305):  z_i = y_i - sum_k L_ik z_k into z (kPending on entry), and x_i set
 //     to kPending for the backward sweep (x may be y: a group reads its own y_i only)
 //   backward (:2309-2315):       x_i = dinv_i (z_i - sum_k U_ik x_k) into x (kPending on entry)
@@ -642,13 +645,13 @@ __global__ void k_fill_pending(long n, double* __restrict__ x) {
 // go over the entries of all rows of the group at once, all loads in flight together; entries
 // inside the group are set aside and solved in registers afterwards.  What bounds a sweep is the
 // chain of dependencies, and the unknowns of one cell are a chain of five: a row at a time each
-// link took an L2 round trip, its polls and a five-step sum (2.1 us); now the five cost one
-// (both sweeps of 100,800 rows: 17.5 ms before, 4.0 now).  A wait that ran out makes the row NaN, so
+// link took an L2 round trip, its polls and a five-step sum (2.1 us; 0.75 now, with kG = 1); in
+// groups the five cost 2.2 (both sweeps of 100,800 rows of the Euler P: 17.5 ms before, 4.0 now).  A wait that ran out makes the row NaN, so
 // the failure reaches callers that only look at the result (the Krylov driver's non-finite checks)
 // as well as fos_ilut_status.
 constexpr int kGroup = 5;
 
-template <bool kBwd>
+template <bool kBwd, int kG>
 __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* __restrict__ col,
                                                     const double* __restrict__ val,
                                                     const int* __restrict__ cnt,
@@ -660,35 +663,36 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
   pdl_entry();
   // the entries between rows of the warp's group (kPending, no number that is stored: no entry; a
   // stored zero counts, its product with an unknown that is not finite is a NaN)
-  __shared__ double in_group[8][kGroup][kGroup];
+  __shared__ double in_group[8][kG][kG];
   const int lane = threadIdx.x & 31;
-  double (*cg)[kGroup] = in_group[threadIdx.x >> 5];
+  double (*cg)[kG] = in_group[threadIdx.x >> 5];
   const size_t slot = (size_t)(lfil > 0 ? lfil : 1);
-  const int ng = (n + kGroup - 1) / kGroup;
+  const int ng = (n + kG - 1) / kG;
   for (;;) {
     int t = 0;
     if (lane == 0) t = atomicAdd(ctr + (kBwd ? 2 : 1), 1);
     t = __shfl_sync(~0u, t, 0);
     if (t >= ng) return;
-    const int r0 = perm[t] * kGroup, nr = min(kGroup, n - r0);
+    const int r0 = perm[t] * kG, nr = min(kG, n - r0);
     const double own = lane < nr ? rhs[r0 + lane] : 0.0;  // before the polls: its load overlaps them
     const double di = kBwd && lane < nr ? dinv[r0 + lane] : 1.0;
-    if (lane < kGroup * kGroup)
-      cg[lane / kGroup][lane % kGroup] = __longlong_as_double((long long)kPending);
+    if (lane < kG * kG)
+      cg[lane / kG][lane % kG] = __longlong_as_double((long long)kPending);
     __syncwarp();
     const int cl = lane < nr ? cnt[r0 + lane] : 0;
     const int longest = __reduce_max_sync(~0u, cl);
-    double acc[8];
+    constexpr int kAcc = kG == 1 ? 1 : 8;
+    double acc[kAcc];
 #pragma unroll
-    for (int r = 0; r < 8; r++) acc[r] = 0.0;
+    for (int r = 0; r < kAcc; r++) acc[r] = 0.0;
     bool ok = true;
     for (int k0 = 0; k0 < longest; k0 += 64) {
-      int j[2][kGroup];
-      double a[2][kGroup], v[2][kGroup];
+      int j[2][kG];
+      double a[2][kG], v[2][kG];
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int r = 0; r < kGroup; r++) {
+        for (int r = 0; r < kG; r++) {
           const int k = k0 + 32 * h + lane;
           const bool in = r < nr && k < __shfl_sync(~0u, cl, r);
           j[h][r] = in ? col[(size_t)(r0 + r) * slot + k] : -1;
@@ -697,7 +701,7 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int r = 0; r < kGroup; r++) {
+        for (int r = 0; r < kG; r++) {
           const int q = j[h][r];
           if (q >= r0 && q < r0 + nr) {
             cg[r][q - r0] = a[h][r];
@@ -714,7 +718,7 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
 #pragma unroll
         for (int h = 0; h < 2; h++)
 #pragma unroll
-          for (int r = 0; r < kGroup; r++) wait |= pending(v[h][r]);
+          for (int r = 0; r < kG; r++) wait |= pending(v[h][r]);
         if (!__any_sync(~0u, wait)) break;
         if (it >= spin) {
           atomicCAS(ctr + 3, 0, kErrTimeout);
@@ -728,29 +732,36 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
 #pragma unroll
         for (int h = 0; h < 2; h++)
 #pragma unroll
-          for (int r = 0; r < kGroup; r++)
+          for (int r = 0; r < kG; r++)
             if (pending(v[h][r])) v[h][r] = ld_poll(out + j[h][r]);
       }
       if (!ok) break;
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int r = 0; r < kGroup; r++) acc[r] = fma(a[h][r], v[h][r], acc[r]);
+        for (int r = 0; r < kG; r++) acc[r] = fma(a[h][r], v[h][r], acc[r]);
     }
     if (!ok) {
 #pragma unroll
-      for (int r = 0; r < kGroup; r++) acc[r] = __longlong_as_double(0x7ff8000000000000ll);
+      for (int r = 0; r < kG; r++) acc[r] = __longlong_as_double(0x7ff8000000000000ll);
     }
-    const double sums = warp_sum8(acc, lane);
+    double sums;  // row r's in lane 4 r
+    if constexpr (kG == 1) {
+      sums = acc[0];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sums += __shfl_xor_sync(~0u, sums, o);
+    } else {
+      sums = warp_sum8(acc, lane);
+    }
     __syncwarp();
     // the group's own triangle, by every lane
-    double w[kGroup];
+    double w[kG];
 #pragma unroll
-    for (int i = 0; i < kGroup; i++) {
-      const int r = kBwd ? kGroup - 1 - i : i;
+    for (int i = 0; i < kG; i++) {
+      const int r = kBwd ? kG - 1 - i : i;
       double s = __shfl_sync(~0u, own, r) - __shfl_sync(~0u, sums, 4 * r);
 #pragma unroll
-      for (int q = 0; q < kGroup; q++)
+      for (int q = 0; q < kG; q++)
         if (kBwd ? q > r : q < r) {
           const double e = cg[r][q];
           if (!pending(e)) s = fma(-e, w[q], s);
@@ -769,8 +780,9 @@ __global__ void __launch_bounds__(256) k_ilut_sweep(int n, int lfil, const int* 
 // Levels of the graph of row groups: 1 + the largest level among the other groups that a group's
 // stored entries read.  The sweeps' own scheme with integers: a warp per group, claimed in the
 // natural order of the sweep, which every dependency respects; a row publishes one word (0: not
-// yet), its group's level in the low half and, for U, its own level in the graph of rows in the
-// high half.  top: the most levels of a row, of L from levL, where the factor kernel left them.
+// yet), its group's level in the low half and its own level in the graph of rows in the high half.
+// ctr[8]: the most levels of a row; ctr[6]: the same, for L of levL, where the factor kernel counted the
+// multipliers that the quick-split dropped too.
 // A link of the chain of groups takes 0.5-0.75 us here, and 100,800 rows of the Euler P 0.6 ms for both
 // orders, 8 ms from the columns on the host; but 20,000 groups that are one chain take 15 ms, on
 // the host 1.7.  So the kernel has the time that the host would take (budget_ns): beyond it, or when
@@ -781,8 +793,7 @@ __global__ void __launch_bounds__(256) k_ilut_levels(int n, int lfil, const int*
                                                      const int* __restrict__ cnt,
                                                      const int* __restrict__ levL,
                                                      unsigned long long* pub, int* __restrict__ lev,
-                                                     int* __restrict__ top, int* __restrict__ ctr,
-                                                     long spin, int withhold,
+                                                     int* __restrict__ ctr, long spin, int withhold,
                                                      unsigned long long budget_ns) {
   pdl_entry();
   const unsigned long long t0 = timer_ns();
@@ -856,32 +867,30 @@ __global__ void __launch_bounds__(256) k_ilut_levels(int n, int lfil, const int*
         }
     }
     mx = __reduce_max_sync(~0u, mx) + 1;
-    int most;
-    if constexpr (kBwd) {
 #pragma unroll
-      for (int r = kGroup - 1; r >= 0; r--) {
-        const unsigned in = __reduce_or_sync(~0u, own[r]);
-        int l = __reduce_max_sync(~0u, row[r]);
+    for (int i = 0; i < kGroup; i++) {
+      const int r = kBwd ? kGroup - 1 - i : i;
+      const unsigned in = __reduce_or_sync(~0u, own[r]);
+      int l = __reduce_max_sync(~0u, row[r]);
 #pragma unroll
-        for (int q = r + 1; q < kGroup; q++)
-          if (in >> q & 1u) l = max(l, row[q]);
-        row[r] = l + 1;
-      }
-      most = row[0];
-#pragma unroll
-      for (int r = 1; r < kGroup; r++) most = max(most, row[r]);
-    } else {
-      most = __reduce_max_sync(~0u, lane < nr ? levL[r0 + lane] : 0);
+      for (int q = 0; q < kGroup; q++)
+        if ((kBwd ? q > r : q < r) && (in >> q & 1u)) l = max(l, row[q]);
+      row[r] = l + 1;
     }
+    int rows = row[0];
+#pragma unroll
+    for (int r = 1; r < kGroup; r++) rows = max(rows, row[r]);  // (1 for a row past the end)
+    const int most = kBwd ? rows : __reduce_max_sync(~0u, lane < nr ? levL[r0 + lane] : 0);
 #pragma unroll
     for (int r = 0; r < kGroup; r++)
       if (lane == r && r < nr && r0 + r != withhold)
         asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(pub + r0 + r),
-                     "l"((unsigned long long)(kBwd ? row[r] : 0) << 32 | (unsigned)mx)
+                     "l"((unsigned long long)row[r] << 32 | (unsigned)mx)
                      : "memory");
     if (lane == 0) {
       lev[g] = mx;
-      atomicMax(top, most);
+      atomicMax(ctr + 6, most);
+      atomicMax(ctr + 8, rows);
       atomicAdd(ctr + 7, 1);
     }
   }
@@ -951,8 +960,8 @@ extern "C" int fos_ilut_create(fos_ilut** out, int n, int lfil) {
   rc = rc ? rc : alloc(&f->d_levL, n);
   rc = rc ? rc : alloc(&f->d_permF, n);
   rc = rc ? rc : alloc(&f->d_permB, n);
-  rc = rc ? rc : alloc(&f->d_ctr, 8);
-  if (!rc && cudaMallocHost((void**)&f->h_ctr, 8 * sizeof(int)) != cudaSuccess) {
+  rc = rc ? rc : alloc(&f->d_ctr, kCtr);
+  if (!rc && cudaMallocHost((void**)&f->h_ctr, kCtr * sizeof(int)) != cudaSuccess) {
     fos_set_error("fos_ilut_create: cudaMallocHost failed");
     rc = -100;
   }
@@ -973,15 +982,19 @@ extern "C" int fos_ilut_create(fos_ilut** out, int n, int lfil) {
 extern "C" void fos_ilut_destroy(fos_ilut* f) { delete f; }
 
 // The levels of k_ilut_levels on the host, from the stored columns (fetched in chunks of rows in the
-// sweep's order, so host memory stays small): lev by group, *most of the rows (of U; L's are levL's).
+// sweep's order, so host memory stays small): lev by group, row by row, *most as in ctr[6].
 static int levels_on_host(fos_ilut* f, bool bwd, const int* d_col, const int* d_cnt, int* lev,
-                          int* most, cudaStream_t s) {
+                          std::vector<int>& row, int* most, cudaStream_t s) {
   const int n = f->n;
   const size_t slot = (size_t)std::max(f->lfil, 1);
   std::fill(lev, lev + (n + kGroup - 1) / kGroup, 1);
-  std::vector<int> row(n, 1);
-  if (!bwd)
+  if (!bwd) {
+    row.resize(n);
     FOS_CUDA(cudaMemcpyAsync(row.data(), f->d_levL, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
+    FOS_CUDA(cudaStreamSynchronize(s));
+    *most = *std::max_element(row.begin(), row.end());
+  }
+  row.assign(n, 1);
   const int chunk = (int)std::min<size_t>(n, std::max<size_t>(1, (size_t)(16u << 20) / (slot * sizeof(int))));
   std::vector<int> cnt(chunk), col(slot * chunk);
   for (int done = 0; done < n; done += chunk) {
@@ -996,55 +1009,84 @@ static int levels_on_host(fos_ilut* f, bool bwd, const int* d_col, const int* d_
       for (int e = 0; e < cnt[i - lo]; e++) {
         const int q = c[e] / kGroup;
         if (q != g) lev[g] = std::max(lev[g], lev[q] + 1);
-        if (bwd) row[i] = std::max(row[i], row[c[e]] + 1);
+        row[i] = std::max(row[i], row[c[e]] + 1);
       }
     }
   }
-  *most = *std::max_element(row.begin(), row.end());
+  if (bwd) *most = *std::max_element(row.begin(), row.end());
   return 0;
 }
 
-// Claim orders of the two sweeps: groups of kGroup rows sorted (stably) by their level.
+// Whether a sweep takes its rows one at a time: by what the two take, from the levels of their graphs.
+// A chain of 20,000 rows (4,000 groups) takes 30.0 ms with rows and 17.3 with groups, both sweeps, so a
+// level of rows costs 0.75 us and one of groups 2.2; and every row that is claimed 0.6 ns more than
+// its share of a group (50,000 rows of a diagonal: 92 and 50 us).  Groups win where the rows of a
+// group hang together (the unknowns of a cell), rows where a group waits for the latest of rows that
+// do not: 27x28x29 cells of a 7-point stencil with 5 entries a row have 274 and 219 levels of rows
+// and 3,150 of groups, 0.45 and 13.7 ms; with 700 and 3,330 1.2 and 14.7; 150x151 cells of a 5-point
+// one with 900 and 330 1.32 and 1.46, with 2,000 and 625 3.3 and 2.6.
+static bool one_at_a_time(int n, int rows, int groups) {
+  return 0.77 * rows + 6.2e-4 * n < 2.2 * groups + 0.5;
+}
+
+// Claim orders of the two sweeps: groups of kGroup rows, or rows, sorted (stably) by their level.
 static int solve_orders(fos_ilut* f, cudaStream_t s) {
   const int n = f->n, ng = (n + kGroup - 1) / kGroup;
-  std::vector<int> lev(ng), perm(ng);
+  std::vector<int> lev, row, perm;
+  std::vector<unsigned long long> pub;
   // what the host takes for an order: 100,000 rows of 8 slots 1.7 ms, 14,000 of 50 1.5.  (A row that
   // is withheld is waited for until the limit on the polls.)
   const unsigned long long host_ns = 50000ull + 5ull * n + 2ull * n * std::max(f->lfil, 1);
   const unsigned long long budget = f->withhold >= 0 ? ~0ull : host_ns;
-  auto order = [&](auto kernel, const int* d_col, const int* d_cnt, int* d_perm, int* nlev,
+  auto order = [&](auto kernel, const int* d_col, const int* d_cnt, int* d_perm, int* per, int* nlev,
                    int* nlev_rows) -> int {
-    FOS_CUDA(cudaMemsetAsync(f->d_ctr, 0, 8 * sizeof(int), s));
+    lev.resize(ng);
+    row.clear();
+    FOS_CUDA(cudaMemsetAsync(f->d_ctr, 0, kCtr * sizeof(int), s));
     FOS_CUDA(cudaMemsetAsync(f->d_z, 0, sizeof(double) * n, s));  // (refilled before every solve)
     kernel<<<grid_for((const void*)kernel, 256, 0, 8, std::min(ng, 2432)), 256, 0, s>>>(
         n, f->lfil, d_col, d_cnt, f->d_levL, reinterpret_cast<unsigned long long*>(f->d_z), d_perm,
-        f->d_ctr + 6, f->d_ctr, f->spin_limit > 0 ? f->spin_limit : kSpinLimit, f->withhold, budget);
+        f->d_ctr, f->spin_limit > 0 ? f->spin_limit : kSpinLimit, f->withhold, budget);
     f->launches++;
     FOS_CUDA(cudaGetLastError());
     FOS_CUDA(cudaMemcpyAsync(lev.data(), d_perm, sizeof(int) * ng, cudaMemcpyDeviceToHost, s));
-    FOS_CUDA(cudaMemcpyAsync(f->h_ctr, f->d_ctr, 7 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    FOS_CUDA(cudaMemcpyAsync(f->h_ctr, f->d_ctr, kCtr * sizeof(int), cudaMemcpyDeviceToHost, s));
     FOS_CUDA(cudaStreamSynchronize(s));
     if (f->h_ctr[3] == kErrSlow) {
-      if (int rc = levels_on_host(f, d_perm == f->d_permB, d_col, d_cnt, lev.data(), f->h_ctr + 6, s))
+      if (int rc = levels_on_host(f, d_perm == f->d_permB, d_col, d_cnt, lev.data(), row, f->h_ctr + 6, s))
         return rc;
+      f->h_ctr[8] = *std::max_element(row.begin(), row.end());
     } else if (f->h_ctr[3]) {
       fos_set_error("fos_ilut_factor_dev: a dependency wait ran out");
       return -6;
     }
-    const int nl = *std::max_element(lev.begin(), lev.end());
+    *nlev_rows = f->h_ctr[6];
+    *per = kGroup;
+    if (one_at_a_time(n, f->h_ctr[8], *std::max_element(lev.begin(), lev.end()))) {
+      *per = 1;
+      if (row.empty()) {  // the rows' levels are where they were published
+        pub.resize(n);
+        row.resize(n);
+        FOS_CUDA(cudaMemcpyAsync(pub.data(), f->d_z, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+        FOS_CUDA(cudaStreamSynchronize(s));
+        for (int i = 0; i < n; i++) row[i] = (int)(pub[i] >> 32);
+      }
+      lev.swap(row);
+    }
+    const int m = (int)lev.size(), nl = *std::max_element(lev.begin(), lev.end());
     std::vector<int> start(nl + 2, 0);
-    for (int g = 0; g < ng; g++) start[lev[g] + 1]++;
+    perm.resize(m);
+    for (int g = 0; g < m; g++) start[lev[g] + 1]++;
     for (int l = 0; l <= nl; l++) start[l + 1] += start[l];
-    for (int g = 0; g < ng; g++) perm[start[lev[g]]++] = g;
-    FOS_CUDA(cudaMemcpyAsync(d_perm, perm.data(), sizeof(int) * ng, cudaMemcpyHostToDevice, s));
+    for (int g = 0; g < m; g++) perm[start[lev[g]]++] = g;
+    FOS_CUDA(cudaMemcpyAsync(d_perm, perm.data(), sizeof(int) * m, cudaMemcpyHostToDevice, s));
     FOS_CUDA(cudaStreamSynchronize(s));
     *nlev = nl;
-    *nlev_rows = f->h_ctr[6];
     return 0;
   };
-  if (int rc = order(k_ilut_levels<false>, f->d_Lcol, f->d_Lcnt, f->d_permF, &f->ngF, &f->nlevF))
+  if (int rc = order(k_ilut_levels<false>, f->d_Lcol, f->d_Lcnt, f->d_permF, &f->perF, &f->swF, &f->nlevF))
     return rc;
-  return order(k_ilut_levels<true>, f->d_Ucol, f->d_Ucnt, f->d_permB, &f->ngB, &f->nlevB);
+  return order(k_ilut_levels<true>, f->d_Ucol, f->d_Ucnt, f->d_permB, &f->perB, &f->swB, &f->nlevB);
 }
 
 int fos_ilut_factor_on(fos_ilut* f, const int* ia, const int* ja, const double* a,
@@ -1093,7 +1135,7 @@ int fos_ilut_factor_on(fos_ilut* f, const int* ia, const int* ja, const double* 
                                                 f->withhold);
     f->launches++;
     FOS_CUDA(cudaGetLastError());
-    FOS_CUDA(cudaMemcpyAsync(f->h_ctr, f->d_ctr, 8 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    FOS_CUDA(cudaMemcpyAsync(f->h_ctr, f->d_ctr, 5 * sizeof(int), cudaMemcpyDeviceToHost, s));
     FOS_CUDA(cudaStreamSynchronize(s));
     const int err = f->h_ctr[3], row = f->h_ctr[4];
     if (err == kErrCapacity) {  // a row outgrew the working copy: redo with twice the room
@@ -1125,18 +1167,19 @@ int fos_ilut_solve_on(fos_ilut* f, const double* y, double* x, cudaStream_t s) {
   const long spin = f->spin_limit > 0 ? f->spin_limit : kSpinLimit;
   k_fill_pending<<<(f->n + 255) / 256, 256, 0, s>>>(f->n, f->d_z);
   // groups in flight: kLookahead levels of the average width, at least one CTA per SM
-  const int ng = (f->n + kGroup - 1) / kGroup;
-  auto sweep_grid = [&](int nlev) {
+  auto sweep = [&](auto kernel, int per, int nlev, const int* col, const double* val, const int* cnt,
+                   const int* perm, const double* rhs, double* out, double* clear, int withhold) {
+    const int ng = (f->n + per - 1) / per;
     const long width = (ng + std::max(nlev, 1) - 1) / std::max(nlev, 1);
     const long warps = std::max((long)FOS_ILUT_MIN_WARPS, kLookahead * width);
-    return std::min(grid_for((const void*)k_ilut_sweep<false>, 256, 0, 8, ng), (int)((warps + 7) / 8));
+    const int grid = std::min(grid_for((const void*)kernel, 256, 0, 8, ng), (int)((warps + 7) / 8));
+    kernel<<<grid, 256, 0, s>>>(f->n, f->lfil, col, val, cnt, f->d_dinv, perm, rhs, out, clear,
+                                f->d_ctr, spin, withhold);
   };
-  k_ilut_sweep<false><<<sweep_grid(f->ngF), 256, 0, s>>>(f->n, f->lfil, f->d_Lcol, f->d_Lval,
-                                                         f->d_Lcnt, f->d_dinv, f->d_permF, y, f->d_z,
-                                                         x, f->d_ctr, spin, f->withhold);
-  k_ilut_sweep<true><<<sweep_grid(f->ngB), 256, 0, s>>>(f->n, f->lfil, f->d_Ucol, f->d_Uval,
-                                                        f->d_Ucnt, f->d_dinv, f->d_permB, f->d_z, x,
-                                                        nullptr, f->d_ctr, spin, -1);
+  sweep(f->perF == 1 ? k_ilut_sweep<false, 1> : k_ilut_sweep<false, kGroup>, f->perF, f->swF, f->d_Lcol,
+        f->d_Lval, f->d_Lcnt, f->d_permF, y, f->d_z, x, f->withhold);
+  sweep(f->perB == 1 ? k_ilut_sweep<true, 1> : k_ilut_sweep<true, kGroup>, f->perB, f->swB, f->d_Ucol,
+        f->d_Uval, f->d_Ucnt, f->d_permB, f->d_z, x, nullptr, -1);
   f->launches += 3;
   FOS_CUDA(cudaGetLastError());
   return 0;

@@ -232,8 +232,8 @@ int fos_ilut_set_wait_limit(fos_ilut* f, long polls, int withhold_row);
  * length (all three pointers null: only the length), < 0 on error */
 long fos_ilut_copy(const fos_ilut* f, double* alu, int* jlu, int* ju, long iwk);
 /* out[0..5] = n, lfil, working-row capacity, kernels launched, levels of the L and U
- * dependency graphs of rows (the sweeps claim groups of five rows, level by level of the graphs
- * of groups).  A plain read of what the factor call left. */
+ * dependency graphs of rows (the sweeps claim rows, or groups of five, level by level of their
+ * graphs).  A plain read of what the factor call left. */
 int fos_ilut_info(const fos_ilut* f, long* out);
 void fos_ilut_destroy(fos_ilut* f);
 /* ILUT parameters of a context created with FOS_PREC_ILUT (fopbc's PBC_PREC_FILL = 50 and

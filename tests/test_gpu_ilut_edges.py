@@ -200,3 +200,112 @@ def test_orders_of_chains(cuda, n, lfil, below, above):
     y = np.random.default_rng(1).normal(size=n)
     xr = O.lusol(n, y, *ref)
     assert np.abs(p.solve(y) - xr).max() <= 1e-12 * np.abs(xr).max()
+
+
+def _stencil(nx, ny, nz):
+    """7-point stencil in natural order: 0-based CSR."""
+    n = nx * ny * nz
+    i = np.arange(n)
+    x, y, z = i % nx, i // nx % ny, i // (nx * ny)
+    ja = np.stack([i - nx * ny, i - nx, i - 1, i, i + 1, i + nx, i + nx * ny], 1)
+    inside = np.stack([z > 0, y > 0, x > 0, x >= 0, x < nx - 1, y < ny - 1, z < nz - 1], 1)
+    a = np.where(np.arange(7) == 3, 6.1, -1.0) * np.ones((n, 1))
+    return (np.concatenate([[0], np.cumsum(inside.sum(1))]).astype(np.int32),
+            ja[inside].astype(np.int32), a[inside])
+
+
+def _random_triangle(n, per_row, upper):
+    rng = np.random.default_rng(n)
+    ia, ja, a = [0], [], []
+    for i in range(n):
+        lo, hi = (i + 1, n) if upper else (0, i)
+        cols = np.unique(np.concatenate([[i], rng.integers(lo, hi, min(per_row, hi - lo)) if hi > lo else []]))
+        ja += cols.astype(int).tolist()
+        a += [12.0 if c == i else rng.uniform(-1.0, 1.0) for c in cols]
+        ia.append(len(ja))
+    return np.array(ia, np.int32), np.array(ja, np.int32), np.array(a)
+
+
+# the sweeps take rows one at a time, or groups of five where these make few enough levels: both, one
+# of each, and a diagonal on either side of the size where that is decided
+SWEEPS = {
+    "stencil": (lambda: _stencil(13, 14, 15), 8, 1e-4),
+    "stencil, groups forward": (lambda: _stencil(41, 5, 3), 60, 0.0),
+    "lower": (lambda: _random_triangle(5003, 4, False), 9, 1e-3),
+    "upper": (lambda: _random_triangle(5003, 4, True), 9, 1e-3),
+    "wide rows": (lambda: _random_triangle(701, 90, False), 120, 0.0),
+    "diagonal 1": (lambda: _random_triangle(1, 0, False), 3, 0.0),
+    "diagonal 3000": (lambda: _random_triangle(3000, 0, False), 3, 0.0),
+    "diagonal 3200": (lambda: _random_triangle(3200, 0, False), 3, 0.0),
+}
+
+
+@pytest.mark.parametrize("name", SWEEPS)
+def test_sweeps_by_rows_and_by_groups(cuda, name):
+    make, lfil, droptol = SWEEPS[name]
+    ia, ja, a = make()
+    n = len(ia) - 1
+    lfil = max(1, min(lfil, n - 1))
+    ref = oracle_ilut(n, a, ja + 1, ia + 1, lfil, droptol) if n > 1 else None
+    p = gpu_ilu(n, a, ja + 1, ia + 1, lfil, droptol)
+    y = np.random.default_rng(1).normal(size=n)
+    xr = O.lusol(n, y, *ref) if n > 1 else y / a
+    if n > 1:
+        assert_same_factors(p, ref)
+    for _ in range(3):
+        assert np.abs(p.solve(y) - xr).max() <= 1e-12 * np.abs(xr).max()
+
+
+def test_solves_take_the_time_of_the_levels_of_rows(cuda):
+    """A stencil whose rows five in a row do not belong together: 500 levels of rows, and 6,300 of
+    groups of five.  A level takes 2-3 us, so a solve stays below 8 us a level of rows."""
+    import torch
+    from fosolvers_gb300.ilut import ILU
+    ia, ja, a = _stencil(27, 28, 29)
+    n = len(ia) - 1
+    p = ILU(n, 5)
+    p.factor_csr(*(torch.from_numpy(v).cuda() for v in (ia, ja, a)), 1e-3)
+    _, jlu, ju = (v.tolist() for v in p.msr())
+    lo, up = [1] * n, [1] * n
+    for i in range(n):
+        lo[i] = 1 + max([lo[c - 1] for c in jlu[jlu[i] - 1:ju[i] - 1]], default=0)
+    for i in reversed(range(n)):
+        up[i] = 1 + max([up[c - 1] for c in jlu[ju[i] - 1:jlu[i + 1] - 1]], default=0)
+    y = torch.ones(n, dtype=torch.float64, device="cuda")
+    x = torch.empty_like(y)
+    times = []
+    for _ in range(8):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        e[0].record()
+        p.solve_dev(y, x)
+        e[1].record()
+        torch.cuda.synchronize()
+        times.append(e[0].elapsed_time(e[1]) * 1e3)
+    assert min(times) <= 8.0 * (max(lo) + max(up))
+
+
+@pytest.mark.parametrize("upper", [False, True], ids=["L", "U"])
+@pytest.mark.parametrize("entry,y11", [(0.0, np.inf), (0.0, np.nan), (np.inf, 12.0)])
+def test_unknowns_that_are_not_finite_in_groups(cuda, entry, y11, upper):
+    """Zeros that a negative tolerance keeps, and an infinite entry, where every row reads the one
+    next to it (a chain, which is swept in groups) and the one seven away."""
+    n = 23
+    ia, ja, a = [0], [], []
+    for i in range(n):
+        cols = {i: 2.0}
+        for d in (1, 7):
+            j = i + d if upper else i - d
+            if 0 <= j < n:
+                cols[j] = entry if j == 11 and d == 1 or (entry == 0.0 and d == 7) else 0.25
+        ja += sorted(cols)
+        a += [cols[j] for j in sorted(cols)]
+        ia.append(len(ja))
+    a, ja, ia = np.array(a), np.array(ja, np.int32) + 1, np.array(ia, np.int32) + 1
+    ref = oracle_ilut(n, a, ja, ia, 5, -1.0)
+    p = gpu_ilu(n, a, ja, ia, 5, -1.0)
+    assert_same_factors(p, ref)
+    y = np.arange(1.0, n + 1)
+    y[11] = y11
+    xr = O.lusol(n, y, *ref)
+    assert (~np.isfinite(xr)).sum() > 3 and np.isfinite(xr).sum() > 3
+    np.testing.assert_allclose(p.solve(y), xr, rtol=1e-12)
